@@ -97,36 +97,22 @@ __global__ void k_b_regen(WaveView w, BatchView b, const uint32_t* sobol) {
   }
 }
 
-// kind 0: extension rays (current queue), 1: shadow rays, 2: MIS rays towards
-// area lights, 3: MIS rays towards environment lights (occlusion).
-// cls_flags (wave mode): extension hits mark their slot's shading class there
-// for k_b_compact instead of appending to the class queues.
+// Rays of the kinds in `kinds` (trace_kinds); the extension queue is that of
+// the current parity, which only the device knows inside a graph.
+struct BTraceArgs {
+  RaySet set[2][4];  // [parity][TraceKinds bit]
+  BatchView b;
+  RecI job;
+  int kinds;
+  int refill_closest, refill_any;
+};
+
 template <int SMEM>
-__global__ void __launch_bounds__(512, 2) k_b_trace(WaveView w, BatchView b, int kind, int refill_below,
-                                                     uint8_t* cls_flags) {
+__global__ void __launch_bounds__(512, 2) k_b_trace(const __grid_constant__ BTraceArgs a) {
   extern __shared__ int2 stack_smem[];
-  BatchCtl& c = *b.ctl;
-  JobScene js{b.jobs, w.job};
-  int n;
-  if (kind == 0) {
-    n = c.counters[CNT_EXT0 + c.cur];
-    trace_persistent<false, SMEM>(js, w.q_ext[c.cur], n, &c.counters[CNT_FETCH_EXT], w.ray_o, w.ray_d, w.hit,
-                                  nullptr, stack_smem, refill_below, &c.error, &c.counters[CNT_CLS0], w.q_cls,
-                                  w.capacity, nullptr, cls_flags);
-  } else if (kind == 1) {
-    n = c.counters[CNT_SH];
-    trace_persistent<true, SMEM>(js, w.q_sh, n, &c.counters[CNT_FETCH_SH], w.sh_o, w.sh_d,
-                                 F4{nullptr}, w.occluded, stack_smem, refill_below, &c.error);
-  } else if (kind == 2) {
-    n = c.counters[CNT_MIS];
-    trace_persistent<false, SMEM>(js, w.q_mis, n, &c.counters[CNT_FETCH_MIS], w.mis_o, w.mis_d,
-                                  F4{w.mis_hit}, nullptr, stack_smem, refill_below, &c.error);
-  } else {  // 3: MIS rays towards environment lights, occlusion only
-    n = c.counters[CNT_MIS_ENV];
-    trace_persistent<true, SMEM>(js, w.q_mis_env, n, &c.counters[CNT_FETCH_MIS_ENV], w.mis_o, w.mis_d,
-                                 F4{nullptr}, w.mis_occluded, stack_smem, refill_below, &c.error);
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&c.rays[kind < 3 ? kind : 2], (unsigned long long)n);
+  BatchCtl& c = *a.b.ctl;
+  trace_kinds<SMEM, false, kMaxStack>(JobScene{a.b.jobs, a.job}, a.set[c.cur], a.kinds, c.counters, stack_smem,
+                                      a.refill_closest, a.refill_any, &c.error);
 }
 
 // Shading of the slots whose extension ray hit a material of class SC (or
@@ -306,22 +292,30 @@ __global__ void k_b_control(BatchView b, cudaGraphConditionalHandle cond, int in
     c.more = more ? 1 : 0;
 }
 
-template <int SMEM>
-void launch_b_trace(const WaveView& w, const BatchView& b, int kind, int grid, int block, int refill,
-                    uint8_t* cls_flags, cudaStream_t s) {
-  k_b_trace<SMEM><<<grid, block, trace_smem_bytes(SMEM, block), s>>>(w, b, kind, refill, cls_flags);
-}
-
-void b_trace(const LaunchConfig& cfg, const WaveView& w, const BatchView& b, int kind, int grid, uint8_t* cls_flags,
+// marks (wave mode): extension hits mark their slot's shading class in qflags
+// for k_b_compact instead of appending to the class queues.
+void b_trace(const LaunchConfig& cfg, const WaveView& w, const BatchView& b, int kinds, int grid, bool marks,
              cudaStream_t s) {
+  BTraceArgs a;
+  WaveView bw = w;  // the batch's queues, rays and errors are counted in its control block
+  bw.counters = b.ctl->counters;
+  bw.ray_stats = b.ctl->rays;
+  for (int cur = 0; cur < 2; ++cur) {
+    wave_ray_sets(bw, cur, a.set[cur]);
+    if (!marks) a.set[cur][0].cls_flags = nullptr;
+  }
+  a.b = b;
+  a.job = w.job;
+  a.kinds = kinds;
+  a.refill_closest = cfg.refill_below < 1 ? 1 : (cfg.refill_below > 32 ? 32 : cfg.refill_below);
+  a.refill_any = a.refill_closest;  // (the batch loop lost 9-13% of its requests/s at the plain renders' threshold)
   const int block = cfg.trace_block;
-  const int refill = cfg.refill_below < 1 ? 1 : (cfg.refill_below > 32 ? 32 : cfg.refill_below);
   switch (cfg.smem_stack) {
-    case 0: launch_b_trace<0>(w, b, kind, grid, block, refill, cls_flags, s); break;
-    case 8: launch_b_trace<8>(w, b, kind, grid, block, refill, cls_flags, s); break;
-    case 24: launch_b_trace<24>(w, b, kind, grid, block, refill, cls_flags, s); break;
-    case 32: launch_b_trace<32>(w, b, kind, grid, block, refill, cls_flags, s); break;
-    default: launch_b_trace<16>(w, b, kind, grid, block, refill, cls_flags, s); break;
+    case 0: k_b_trace<0><<<grid, block, trace_smem_bytes(0, block), s>>>(a); break;
+    case 8: k_b_trace<8><<<grid, block, trace_smem_bytes(8, block), s>>>(a); break;
+    case 24: k_b_trace<24><<<grid, block, trace_smem_bytes(24, block), s>>>(a); break;
+    case 32: k_b_trace<32><<<grid, block, trace_smem_bytes(32, block), s>>>(a); break;
+    default: k_b_trace<16><<<grid, block, trace_smem_bytes(16, block), s>>>(a); break;
   }
 }
 
@@ -390,7 +384,7 @@ void enqueue_iteration(const WaveView& w, const BatchView& b, const uint32_t* so
   end();
   const int cgrid = grid_cap(cap, kCompactSpan, cfg.num_sms * 8);
   begin(ST_TRACE_EXT);
-  b_trace(cfg, w, b, 0, tgrid, waves ? w.qflags : nullptr, stream);
+  b_trace(cfg, w, b, TK_EXT, tgrid, waves, stream);
   end();
   if (waves) {  // the trace marked the slots' shading classes: list them in slot order
     begin(ST_OTHER);
@@ -418,11 +412,10 @@ void enqueue_iteration(const WaveView& w, const BatchView& b, const uint32_t* so
     end();
   }
   begin(ST_TRACE_SHADOW);
-  b_trace(cfg, w, b, 1, tgrid, nullptr, stream);
+  b_trace(cfg, w, b, TK_SHADOW, tgrid, false, stream);
   end();
   begin(ST_TRACE_MIS);
-  b_trace(cfg, w, b, 2, tgrid, nullptr, stream);
-  b_trace(cfg, w, b, 3, tgrid, nullptr, stream);
+  b_trace(cfg, w, b, TK_MIS | TK_MIS_ENV, tgrid, false, stream);
   end();
   begin(ST_RESOLVE);
   k_b_resolve<<<sgrid, cfg.shade_block, 0, stream>>>(w, b);

@@ -4,15 +4,15 @@
 // each run over a device queue of path slots:
 //
 //   k_camera      Pinhole::generateRay for every path of the wave
-//   k_trace       closest hit for the extension rays
+//   k_trace       the bounce's extension rays (closest hit), and the previous
+//                 bounce's light rays: shadow rays (any hit) and the
+//                 BSDF-sampled MIS rays (traced once; the reference traces
+//                 that ray twice, once inside Triangle::pdf and once in
+//                 estimateDirect)
 //   k_shade       emission, BSDF construction, light sampling
 //                 (uniformSampleOneLight / estimateDirect,
 //                 src/core/integrator.cpp:8-90), BSDF sampling, Russian
 //                 roulette; appends shadow / MIS / next-bounce work
-//   k_trace_sh    occlusion for the light-sample shadow rays
-//   k_trace       closest hit for the BSDF-sampled MIS rays (traced once;
-//                 the reference traces that ray twice, once inside
-//                 Triangle::pdf and once in estimateDirect)
 //   k_film        per-pixel sums in sample order (RenderTarget::acumulate)
 //
 // A path's direct-lighting estimate is added to its radiance by its next
@@ -52,33 +52,23 @@ __global__ void k_camera(SceneView s, WaveView w, WaveArgs a) {
   }
 }
 
-// Closest hit: extension rays (RayView = RecF4, hits into the path records,
-// slots sorted by shading class) or MIS rays (NeeF4, hits into mis_hit).
-// COUNT: the same traversal, adding its node visits and triangle tests to
-// work[0] and work[3] (a diagnostic render; see WaveView::trace_work).
-// CAP: traversal stack capacity (kTestStackEntries only in the kernels that
-// exercise the overflow report); overflows set bits of *err.
-template <int SMEM, class RayView, class HitView, bool COUNT = false, int CAP = kMaxStack>
-__global__ void __launch_bounds__(512, 2)
-    k_trace(SceneView s, const int* queue, const int* count, int* fetch, RayView ray_o, RayView ray_d, HitView hit,
-            unsigned long long* stat, int refill_below, int* cls_counters, int* q_cls, int cls_stride,
-            unsigned long long* work, int* err, uint8_t* cls_flags) {
-  extern __shared__ int2 stack_smem[];
-  const int n = *count;
-  trace_persistent<false, SMEM, COUNT, CAP>(SingleScene{&s}, queue, n, fetch, ray_o, ray_d, hit, nullptr, stack_smem,
-                                            refill_below, err, cls_counters, q_cls, cls_stride, work, cls_flags);
-  if (stat && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(stat, (unsigned long long)n);
-}
+// All rays that wait at the start of a bounce (trace_kinds). CAP: traversal
+// stack capacity (kTestStackEntries only in the kernels that exercise the
+// overflow report).
+struct TraceArgs {
+  SceneView scene;
+  RaySet set[4];  // by TraceKinds bit
+  int* counters;
+  int* err;
+  int kinds;  // the TraceKinds to trace
+  int refill_closest, refill_any;
+};
 
 template <int SMEM, bool COUNT = false, int CAP = kMaxStack>
-__global__ void __launch_bounds__(512, 2)
-    k_trace_sh(SceneView s, const int* queue, const int* count, int* fetch, NeeF4 ray_o, NeeF4 ray_d, int* occluded,
-               unsigned long long* stat, int refill_below, unsigned long long* work, int* err) {
+__global__ void __launch_bounds__(512, 2) k_trace(const __grid_constant__ TraceArgs a) {
   extern __shared__ int2 stack_smem[];
-  const int n = *count;
-  trace_persistent<true, SMEM, COUNT, CAP>(SingleScene{&s}, queue, n, fetch, ray_o, ray_d, F4{nullptr}, occluded,
-                                           stack_smem, refill_below, err, nullptr, nullptr, 0, work);
-  if (stat && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(stat, (unsigned long long)n);
+  trace_kinds<SMEM, COUNT, CAP>(SingleScene{&a.scene}, a.set, a.kinds, a.counters, stack_smem, a.refill_closest,
+                                a.refill_any, a.err);
 }
 
 // One bounce for every path whose extension ray hit a material of shading
@@ -91,6 +81,11 @@ __global__ void __launch_bounds__(512, 2)
 // shading finished them.
 template <int SC>
 __global__ void __launch_bounds__(128, 5) k_shade(SceneView s, WaveView w, WaveArgs a, int bounce, int cur) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {  // the trace launch is done with these: empty them for k_compact_queues
+    w.counters[CNT_EXT0 + (cur ^ 1)] = w.counters[CNT_SH] = w.counters[CNT_MIS] = w.counters[CNT_MIS_ENV] = 0;
+    w.counters[CNT_FETCH_EXT] = w.counters[CNT_FETCH_SH] = w.counters[CNT_FETCH_MIS] = 0;
+    w.counters[CNT_FETCH_MIS_ENV] = 0;
+  }
   const int n = w.counters[CNT_CLS0 + SC];
   const int* in_q = w.q_cls + (size_t)SC * w.capacity;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
@@ -159,20 +154,6 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact_queues(uint8_t* fla
 __global__ void k_reset_counters(int* counters, int slots, int keep_slot, int keep_value) {
   int i = threadIdx.x;
   if (i < slots) counters[i] = (i == keep_slot) ? keep_value : 0;
-}
-
-// Start of a bounce: empty the queues this bounce fills, zero the fetch counters.
-__global__ void k_reset_bounce_counters(int* counters, int next_ext) {
-  int i = threadIdx.x;
-  if (i == 0) counters[next_ext] = 0;
-  if (i == 1) counters[CNT_NEE] = 0;
-  if (i == 2) counters[CNT_SH] = 0;
-  if (i == 3) counters[CNT_MIS] = 0;
-  if (i == 4) counters[CNT_FETCH_EXT] = 0;
-  if (i == 5) counters[CNT_FETCH_SH] = 0;
-  if (i == 6) counters[CNT_FETCH_MIS] = 0;
-  if (i == CNT_MIS_ENV || i == CNT_FETCH_MIS_ENV) counters[i] = 0;
-  if (i >= CNT_CLS0 && i < CNT_CLS0 + kShadeClasses) counters[i] = 0;
 }
 
 // ------------------------------------------------------------ test hooks
@@ -287,58 +268,37 @@ int grid_for(int64_t n, int block, int max_blocks) {
   return (int)(g < 1 ? 1 : g);
 }
 
-enum TraceKind { TK_EXT = 0, TK_SHADOW = 1, TK_MIS = 2, TK_MIS_ENV = 3 };
-
 template <int SMEM, bool COUNT = false, int CAP = kMaxStack>
-void launch_trace_kernels(int kind, const SceneView& s, const WaveView& w, int cur, const LaunchConfig& cfg,
-                          int grid, cudaStream_t stream) {
-  const int block = cfg.trace_block;
-  const int refill = cfg.refill_below < 1 ? 1 : (cfg.refill_below > 32 ? 32 : cfg.refill_below);
-  // Any-hit rays end early and unevenly; their warps refill at 4 lanes more
-  // (1024x1024 x 64 spp displaced sphere: 804 Mpaths/s against 798 at the
-  // closest-hit threshold of 20, 787 at 16).
-  const int refill_any = refill + 4 > 32 ? 32 : refill + 4;
-  const size_t smem = trace_smem_bytes(SMEM, block);
-  unsigned long long* work = w.trace_work;  // nodes[ext, shadow, mis], then tris[ext, shadow, mis]
-  int* err = w.error_word;
-  if (kind == TK_EXT)
-    k_trace<SMEM, RecF4, RecF4, COUNT, CAP><<<grid, block, smem, stream>>>(
-        s, w.q_ext[cur], w.counters + cur, w.counters + CNT_FETCH_EXT, w.ray_o, w.ray_d, w.hit, w.ray_stats, refill,
-        w.counters + CNT_CLS0, w.q_cls, w.capacity, work, err, w.qflags);
-  else if (kind == TK_SHADOW)
-    k_trace_sh<SMEM, COUNT, CAP><<<grid, block, smem, stream>>>(s, w.q_sh, w.counters + CNT_SH,
-                                                                w.counters + CNT_FETCH_SH, w.sh_o, w.sh_d, w.occluded,
-                                                                w.ray_stats + 1, refill_any,
-                                                                COUNT ? work + 1 : nullptr, err);
-  else if (kind == TK_MIS_ENV)
-    k_trace_sh<SMEM, COUNT, CAP><<<grid, block, smem, stream>>>(s, w.q_mis_env, w.counters + CNT_MIS_ENV,
-                                                                w.counters + CNT_FETCH_MIS_ENV, w.mis_o, w.mis_d,
-                                                                w.mis_occluded, w.ray_stats + 2, refill_any,
-                                                                COUNT ? work + 2 : nullptr, err);
-  else
-    k_trace<SMEM, NeeF4, F4, COUNT, CAP><<<grid, block, smem, stream>>>(s, w.q_mis, w.counters + CNT_MIS,
-                                                                        w.counters + CNT_FETCH_MIS, w.mis_o, w.mis_d,
-                                                                        F4{w.mis_hit}, w.ray_stats + 2, refill,
-                                                                        nullptr, nullptr, 0,
-                                                                        COUNT ? work + 2 : nullptr, err, nullptr);
+void launch_trace_kernel(int kinds, const SceneView& s, const WaveView& w, int cur, const LaunchConfig& cfg, int grid,
+                         cudaStream_t stream) {
+  TraceArgs a;
+  a.scene = s;
+  wave_ray_sets(w, cur, a.set);
+  a.counters = w.counters;
+  a.err = w.error_word;
+  a.kinds = kinds;
+  a.refill_closest = cfg.refill_below < 1 ? 1 : (cfg.refill_below > 32 ? 32 : cfg.refill_below);
+  a.refill_any = refill_any_hit(a.refill_closest);
+  k_trace<SMEM, COUNT, CAP><<<grid, cfg.trace_block, trace_smem_bytes(SMEM, cfg.trace_block), stream>>>(a);
 }
 
-void trace_dispatch(int kind, const SceneView& s, const WaveView& w, int cur, const LaunchConfig& cfg, int grid,
+// kinds: TraceKinds bits.
+void trace_dispatch(int kinds, const SceneView& s, const WaveView& w, int cur, const LaunchConfig& cfg, int grid,
                     cudaStream_t stream) {
   if (w.trace_work) {  // counting render: the stack's split between shared and local memory is irrelevant
-    launch_trace_kernels<0, true>(kind, s, w, cur, cfg, grid, stream);
+    launch_trace_kernel<0, true>(kinds, s, w, cur, cfg, grid, stream);
     return;
   }
   if (cfg.test_stack_entries) {  // orion_gpu_set_test_limits: kernels with a kTestStackEntries-entry stack
-    launch_trace_kernels<0, false, kTestStackEntries>(kind, s, w, cur, cfg, grid, stream);
+    launch_trace_kernel<0, false, kTestStackEntries>(kinds, s, w, cur, cfg, grid, stream);
     return;
   }
   switch (cfg.smem_stack) {
-    case 0: launch_trace_kernels<0>(kind, s, w, cur, cfg, grid, stream); break;
-    case 8: launch_trace_kernels<8>(kind, s, w, cur, cfg, grid, stream); break;
-    case 24: launch_trace_kernels<24>(kind, s, w, cur, cfg, grid, stream); break;
-    case 32: launch_trace_kernels<32>(kind, s, w, cur, cfg, grid, stream); break;
-    default: launch_trace_kernels<16>(kind, s, w, cur, cfg, grid, stream); break;
+    case 0: launch_trace_kernel<0>(kinds, s, w, cur, cfg, grid, stream); break;
+    case 8: launch_trace_kernel<8>(kinds, s, w, cur, cfg, grid, stream); break;
+    case 24: launch_trace_kernel<24>(kinds, s, w, cur, cfg, grid, stream); break;
+    case 32: launch_trace_kernel<32>(kinds, s, w, cur, cfg, grid, stream); break;
+    default: launch_trace_kernel<16>(kinds, s, w, cur, cfg, grid, stream); break;
   }
 }
 
@@ -374,12 +334,24 @@ void launch_wave(const SceneView& s, const WaveView& w, const WaveArgs& a, const
     class_tg.queue[c] = w.q_cls + (size_t)c * w.capacity, class_tg.counter[c] = w.counters + CNT_CLS0 + c;
   int cur = 0;
   for (int bounce = 0; bounce <= a.max_depth; ++bounce) {
-    begin(ST_OTHER);
-    k_reset_bounce_counters<<<1, 32, 0, stream>>>(w.counters, cur ^ 1);
-    end();
-    begin(ST_TRACE_EXT);
-    trace_dispatch(TK_EXT, s, w, cur, cfg, tgrid, stream);
-    end();
+    // The bounce's extension rays and the previous bounce's light rays. A
+    // render that times its stages traces them kind by kind.
+    if (!timer) {
+      trace_dispatch(bounce > 0 ? TK_ALL : TK_EXT, s, w, cur, cfg, tgrid, stream);
+      ++nl;
+    } else {
+      begin(ST_TRACE_EXT);
+      trace_dispatch(TK_EXT, s, w, cur, cfg, tgrid, stream);
+      end();
+      if (bounce > 0) {
+        begin(ST_TRACE_SHADOW);
+        trace_dispatch(TK_SHADOW, s, w, cur, cfg, tgrid, stream);
+        end();
+        begin(ST_TRACE_MIS);
+        trace_dispatch(TK_MIS | TK_MIS_ENV, s, w, cur, cfg, tgrid, stream);
+        end();
+      }
+    }
     // The trace marked each finished ray's shading class; list them by class in slot order.
     begin(ST_OTHER);
     k_compact_queues<kShadeClasses><<<compact_grid, kCompactThreads, 0, stream>>>(w.qflags, w.q_ext[cur],
@@ -414,27 +386,8 @@ void launch_wave(const SceneView& s, const WaveView& w, const WaveArgs& a, const
                                                                            tg);
       end();
     }
-    if (bounce < a.max_depth) {
-      begin(ST_TRACE_SHADOW);
-      trace_dispatch(TK_SHADOW, s, w, cur, cfg, tgrid, stream);
-      end();
-      // MIS rays exist only towards area lights (closest hit) and environment
-      // lights (occlusion); a scene without one kind skips its launch.
-      begin(ST_TRACE_MIS);
-      int mis = 0;
-      if (s.num_area_lights > 0) {
-        trace_dispatch(TK_MIS, s, w, cur, cfg, tgrid, stream);
-        ++mis;
-      }
-      if (s.num_env > 0) {
-        trace_dispatch(TK_MIS_ENV, s, w, cur, cfg, tgrid, stream);
-        ++mis;
-      }
-      nl += mis - 1;  // end() counts one
-      end();
-      // No resolve pass: each path's light sample is added to its radiance by
-      // its next shading, or by k_film if the path ends here (shade_one, DEFER).
-    }
+    // No resolve pass: each path's light sample is added to its radiance by
+    // its next shading, or by k_film if the path ends here (shade_one, DEFER).
     cur ^= 1;
   }
   if (film_wait) cudaStreamWaitEvent(stream, film_wait, 0);
@@ -483,17 +436,9 @@ cudaError_t limit_of(const void* f, int smem_bytes, int* max_block) {
 }  // namespace
 
 cudaError_t configure_kernels(int smem_bytes, KernelLimits* lim) {
-  const void* trace[] = {
-      (const void*)k_trace<0, RecF4, RecF4>,  (const void*)k_trace<8, RecF4, RecF4>,
-      (const void*)k_trace<16, RecF4, RecF4>, (const void*)k_trace<24, RecF4, RecF4>,
-      (const void*)k_trace<32, RecF4, RecF4>, (const void*)k_trace<0, NeeF4, F4>,
-      (const void*)k_trace<8, NeeF4, F4>,     (const void*)k_trace<16, NeeF4, F4>,
-      (const void*)k_trace<24, NeeF4, F4>,    (const void*)k_trace<32, NeeF4, F4>,
-      (const void*)k_trace_sh<0>,             (const void*)k_trace_sh<8>,
-      (const void*)k_trace_sh<16>,            (const void*)k_trace_sh<24>,
-      (const void*)k_trace_sh<32>,            (const void*)k_trace_rays<16>,
-      (const void*)k_trace<0, RecF4, RecF4, true>, (const void*)k_trace<0, NeeF4, F4, true>,
-      (const void*)k_trace_sh<0, true>};
+  const void* trace[] = {(const void*)k_trace<0>,        (const void*)k_trace<8>,  (const void*)k_trace<16>,
+                         (const void*)k_trace<24>,       (const void*)k_trace<32>, (const void*)k_trace<0, true>,
+                         (const void*)k_trace_rays<16>};
   const void* shade[] = {(const void*)k_shade<SC_DIFFUSE>, (const void*)k_shade<SC_CONDUCTOR>,
                          (const void*)k_shade<SC_SPECULAR>, (const void*)k_shade<SC_DIELECTRIC>,
                          (const void*)k_shade<SC_PLASTIC>, (const void*)k_shade<SC_GENERAL>, (const void*)k_shade<SC_TEXTURED>,

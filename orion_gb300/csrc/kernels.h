@@ -116,6 +116,9 @@ enum CounterSlot { CNT_EXT0 = 0, CNT_EXT1 = 1, CNT_NEE = 2, CNT_SH = 3, CNT_MIS 
                    CNT_FETCH_EXT = 8, CNT_FETCH_SH = 9, CNT_FETCH_MIS = 10, CNT_MIS_ENV = 11,
                    CNT_FETCH_MIS_ENV = 12, CNT_CLS0 = 16, kCounterSlots = 32 };
 
+// Ray kinds of one trace launch (k_trace), as bits.
+enum TraceKinds { TK_EXT = 1, TK_MIS = 2, TK_SHADOW = 4, TK_MIS_ENV = 8, TK_ALL = 15 };
+
 // ------------------------------------------------------------ batched mode
 //
 // Many render jobs (scenes, views, resolutions, spp, depths) share one pool
@@ -157,6 +160,52 @@ struct BatchView {
   int* q_retire;
   int* q_free;
 };
+
+// One kind of queued rays, as a trace kernel takes them: ray k of `count` is
+// that of path slot queue[k], its origin and direction at o / d + slot x
+// stride (float4 units).
+struct RaySet {
+  const int* queue;
+  const int* count;
+  int* fetch;         // next ray to take; zero at launch
+  const float4* o;    // any hit: w = tmax
+  const float4* d;
+  float4* hit;        // closest hit: t, u, v, primitive at hit + slot x hit_stride
+  int* occluded;      // any hit: 0 or 1 per slot
+  int stride, hit_stride;
+  // Closest hit, or null: the shading class of what each ray hit goes to its
+  // slot's byte here (bit ShadeClass), for a compaction pass, or, without
+  // flags, the slot to that class's queue.
+  uint8_t* cls_flags;
+  int* q_cls;         // kShadeClasses queues, cls_stride ints apart, or null
+  int* cls_counters;
+  int cls_stride;
+  unsigned long long* stat;  // rays traced
+  unsigned long long* work;  // counting kernels: node visits at [0], triangle tests at [3]
+};
+
+// The rays of a wave at the start of a bounce, by TraceKinds bit: extension
+// (queue `cur`), MIS, shadow, environment MIS.
+inline void wave_ray_sets(const WaveView& w, int cur, RaySet set[4]) {
+  constexpr int kRec = sizeof(PathRec) / sizeof(float4), kNee = sizeof(NeeRec) / sizeof(float4);
+  set[0] = RaySet{w.q_ext[cur], w.counters + CNT_EXT0 + cur, w.counters + CNT_FETCH_EXT, w.ray_o.p, w.ray_d.p,
+                  w.hit.p, nullptr, kRec, kRec, w.qflags, w.q_cls, w.counters + CNT_CLS0, w.capacity, w.ray_stats,
+                  w.trace_work};
+  set[1] = RaySet{w.q_mis, w.counters + CNT_MIS, w.counters + CNT_FETCH_MIS, w.mis_o.p, w.mis_d.p,
+                  w.mis_hit, nullptr, kNee, 1, nullptr, nullptr, nullptr, 0, w.ray_stats + 2,
+                  w.trace_work ? w.trace_work + 2 : nullptr};
+  set[2] = RaySet{w.q_sh, w.counters + CNT_SH, w.counters + CNT_FETCH_SH, w.sh_o.p, w.sh_d.p,
+                  nullptr, w.occluded, kNee, 0, nullptr, nullptr, nullptr, 0, w.ray_stats + 1,
+                  w.trace_work ? w.trace_work + 1 : nullptr};
+  set[3] = RaySet{w.q_mis_env, w.counters + CNT_MIS_ENV, w.counters + CNT_FETCH_MIS_ENV, w.mis_o.p, w.mis_d.p,
+                  nullptr, w.mis_occluded, kNee, 0, nullptr, nullptr, nullptr, 0, w.ray_stats + 2,
+                  w.trace_work ? w.trace_work + 2 : nullptr};
+}
+
+// Refill threshold of any-hit warps: their rays end early and unevenly, so
+// they refill at 4 lanes more (1024x1024 x 64 spp displaced sphere: 804
+// Mpaths/s against 798 at the closest-hit threshold of 20, 787 at 16).
+inline int refill_any_hit(int refill_closest) { return refill_closest + 4 > 32 ? 32 : refill_closest + 4; }
 
 #ifdef __CUDACC__
 // Sample index of a batched path slot (kept in L.w and meta.w).
