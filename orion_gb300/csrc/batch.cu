@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(128, 5) k_b_shade(WaveView w, BatchView b, con
     const DevJob& J = b.jobs[meta.y];
     const int bounce = meta.z;
     ShadeResult r = shade_one<lobes_of_class(SC), SC == SC_TEXTURED>(
-        J.scene, w, sobol, pid, (uint64_t)slot_index(w, pid), bounce, J.max_depth, J.rr_depth);
+        J.scene, w, sobol, pid, (uint64_t)slot_index(w, pid), meta.x, bounce, J.max_depth, J.rr_depth);
     if (r.alive) w.bounce[pid] = bounce + 1;
     if (waves) {
       w.qflags[pid] = (uint8_t)((r.alive ? kQfExt : 0) | (r.did_nee ? kQfNee : 0) | (r.want_sh ? kQfShadow : 0) |

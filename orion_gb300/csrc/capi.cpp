@@ -462,7 +462,6 @@ static int render_impl(orion_gpu_ctx* ctx, orion_scene_id id, const orion_render
   if (max_depth < 0 || max_depth > 120) return fail(ORION_ERR_INVALID, "max_depth out of range");
   const int64_t wh = (int64_t)d.width * d.height;
   const int64_t total = wh * spp;
-  const int64_t first = p.first_pass * wh;
   // Dimensions used: 5 + 2 (lens) + per bounce up to 8; the table has 1024.
   if (9 + 8 * (int64_t)(max_depth + 1) > 1024) return fail(ORION_ERR_INVALID, "max_depth exceeds Sobol dimensions");
   int64_t wave = p.wave_paths > 0 ? p.wave_paths : ctx->default_wave;
@@ -478,28 +477,44 @@ static int render_impl(orion_gpu_ctx* ctx, orion_scene_id id, const orion_render
     if (nw < want) nw = want;
     wave = std::max<int64_t>(1, (total + nw - 1) / nw);
   }
-  int rc = ensure_wave(ctx, (int)wave);
+  // A wave renders `passes` passes of some chunks of the film's pixels
+  // (WaveArgs). Only a wave smaller than a pixel's samples splits them: then
+  // several groups of passes follow one another.
+  const int64_t groups = (spp + wave - 1) / std::max<int64_t>(wave, 1);
+  const int passes = (int)((spp + groups - 1) / groups);
+  const int64_t wave_pixels = std::max<int64_t>(1, wave / passes);
+  int chunk_log2 = 8;  // at most a sixteenth of a wave's pixels
+  while (chunk_log2 > 0 && (int64_t)16 << chunk_log2 > wave_pixels) --chunk_log2;
+  const int64_t chunks = (wh + ((int64_t)1 << chunk_log2) - 1) >> chunk_log2;
+  // The film's waves: as few as `wave` allows, where the last chunk may take a
+  // wave over it (by a sixteenth at most) unless the caller set it.
+  const int64_t group_waves =
+      p.wave_paths > 0 ? (chunks + std::max<int64_t>(1, wave_pixels >> chunk_log2) - 1) /
+                             std::max<int64_t>(1, wave_pixels >> chunk_log2)
+                       : std::min<int64_t>(chunks, (wh + wave_pixels - 1) / wave_pixels);
+  // Wave k's chunks are k, k + group_waves, ...; the last chunk may be partial.
+  auto pixels_of = [&](int64_t k) {
+    const int64_t n = (chunks - k + group_waves - 1) / group_waves;
+    const bool has_last = (chunks - 1) % group_waves == k;
+    return (n << chunk_log2) - (has_last ? (chunks << chunk_log2) - wh : 0);
+  };
+  const int64_t capacity = std::min<int64_t>(((chunks + group_waves - 1) / group_waves) << chunk_log2, wh) * passes;
+  int rc = ensure_wave(ctx, (int)capacity);
   if (rc != ORION_OK) return rc;
-  // Consecutive waves take turns on `ns` streams, each with its own
-  // path-state block, so one wave's kernels fill the SMs that another's
-  // kernel tails leave idle; the film is written wave after wave (events),
-  // so every pixel still sums its samples in sample order. Profiled renders
-  // stay on one stream so that stage times add up.
-  const int64_t nwaves = (total + wave - 1) / wave;
+  // Waves take turns on `ns` streams, each with its own path-state block, so
+  // one wave's kernels fill the SMs that another's kernel tails leave idle.
+  // Waves of other passes of the same pixels write the film one after the
+  // other (events), so every pixel still sums its samples in sample order.
+  // Profiled renders stay on one stream so that stage times add up.
+  const int64_t nwaves = groups * group_waves;
   const int ns = ctx->profiling ? 1 : (int)std::min<int64_t>(ctx->wave_streams, nwaves);
   for (int i = 1; i < ns; ++i)
-    if ((rc = alloc_wave(ctx->xwave[i - 1], (int)wave)) != ORION_OK) return rc;
+    if ((rc = alloc_wave(ctx->xwave[i - 1], (int)capacity)) != ORION_OK) return rc;
   auto wave_view = [&](int i) -> const WaveView& { return i == 0 ? ctx->wave.view : ctx->xwave[i - 1].view; };
   auto wave_stream = [&](int i) { return i == 0 ? ctx->stream : ctx->xstream[i - 1]; };
   const bool fp64 = sum64 != nullptr;
   if ((rc = ensure_film(ctx, wh, fp64)) != ORION_OK) return rc;
   cudaStream_t s = ctx->stream;
-  CUDA_TRY(cudaMemsetAsync(ctx->film_sum.p, 0, wh * 3 * sizeof(float), s));
-  CUDA_TRY(cudaMemsetAsync(ctx->film_count.p, 0, wh * sizeof(uint32_t), s));
-  if (fp64) {
-    CUDA_TRY(cudaMemsetAsync(ctx->film64.p, 0, wh * 3 * sizeof(double), s));
-    CUDA_TRY(cudaMemsetAsync(ctx->filmsq64.p, 0, wh * 3 * sizeof(double), s));
-  }
   const bool count_work = ctx->count_work;
   for (int i = 0; i < ns; ++i) {
     CUDA_TRY(cudaMemsetAsync(wave_view(i).ray_stats, 0, 10 * sizeof(unsigned long long), s));
@@ -510,8 +525,7 @@ static int render_impl(orion_gpu_ctx* ctx, orion_scene_id id, const orion_render
   int launches = 0;
   StageTimer timer{nullptr, nullptr, 0, 0};
   if (ctx->profiling) {
-    const int64_t waves = (total + wave - 1) / wave;
-    const int need = (int)std::min<int64_t>(waves * (8 * (max_depth + 1) + 4), 200000);
+    const int need = (int)std::min<int64_t>(nwaves * (8 * (max_depth + 1) + 4), 200000);
     while ((int)ctx->prof_events.size() < 2 * need) {
       cudaEvent_t e;
       CUDA_TRY(cudaEventCreate(&e));
@@ -525,20 +539,26 @@ static int render_impl(orion_gpu_ctx* ctx, orion_scene_id id, const orion_render
     CUDA_TRY(cudaEventRecord(ctx->ev_fork, s));
     for (int i = 1; i < ns; ++i) CUDA_TRY(cudaStreamWaitEvent(wave_stream(i), ctx->ev_fork, 0));
   }
-  int64_t k = 0;
-  for (int64_t off = 0; off < total; off += wave, ++k) {
+  for (int64_t k = 0; k < nwaves; ++k) {
     const int slot = (int)(k % ns);
+    const int64_t group = k / group_waves;
     WaveArgs a;
     a.sobol = ctx->sobol.as<uint32_t>();
-    a.base_index = first + off;
-    a.n_paths = (int)std::min<int64_t>(wave, total - off);
+    a.first_pass = p.first_pass + group * passes;
+    a.passes = (int)std::min<int64_t>(passes, spp - group * passes);
+    a.wave = (int)(k % group_waves);
+    a.waves = (int)group_waves;
+    a.chunk_log2 = chunk_log2;
+    a.add = group > 0;
+    a.n_paths = (int)(pixels_of(a.wave) * a.passes);
     a.width = d.width;
     a.height = d.height;
     a.max_depth = max_depth;
     a.rr_depth = rr_depth;
     a.class_mask = d.class_mask;
-    const cudaEvent_t film_wait = ns > 1 && k > 0 ? ctx->ev_film[(k - 1) % ns] : nullptr;
-    const cudaEvent_t film_done = ns > 1 ? ctx->ev_film[k % ns] : nullptr;
+    const bool ordered = ns > 1 && groups > 1;
+    const cudaEvent_t film_wait = ordered && k > 0 ? ctx->ev_film[(k - 1) % ns] : nullptr;
+    const cudaEvent_t film_done = ordered ? ctx->ev_film[k % ns] : nullptr;
     WaveView wv = wave_view(slot);
     if (count_work) wv.trace_work = wv.ray_stats + 4;
     launch_wave(d.view, wv, a, film, ctx->cfg, wave_stream(slot), &launches, ctx->profiling ? &timer : nullptr,

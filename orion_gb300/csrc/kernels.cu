@@ -30,12 +30,29 @@ namespace orion_gb300 {
 
 namespace {
 
+// The pixel of a wave's local pixel `lp` (WaveArgs): its place in the render's
+// pixel order, which runs through tiles of 8 x 4 pixels, tile row after tile
+// row, row by row within a tile (edge tiles are smaller).
+__device__ __forceinline__ void wave_pixel(const WaveArgs& a, int lp, int* x, int* y) {
+  const int64_t pos = (((int64_t)(lp >> a.chunk_log2) * a.waves + a.wave) << a.chunk_log2) +
+                      (lp & ((1 << a.chunk_log2) - 1));
+  const uint32_t band_pixels = 4u * (uint32_t)a.width;
+  const int band = pos >> 32 ? (int)(pos / band_pixels) : (int)((uint32_t)pos / band_pixels), y0 = 4 * band;
+  const int rows = min(4, a.height - y0), in_band = (int)(pos - (int64_t)band * band_pixels);
+  const int tile = in_band / (8 * rows), x0 = 8 * tile, cols = min(8, a.width - x0);
+  const int in_tile = in_band - 8 * rows * tile, row = in_tile / cols;
+  *x = x0 + in_tile - row * cols;
+  *y = y0 + row;
+}
+
 __global__ void k_camera(SceneView s, WaveView w, WaveArgs a) {
+  if (blockIdx.x == 0 && threadIdx.x < kCounterSlots) w.counters[threadIdx.x] = threadIdx.x == CNT_EXT0 ? a.n_paths : 0;
   const int64_t wh = (int64_t)a.width * a.height;
   for (int pid = blockIdx.x * blockDim.x + threadIdx.x; pid < a.n_paths; pid += gridDim.x * blockDim.x) {
-    int64_t index = a.base_index + pid;
-    int64_t pix = index % wh;
-    int i = (int)(pix % a.width), j = (int)(pix / a.width);
+    const int lp = pid / a.passes;
+    int i, j;
+    wave_pixel(a, lp, &i, &j);
+    const int64_t index = (a.first_pass + (pid - lp * a.passes)) * wh + (int64_t)j * a.width + i;
     V3 o, d;
     const uint32_t dim = camera_ray_block(s.cam, a.sobol, (uint64_t)index, i, j, &o, &d);
     // Whole 32-byte sectors only (a partly written sector costs L2 a DRAM
@@ -46,7 +63,7 @@ __global__ void k_camera(SceneView s, WaveView w, WaveArgs a) {
     r.o = f4(o, 0.f);
     r.d = f4(d, 0.f);
     r.hit = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-    r.meta = make_int4((int)dim, 0, 0, 0);
+    r.meta = make_int4((int)dim, (int)(uint32_t)(uint64_t)index, 0, (int)((uint64_t)index >> 32));
     w.q_ext[0][pid] = pid;
     w.qflags[pid] = 0;
   }
@@ -90,57 +107,79 @@ __global__ void __launch_bounds__(128, 5) k_shade(SceneView s, WaveView w, WaveA
   const int* in_q = w.q_cls + (size_t)SC * w.capacity;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
     const int pid = in_q[q];
+    const int4 meta = w.rec[pid].meta;
+    const uint64_t index = ((uint64_t)(uint32_t)meta.w << 32) | (uint32_t)meta.y;
     ShadeResult r = shade_one<lobes_of_class(SC), SC == SC_TEXTURED, true, true>(
-        s, w, a.sobol, pid, (uint64_t)(a.base_index + pid), bounce, a.max_depth, a.rr_depth);
+        s, w, a.sobol, pid, index, meta.x, bounce, a.max_depth, a.rr_depth);
     w.qflags[pid] = (uint8_t)((r.alive ? kQfExt : 0) | (r.want_sh ? kQfShadow : 0) |
                               (r.want_mis ? kQfMis : 0) | (r.want_mis_env ? kQfMisEnv : 0));
   }
 }
 
-// Per-pixel accumulation in sample order: thread t owns the pixel of sample
-// base + t and walks that pixel's samples of the wave in index order.
-// A path whose last light sample is still pending (it ended right after
-// sampling it) gets it added here, before its radiance is summed.
-__global__ void k_film(SceneView s, WaveView w, WaveArgs a, FilmView film) {
-  const int64_t wh = (int64_t)a.width * a.height;
-  const int64_t nt = a.n_paths < wh ? a.n_paths : wh;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nt; t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t pix = (a.base_index + t) % wh;
-    float r = film.sum[3 * pix], g = film.sum[3 * pix + 1], b = film.sum[3 * pix + 2];
-    double r64 = 0, g64 = 0, b64 = 0, rr = 0, gg = 0, bb = 0;
-    uint32_t c = 0;
-    for (int64_t k = t; k < a.n_paths; k += wh) {
-      float4 l = w.L[k];
-      if (w.dim[k] & kNeePending) {
-        const V3 e = xyz(l) + nee_estimate(s, w, (int)k);
-        l.x = e.x;
-        l.y = e.y;
-        l.z = e.z;
+// Per-pixel accumulation in sample order. A pixel's samples are consecutive
+// slots: a block reads whole pixels' samples into shared memory, one thread a
+// sample (a path whose last light sample is still pending, since it ended
+// right after sampling it, gets it added here), then one thread per pixel and
+// channel adds them up in order. Pixels of more samples than threads are read
+// in several goes.
+constexpr int kFilmThreads = 256;
+
+__global__ void __launch_bounds__(kFilmThreads) k_film(SceneView s, WaveView w, WaveArgs a, FilmView film) {
+  // A pixel's samples are padded by one, so that the adding threads meet in different banks.
+  __shared__ float buf[3][2 * kFilmThreads];
+  const int t = threadIdx.x, P = a.passes;
+  const int group = P < kFilmThreads ? kFilmThreads / P : 1;  // pixels of a go
+  const int go = P < kFilmThreads ? P : kFilmThreads;         // samples of each
+  const int mine = t / go;                                    // this thread's pixel of the group, its sample
+  const int n_pixels = a.n_paths / P;
+  for (int first = blockIdx.x * group; first < n_pixels; first += gridDim.x * group) {
+    const int npx = min(group, n_pixels - first);
+    float r = 0.f;  // sums carried from go to go: pixels of several goes only (one pixel, threads 0..2)
+    double r64 = 0, rr = 0;
+    for (int from = 0; from < P; from += go) {
+      const int n = min(go, P - from);
+      const int k = t - mine * go;
+      if (mine < npx && k < n) {
+        const int pid = (first + mine) * P + from + k;
+        float4 l = w.L[pid];
+        if (w.dim[pid] & kNeePending) {
+          const V3 e = xyz(l) + nee_estimate(s, w, pid);
+          l.x = e.x;
+          l.y = e.y;
+          l.z = e.z;
+        }
+        const int at = mine * (go + 1) + k;
+        buf[0][at] = l.x;
+        buf[1][at] = l.y;
+        buf[2][at] = l.z;
       }
-      r += l.x;
-      g += l.y;
-      b += l.z;
-      ++c;
-      if (film.sum64) {
-        r64 += l.x;
-        g64 += l.y;
-        b64 += l.z;
-        rr += (double)l.x * l.x;
-        gg += (double)l.y * l.y;
-        bb += (double)l.z * l.z;
+      __syncthreads();
+      for (int u = t; u < 3 * npx; u += kFilmThreads) {
+        const int px = u / 3, c = u - 3 * px;
+        int x, y;
+        wave_pixel(a, first + px, &x, &y);
+        const int64_t pix = (int64_t)y * a.width + x;
+        if (from == 0) {
+          r = a.add ? film.sum[3 * pix + c] : 0.f;
+          r64 = rr = 0;
+        }
+        const float* v = buf[c] + px * (go + 1);
+        for (int i = 0; i < n; ++i) r += v[i];
+        if (film.sum64)
+          for (int i = 0; i < n; ++i) {
+            r64 += v[i];
+            rr += (double)v[i] * v[i];
+          }
+        if (from + n == P) {
+          film.sum[3 * pix + c] = r;
+          if (c == 0 && film.count) film.count[pix] = (a.add ? film.count[pix] : 0u) + (uint32_t)P;
+          if (film.sum64) {
+            film.sum64[3 * pix + c] = (a.add ? film.sum64[3 * pix + c] : 0.0) + r64;
+            film.sumsq64[3 * pix + c] = (a.add ? film.sumsq64[3 * pix + c] : 0.0) + rr;
+          }
+        }
       }
-    }
-    film.sum[3 * pix] = r;
-    film.sum[3 * pix + 1] = g;
-    film.sum[3 * pix + 2] = b;
-    if (film.count) film.count[pix] += c;
-    if (film.sum64) {
-      film.sum64[3 * pix] += r64;
-      film.sum64[3 * pix + 1] += g64;
-      film.sum64[3 * pix + 2] += b64;
-      film.sumsq64[3 * pix] += rr;
-      film.sumsq64[3 * pix + 1] += gg;
-      film.sumsq64[3 * pix + 2] += bb;
+      __syncthreads();
     }
   }
 }
@@ -316,9 +355,6 @@ void launch_wave(const SceneView& s, const WaveView& w, const WaveArgs& a, const
     if (timer) timer->end(stream);
     ++nl;
   };
-  begin(ST_OTHER);
-  k_reset_counters<<<1, 32, 0, stream>>>(w.counters, kCounterSlots, CNT_EXT0, a.n_paths);
-  end();
   begin(ST_CAMERA);
   k_camera<<<grid_for(a.n_paths, 256, persistent * 4), 256, 0, stream>>>(s, w, a);
   end();
@@ -392,7 +428,7 @@ void launch_wave(const SceneView& s, const WaveView& w, const WaveArgs& a, const
   }
   if (film_wait) cudaStreamWaitEvent(stream, film_wait, 0);
   begin(ST_FILM);
-  k_film<<<grid_for(a.n_paths, 256, persistent * 4), 256, 0, stream>>>(s, w, a, film);
+  k_film<<<grid_for(a.n_paths, kFilmThreads / 2, persistent * 4), kFilmThreads, 0, stream>>>(s, w, a, film);
   end();
   if (film_done) cudaEventRecord(film_done, stream);
   if (launches) *launches += nl;

@@ -51,6 +51,7 @@ struct PathRec {
   float4 L;     // radiance so far; w = batched mode: sample index, low 32 bits
   float4 hit;   // t, u, v, primitive (int bits; -1 miss)
   int4 meta;    // Sobol dimension counter; batched mode: job, bounce, sample index high 32 bits
+                // (plain waves: y, w hold the sample index)
 };
 static_assert(sizeof(PathRec) == 96, "PathRec is three sectors");
 
@@ -215,10 +216,19 @@ __device__ __forceinline__ long long slot_index(const WaveView& w, int pid) {
 }
 #endif
 
+// A wave renders `passes` sample passes of some of the film's pixels. Its slots
+// hold pixel after pixel, and each pixel's passes in order: slot = local
+// pixel x passes + pass, so the rays of a warp leave through one pixel or a few
+// neighbouring ones. The render's pixels, in tile order (wave_pixel), are cut
+// into chunks of 2^chunk_log2, dealt to its `waves` waves in turn: waves that
+// run at once then cost about the same.
 struct WaveArgs {
   const uint32_t* sobol;          // Sobol tables (sobol_sample, dmath.cuh)
-  int64_t base_index;  // sample index of path slot 0
-  int n_paths;
+  int64_t first_pass;  // sample index = (first_pass + pass) x width x height + pixel
+  int passes;
+  int wave, waves, chunk_log2;
+  int add;             // 1: an earlier wave wrote the film for these pixels (other passes)
+  int n_paths;         // local pixels x passes
   int width, height;
   int max_depth;
   int rr_depth;
@@ -267,8 +277,8 @@ struct StageTimer {
 
 // One full wave: camera rays, then (trace, shade, shadow/MIS trace,
 // resolve) per bounce, then film accumulation. All on `stream`, no host sync.
-// The film kernel first waits for `film_wait` (the previous wave's film
-// write, when waves run on two streams) and then records `film_done`.
+// The film kernel first waits for `film_wait` (the film write of an earlier
+// wave of the same pixels) and then records `film_done`.
 void launch_wave(const SceneView& s, const WaveView& w, const WaveArgs& a, const FilmView& film,
                  const LaunchConfig& cfg, cudaStream_t stream, int* launches, StageTimer* timer = nullptr,
                  cudaEvent_t film_wait = nullptr, cudaEvent_t film_done = nullptr);

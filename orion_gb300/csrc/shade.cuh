@@ -254,9 +254,11 @@ __device__ __forceinline__ V3 nee_estimate(const SceneView& s, const WaveView& w
 // added to its radiance here, first, as a separate resolve pass would have
 // added it before this bounce; this bounce's sample is left pending
 // (kNeePending) for the next shading or, if the path ends, for k_film.
+// index, dimw: the path's sample index and Sobol dimension word (rec.meta).
 template <unsigned KM = kLobeAll, bool TEX = false, bool FRESH = false, bool DEFER = false>
 __device__ __forceinline__ ShadeResult shade_one(const SceneView& s, const WaveView& w, const uint32_t* sobol,
-                                                 int pid, uint64_t index, int bounce, int max_depth, int rr_depth) {
+                                                 int pid, uint64_t index, int dimw, int bounce, int max_depth,
+                                                 int rr_depth) {
   LightDistrib distrib{s.light_func, s.light_cdf, s.light_func_int, s.num_lights};
     const float4 hv = w.hit[pid];
     const int prim = __float_as_int(hv.w);  // the trace stores the primitive, -1 for a miss
@@ -268,7 +270,6 @@ __device__ __forceinline__ ShadeResult shade_one(const SceneView& s, const WaveV
     const bool spec_prev = b4.w != 0.f;
     const float4 L4 = fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : w.L[pid];
     V3 L = xyz(L4);
-    const int dimw = DEFER ? w.dim[pid] : 0;
     if (DEFER && (dimw & kNeePending)) L = L + nee_estimate(s, w, pid);
 
     // Emission on the first hit or after a specular bounce (path.cpp:61-69).
@@ -301,7 +302,7 @@ __device__ __forceinline__ ShadeResult shade_one(const SceneView& s, const WaveV
       // This bounce consumes at most 8 sample dimensions (light choice 1,
       // light point 2, BSDF for MIS 2, continuation 2, roulette 1), drawn
       // together: their table lookups are independent.
-      const uint32_t d0 = DEFER ? (uint32_t)(dimw & ~kNeePending) : (uint32_t)w.dim[pid];
+      const uint32_t d0 = DEFER ? (uint32_t)(dimw & ~kNeePending) : (uint32_t)dimw;
       float u[8];
       sobol_dims<8>(sobol, index, d0, u);
       int used = 0;

@@ -84,3 +84,29 @@ def test_traversal_work_counts(ctx, scene):
             assert w["nodes"] < 10_000 * w["rays"], kind
     ctx.render(scene, 48, 48, wave_paths=4096)
     assert ctx.traversal_work()["ext"]["nodes"] == 0
+
+
+@pytest.mark.parametrize("width,height,spp", [(1, 1, 1), (3, 5, 7), (9, 4, 1), (33, 6, 255), (7, 41, 257), (64, 48, 3),
+                                              (8, 3, 700)])
+def test_pixel_order_at_ragged_sizes(ctx, width, height, spp):
+    """Slots run pixel after pixel through tiles of 8 x 4 pixels, each pixel's passes in order, and the
+    film adds up to 256 samples of a pixel at a go: films with cut-off tiles, chunks and sample runs
+    equal the batch engine's, which numbers its slots pass after pass (FP64 sums, 1e-5 as its tests:
+    the two engines' FP32 paths are compiled apart), and do not depend on the wave size."""
+    from orion_gb300 import scenegen
+    s = scenegen.zoo(subdiv=1, spp=spp, max_depth=3)
+    s.width, s.height = width, height
+    host = scenegen.to_host_scene(s)
+    sid = ctx.upload(host)
+    try:
+        (want, _, _), = ctx.render_batch([dict(sid=sid, width=width, height=height, first_pass=5)])[0]
+        got, _ = ctx.render(sid, width, height, first_pass=5, fp64=True)
+        assert np.allclose(got, want, rtol=1e-5, atol=1e-7)
+        ref, cnt = ctx.render(sid, width, height, first_pass=5)
+        assert (cnt == spp).all()
+        for wave in (width * height * spp, 1000, 64):
+            img, c = ctx.render(sid, width, height, first_pass=5, wave_paths=wave)
+            assert np.array_equal(c, cnt)
+            assert np.array_equal(img.view(np.uint32), ref.view(np.uint32)), f"wave {wave}"
+    finally:
+        ctx.release(sid)
