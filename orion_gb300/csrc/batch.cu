@@ -44,16 +44,11 @@ __global__ void k_b_plan(BatchView b) {
   c.cursor += (unsigned long long)take;
   c.counters[CNT_FREE] = nfree - take;
   c.counters[CNT_NEE] = 0;
-  c.counters[CNT_SH] = 0;
-  c.counters[CNT_MIS] = 0;
   c.counters[CNT_RETIRE] = 0;
-  c.counters[CNT_EXT0 + (c.cur ^ 1)] = 0;
-  c.counters[CNT_FETCH_EXT] = 0;
-  c.counters[CNT_FETCH_SH] = 0;
-  c.counters[CNT_FETCH_MIS] = 0;
-  c.counters[CNT_MIS_ENV] = 0;
-  c.counters[CNT_FETCH_MIS_ENV] = 0;
-  for (int k = 0; k < kShadeClasses; ++k) c.counters[CNT_CLS0 + k] = 0;
+  c.counters[cnt_rays(RK_EXT, c.cur ^ 1)] = 0;
+  for (int k = 1; k < kRayKinds; ++k) c.counters[cnt_rays(k, 0)] = c.counters[cnt_rays(k, 1)] = 0;
+  for (int k = 0; k < kRayKinds; ++k) c.counters[CNT_FETCH + k] = 0;
+  for (int k = 0; k < kShadeClasses; ++k) c.counters[cnt_cls(k, c.cur)] = 0;
 }
 
 __device__ __forceinline__ int job_of_work(const DevJob* jobs, int njobs, unsigned long long work) {
@@ -93,7 +88,7 @@ __global__ void k_b_regen(WaveView w, BatchView b, const uint32_t* sobol) {
     r.hit = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
     r.meta = make_int4((int)smp.dim, job, 0, (int)((unsigned long long)index >> 32));
     w.rec[slot] = r;
-    queue_append(&c.counters[CNT_EXT0 + cur], w.q_ext[cur], slot, true);
+    queue_append(&c.counters[cnt_rays(RK_EXT, cur)], w.q_ext[cur], slot, true);
   }
 }
 
@@ -104,6 +99,7 @@ struct BTraceArgs {
   BatchView b;
   RecI job;
   int kinds;
+  int flip;  // 1: the rays that this iteration's shading sent out (the other parity)
   int refill_closest, refill_any;
 };
 
@@ -111,7 +107,8 @@ template <int SMEM>
 __global__ void __launch_bounds__(512, 2) k_b_trace(const __grid_constant__ BTraceArgs a) {
   extern __shared__ int2 stack_smem[];
   BatchCtl& c = *a.b.ctl;
-  trace_kinds<SMEM, false, kMaxStack>(JobScene{a.b.jobs, a.job}, a.set[c.cur], a.kinds, c.counters, stack_smem,
+  const int cur = c.cur ^ a.flip;
+  trace_kinds<SMEM, false, kMaxStack>(JobScene{a.b.jobs, a.job}, a.set[cur], a.kinds, c.counters, cur, stack_smem,
                                       a.refill_closest, a.refill_any, &c.error);
 }
 
@@ -125,7 +122,7 @@ __global__ void __launch_bounds__(128, 5) k_b_shade(WaveView w, BatchView b, con
                                                     int waves) {
   BatchCtl& c = *b.ctl;
   const int cur = c.cur;
-  const int n = c.counters[CNT_CLS0 + SC];
+  const int n = c.counters[cnt_cls(SC, cur)];
   const int* in_q = w.q_cls + (size_t)SC * w.capacity;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
     const int pid = in_q[q];
@@ -141,10 +138,10 @@ __global__ void __launch_bounds__(128, 5) k_b_shade(WaveView w, BatchView b, con
       continue;
     }
     queue_append(&c.counters[CNT_NEE], w.q_nee, pid, r.did_nee);
-    queue_append(&c.counters[CNT_SH], w.q_sh, pid, r.want_sh);
-    queue_append(&c.counters[CNT_MIS], w.q_mis, pid, r.want_mis);
-    queue_append(&c.counters[CNT_MIS_ENV], w.q_mis_env, pid, r.want_mis_env);
-    queue_append(&c.counters[CNT_EXT0 + (cur ^ 1)], w.q_ext[cur ^ 1], pid, r.alive);
+    queue_append(&c.counters[cnt_rays(RK_SHADOW, cur ^ 1)], w.q_sh, pid, r.want_sh);
+    queue_append(&c.counters[cnt_rays(RK_MIS, cur ^ 1)], w.q_mis, pid, r.want_mis);
+    queue_append(&c.counters[cnt_rays(RK_MIS_ENV, cur ^ 1)], w.q_mis_env, pid, r.want_mis_env);
+    queue_append(&c.counters[cnt_rays(RK_EXT, cur ^ 1)], w.q_ext[cur ^ 1], pid, r.alive);
     queue_append(&c.counters[CNT_RETIRE], b.q_retire, pid, !r.alive);
   }
 }
@@ -160,16 +157,15 @@ __global__ void __launch_bounds__(kCompactThreads) k_b_compact(WaveView w, Batch
   if (which == 0) {
     for (int k = 0; k < kShadeClasses; ++k) {
       tg.queue[k] = w.q_cls + (size_t)k * w.capacity;
-      tg.counter[k] = &c.counters[CNT_CLS0 + k];
+      tg.counter[k] = &c.counters[cnt_cls(k, cur)];
     }
-    compact_queues<kShadeClasses>(w.qflags, w.q_ext[cur], &c.counters[CNT_EXT0 + cur], tg);
+    compact_queues<kShadeClasses>(w.qflags, w.q_ext[cur], &c.counters[cnt_rays(RK_EXT, cur)], tg);
   } else {
     const int next = cur ^ 1;
-    int* qs[5] = {w.q_ext[next], w.q_nee, w.q_sh, w.q_mis, w.q_mis_env};
-    int* cs[5] = {&c.counters[CNT_EXT0 + next], &c.counters[CNT_NEE], &c.counters[CNT_SH], &c.counters[CNT_MIS],
-                  &c.counters[CNT_MIS_ENV]};
-    for (int k = 0; k < 5; ++k) tg.queue[k] = qs[k], tg.counter[k] = cs[k];
-    compact_queues<5>(w.qflags, w.q_ext[cur], &c.counters[CNT_EXT0 + cur], tg);
+    int* qs[5] = {w.q_ext[next], w.q_mis, w.q_sh, w.q_mis_env, w.q_nee};  // as the QueueFlag bits
+    for (int k = 0; k < 5; ++k)
+      tg.queue[k] = qs[k], tg.counter[k] = &c.counters[k < kRayKinds ? cnt_rays(k, next) : (int)CNT_NEE];
+    compact_queues<5>(w.qflags, w.q_ext[cur], &c.counters[cnt_rays(RK_EXT, cur)], tg);
   }
 }
 
@@ -223,7 +219,7 @@ __global__ void k_b_wave_begin(BatchView b, int n, int iteration_cap) {
   c.take = 0;
   c.cur = 0;
   for (int k = 0; k < kCounterSlots; ++k) c.counters[k] = 0;
-  c.counters[CNT_EXT0] = n;
+  c.counters[cnt_rays(RK_EXT, 0)] = n;
   c.max_iterations = c.iterations + iteration_cap;
   c.more = 1;
 }
@@ -281,7 +277,7 @@ __global__ void k_b_control(BatchView b, cudaGraphConditionalHandle cond, int in
   BatchCtl& c = *b.ctl;
   c.cur ^= 1;
   c.iterations += 1;
-  bool more = c.cursor < c.total || c.counters[CNT_EXT0 + c.cur] > 0;
+  bool more = c.cursor < c.total || c.counters[cnt_rays(RK_EXT, c.cur)] > 0;
   if (more && c.iterations >= c.max_iterations) {
     c.error |= kErrIterationCap;  // bounded loop: report instead of spinning on
     more = false;
@@ -301,12 +297,12 @@ void b_trace(const LaunchConfig& cfg, const WaveView& w, const BatchView& b, int
   bw.counters = b.ctl->counters;
   bw.ray_stats = b.ctl->rays;
   for (int cur = 0; cur < 2; ++cur) {
-    wave_ray_sets(bw, cur, a.set[cur]);
-    if (!marks) a.set[cur][0].cls_flags = nullptr;
+    wave_ray_sets(bw, cur, marks, a.set[cur]);
   }
   a.b = b;
   a.job = w.job;
   a.kinds = kinds;
+  a.flip = kinds & TK_EXT ? 0 : 1;
   a.refill_closest = cfg.refill_below < 1 ? 1 : (cfg.refill_below > 32 ? 32 : cfg.refill_below);
   a.refill_any = a.refill_closest;  // (the batch loop lost 9-13% of its requests/s at the plain renders' threshold)
   const int block = cfg.trace_block;

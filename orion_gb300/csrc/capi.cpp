@@ -555,6 +555,7 @@ static int render_impl(orion_gpu_ctx* ctx, orion_scene_id id, const orion_render
     a.height = d.height;
     a.max_depth = max_depth;
     a.rr_depth = rr_depth;
+    a.append = a.n_paths <= kAppendPaths;
     a.class_mask = d.class_mask;
     const bool ordered = ns > 1 && groups > 1;
     const cudaEvent_t film_wait = ordered && k > 0 ? ctx->ev_film[(k - 1) % ns] : nullptr;

@@ -46,7 +46,7 @@ __device__ __forceinline__ void wave_pixel(const WaveArgs& a, int lp, int* x, in
 }
 
 __global__ void k_camera(SceneView s, WaveView w, WaveArgs a) {
-  if (blockIdx.x == 0 && threadIdx.x < kCounterSlots) w.counters[threadIdx.x] = threadIdx.x == CNT_EXT0 ? a.n_paths : 0;
+  if (blockIdx.x == 0 && threadIdx.x < kCounterSlots) w.counters[threadIdx.x] = threadIdx.x == cnt_rays(RK_EXT, 0) ? a.n_paths : 0;
   const int64_t wh = (int64_t)a.width * a.height;
   for (int pid = blockIdx.x * blockDim.x + threadIdx.x; pid < a.n_paths; pid += gridDim.x * blockDim.x) {
     const int lp = pid / a.passes;
@@ -78,14 +78,15 @@ struct TraceArgs {
   int* counters;
   int* err;
   int kinds;  // the TraceKinds to trace
+  int cur;    // parity
   int refill_closest, refill_any;
 };
 
 template <int SMEM, bool COUNT = false, int CAP = kMaxStack>
 __global__ void __launch_bounds__(512, 2) k_trace(const __grid_constant__ TraceArgs a) {
   extern __shared__ int2 stack_smem[];
-  trace_kinds<SMEM, COUNT, CAP>(SingleScene{&a.scene}, a.set, a.kinds, a.counters, stack_smem, a.refill_closest,
-                                a.refill_any, a.err);
+  trace_kinds<SMEM, COUNT, CAP>(SingleScene{&a.scene}, a.set, a.kinds, a.counters, a.cur, stack_smem,
+                                a.refill_closest, a.refill_any, a.err);
 }
 
 // One bounce for every path whose extension ray hit a material of shading
@@ -103,12 +104,8 @@ __global__ void __launch_bounds__(512, 2) k_trace(const __grid_constant__ TraceA
 template <int SC>
 __global__ void __launch_bounds__(128, 5) k_shade(SceneView s, WaveView w, WaveArgs a, int bounce, int cur) {
   asm volatile("griddepcontrol.launch_dependents;");
-  if (blockIdx.x == 0 && threadIdx.x == 0) {  // the trace launch is done with these: empty them for k_compact_queues
-    w.counters[CNT_EXT0 + (cur ^ 1)] = w.counters[CNT_SH] = w.counters[CNT_MIS] = w.counters[CNT_MIS_ENV] = 0;
-    w.counters[CNT_FETCH_EXT] = w.counters[CNT_FETCH_SH] = w.counters[CNT_FETCH_MIS] = 0;
-    w.counters[CNT_FETCH_MIS_ENV] = 0;
-  }
-  const int n = w.counters[CNT_CLS0 + SC];
+  if (blockIdx.x == 0 && threadIdx.x < kRayKinds) w.counters[CNT_FETCH + threadIdx.x] = 0;  // for the next trace
+  const int n = w.counters[cnt_cls(SC, cur)];
   const int* in_q = w.q_cls + (size_t)SC * w.capacity;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
     const int pid = in_q[q];
@@ -116,8 +113,16 @@ __global__ void __launch_bounds__(128, 5) k_shade(SceneView s, WaveView w, WaveA
     const uint64_t index = ((uint64_t)(uint32_t)meta.w << 32) | (uint32_t)meta.y;
     ShadeResult r = shade_one<lobes_of_class(SC), SC == SC_TEXTURED, true, true>(
         s, w, a.sobol, pid, index, meta.x, bounce, a.max_depth, a.rr_depth);
-    w.qflags[pid] = (uint8_t)((r.alive ? kQfExt : 0) | (r.want_sh ? kQfShadow : 0) |
-                              (r.want_mis ? kQfMis : 0) | (r.want_mis_env ? kQfMisEnv : 0));
+    if (a.append) {
+      int* next = w.counters + (cur ^ 1);
+      queue_append(next + cnt_rays(RK_EXT, 0), w.q_ext[cur ^ 1], pid, r.alive);
+      queue_append(next + cnt_rays(RK_MIS, 0), w.q_mis, pid, r.want_mis);
+      queue_append(next + cnt_rays(RK_SHADOW, 0), w.q_sh, pid, r.want_sh);
+      queue_append(next + cnt_rays(RK_MIS_ENV, 0), w.q_mis_env, pid, r.want_mis_env);
+    } else {
+      w.qflags[pid] = (uint8_t)((r.alive ? kQfExt : 0) | (r.want_sh ? kQfShadow : 0) |
+                                (r.want_mis ? kQfMis : 0) | (r.want_mis_env ? kQfMisEnv : 0));
+    }
   }
   if (blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
@@ -314,36 +319,37 @@ int grid_for(int64_t n, int block, int max_blocks) {
 }
 
 template <int SMEM, bool COUNT = false, int CAP = kMaxStack>
-void launch_trace_kernel(int kinds, const SceneView& s, const WaveView& w, int cur, const LaunchConfig& cfg, int grid,
-                         cudaStream_t stream) {
+void launch_trace_kernel(int kinds, const SceneView& s, const WaveView& w, int cur, bool marks, const LaunchConfig& cfg,
+                         int grid, cudaStream_t stream) {
   TraceArgs a;
   a.scene = s;
-  wave_ray_sets(w, cur, a.set);
+  wave_ray_sets(w, cur, marks, a.set);
   a.counters = w.counters;
   a.err = w.error_word;
   a.kinds = kinds;
+  a.cur = cur;
   a.refill_closest = cfg.refill_below < 1 ? 1 : (cfg.refill_below > 32 ? 32 : cfg.refill_below);
   a.refill_any = refill_any_hit(a.refill_closest);
   k_trace<SMEM, COUNT, CAP><<<grid, cfg.trace_block, trace_smem_bytes(SMEM, cfg.trace_block), stream>>>(a);
 }
 
 // kinds: TraceKinds bits.
-void trace_dispatch(int kinds, const SceneView& s, const WaveView& w, int cur, const LaunchConfig& cfg, int grid,
-                    cudaStream_t stream) {
+void trace_dispatch(int kinds, const SceneView& s, const WaveView& w, int cur, bool marks, const LaunchConfig& cfg,
+                    int grid, cudaStream_t stream) {
   if (w.trace_work) {  // counting render: the stack's split between shared and local memory is irrelevant
-    launch_trace_kernel<0, true>(kinds, s, w, cur, cfg, grid, stream);
+    launch_trace_kernel<0, true>(kinds, s, w, cur, marks, cfg, grid, stream);
     return;
   }
   if (cfg.test_stack_entries) {  // orion_gpu_set_test_limits: kernels with a kTestStackEntries-entry stack
-    launch_trace_kernel<0, false, kTestStackEntries>(kinds, s, w, cur, cfg, grid, stream);
+    launch_trace_kernel<0, false, kTestStackEntries>(kinds, s, w, cur, marks, cfg, grid, stream);
     return;
   }
   switch (cfg.smem_stack) {
-    case 0: launch_trace_kernel<0>(kinds, s, w, cur, cfg, grid, stream); break;
-    case 8: launch_trace_kernel<8>(kinds, s, w, cur, cfg, grid, stream); break;
-    case 24: launch_trace_kernel<24>(kinds, s, w, cur, cfg, grid, stream); break;
-    case 32: launch_trace_kernel<32>(kinds, s, w, cur, cfg, grid, stream); break;
-    default: launch_trace_kernel<16>(kinds, s, w, cur, cfg, grid, stream); break;
+    case 0: launch_trace_kernel<0>(kinds, s, w, cur, marks, cfg, grid, stream); break;
+    case 8: launch_trace_kernel<8>(kinds, s, w, cur, marks, cfg, grid, stream); break;
+    case 24: launch_trace_kernel<24>(kinds, s, w, cur, marks, cfg, grid, stream); break;
+    case 32: launch_trace_kernel<32>(kinds, s, w, cur, marks, cfg, grid, stream); break;
+    default: launch_trace_kernel<16>(kinds, s, w, cur, marks, cfg, grid, stream); break;
   }
 }
 
@@ -405,46 +411,45 @@ void launch_wave(const SceneView& s, const WaveView& w, const WaveArgs& a, const
   const int tgrid = grid_for(a.n_paths, cfg.trace_block, persistent);
   const int sgrid = grid_for(a.n_paths, cfg.shade_block, persistent * 2);
   const int compact_grid = grid_for(a.n_paths, kCompactSpan, cfg.num_sms * 8);
-  CompactTargets class_tg{};
-  for (int c = 0; c < kShadeClasses; ++c)
-    class_tg.queue[c] = w.q_cls + (size_t)c * w.capacity, class_tg.counter[c] = w.counters + CNT_CLS0 + c;
   int cur = 0;
   for (int bounce = 0; bounce <= a.max_depth; ++bounce) {
     // The bounce's extension rays and the previous bounce's light rays. A
     // render that times its stages traces them kind by kind.
     if (!timer) {
-      trace_dispatch(bounce > 0 ? TK_ALL : TK_EXT, s, w, cur, cfg, tgrid, stream);
+      trace_dispatch(bounce > 0 ? TK_ALL : TK_EXT, s, w, cur, !a.append, cfg, tgrid, stream);
       ++nl;
     } else {
       begin(ST_TRACE_EXT);
-      trace_dispatch(TK_EXT, s, w, cur, cfg, tgrid, stream);
+      trace_dispatch(TK_EXT, s, w, cur, !a.append, cfg, tgrid, stream);
       end();
       if (bounce > 0) {
         begin(ST_TRACE_SHADOW);
-        trace_dispatch(TK_SHADOW, s, w, cur, cfg, tgrid, stream);
+        trace_dispatch(TK_SHADOW, s, w, cur, !a.append, cfg, tgrid, stream);
         end();
         begin(ST_TRACE_MIS);
-        trace_dispatch(TK_MIS | TK_MIS_ENV, s, w, cur, cfg, tgrid, stream);
+        trace_dispatch(TK_MIS | TK_MIS_ENV, s, w, cur, !a.append, cfg, tgrid, stream);
         end();
       }
     }
-    // The trace marked each finished ray's shading class; list them by class in slot order.
-    begin(ST_OTHER);
-    k_compact_queues<kShadeClasses><<<compact_grid, kCompactThreads, 0, stream>>>(w.qflags, w.q_ext[cur],
-                                                                                  w.counters + cur, class_tg);
-    end();
+    if (!a.append) {  // the trace marked each finished ray's shading class: list them by class in slot order
+      begin(ST_OTHER);
+      CompactTargets tg{};
+      for (int c = 0; c < kShadeClasses; ++c)
+        tg.queue[c] = w.q_cls + (size_t)c * w.capacity, tg.counter[c] = w.counters + cnt_cls(c, cur);
+      k_compact_queues<kShadeClasses><<<compact_grid, kCompactThreads, 0, stream>>>(
+          w.qflags, w.q_ext[cur], w.counters + cnt_rays(RK_EXT, cur), tg);
+      end();
+    }
     begin(ST_SHADE);
     nl += launch_shading(s, w, a, bounce, cur, sgrid, cfg.shade_block, stream) - 1;  // end() counts one of them
     end();
-    if (bounce < a.max_depth) {  // after the last bounce no path goes on and no queue is read
+    if (!a.append && bounce < a.max_depth) {  // after the last bounce no path goes on and no queue is read
       begin(ST_OTHER);
       CompactTargets tg{};
-      int* qs[5] = {w.q_ext[cur ^ 1], w.q_nee, w.q_sh, w.q_mis, w.q_mis_env};
-      int* cs[5] = {w.counters + (cur ^ 1), w.counters + CNT_NEE, w.counters + CNT_SH, w.counters + CNT_MIS,
-                    w.counters + CNT_MIS_ENV};
-      for (int q = 0; q < 5; ++q) tg.queue[q] = qs[q], tg.counter[q] = cs[q];
-      k_compact_queues<5><<<compact_grid, kCompactThreads, 0, stream>>>(w.qflags, w.q_ext[cur], w.counters + cur,
-                                                                           tg);
+      int* qs[kRayKinds] = {w.q_ext[cur ^ 1], w.q_mis, w.q_sh, w.q_mis_env};  // as the QueueFlag bits
+      for (int k = 0; k < kRayKinds; ++k) tg.queue[k] = qs[k], tg.counter[k] = w.counters + cnt_rays(k, cur ^ 1);
+      k_compact_queues<kRayKinds><<<compact_grid, kCompactThreads, 0, stream>>>(
+          w.qflags, w.q_ext[cur], w.counters + cnt_rays(RK_EXT, cur), tg);
       end();
     }
     // No resolve pass: each path's light sample is added to its radiance by
@@ -473,10 +478,10 @@ void launch_trace(const SceneView& s, int64_t n, const float* rays, int any_hit,
 
 void launch_trace_wave(const SceneView& s, const WaveView& w, int n, const float* rays, int any_hit, float* t,
                        float* u, float* v, int* prim, const LaunchConfig& cfg, cudaStream_t stream) {
-  k_reset_counters<<<1, 32, 0, stream>>>(w.counters, kCounterSlots, any_hit ? CNT_SH : CNT_EXT0, n);
+  k_reset_counters<<<1, 32, 0, stream>>>(w.counters, kCounterSlots, cnt_rays(any_hit ? RK_SHADOW : RK_EXT, 0), n);
   k_load_rays<<<grid_for(n, 256, 4096), 256, 0, stream>>>(w, n, rays, any_hit);
   const int tgrid = grid_for(n, cfg.trace_block, cfg.num_sms * cfg.blocks_per_sm);
-  trace_dispatch(any_hit ? TK_SHADOW : TK_EXT, s, w, 0, cfg, tgrid, stream);
+  trace_dispatch(any_hit ? TK_SHADOW : TK_EXT, s, w, 0, true, cfg, tgrid, stream);
   k_store_hits<<<grid_for(n, 256, 4096), 256, 0, stream>>>(w, n, any_hit, t, u, v, prim);
 }
 

@@ -105,7 +105,7 @@ struct WaveView {
 };
 
 // Bits of WaveView::qflags: the queues a shaded path goes to.
-enum QueueFlag { kQfExt = 1, kQfNee = 2, kQfShadow = 4, kQfMis = 8, kQfMisEnv = 16 };
+enum QueueFlag { kQfExt = 1, kQfMis = 2, kQfShadow = 4, kQfMisEnv = 8, kQfNee = 16 };
 
 // Bits of a launch's error word (plain renders: WaveView::error_word; batches: BatchCtl::error).
 constexpr int kErrIterationCap = 1;    // a batch loop reached its iteration bound
@@ -113,11 +113,20 @@ constexpr int kErrTraversalStack = 2;  // a traversal needed more stack entries 
 // Stack capacity of the test-only trace kernels (orion_gpu_set_test_limits).
 constexpr int kTestStackEntries = 2;
 
-enum CounterSlot { CNT_EXT0 = 0, CNT_EXT1 = 1, CNT_NEE = 2, CNT_SH = 3, CNT_MIS = 4, CNT_RETIRE = 5, CNT_FREE = 6,
-                   CNT_FETCH_EXT = 8, CNT_FETCH_SH = 9, CNT_FETCH_MIS = 10, CNT_MIS_ENV = 11,
-                   CNT_FETCH_MIS_ENV = 12, CNT_CLS0 = 16, kCounterSlots = 32 };
+// Counters of a wave's queues. The queues of rays (one per kind and parity)
+// and of shaded classes (one per class and parity) are filled for one bounce
+// while the last bounce's counters are still being read, so each has two:
+// bounce b's trace reads the ray counters of parity b & 1, counts classes
+// under the same parity, and empties the other parity's for the next shading
+// and trace to fill.
+enum CounterSlot { CNT_RAYS = 0 /* + 2 x kind + parity */, CNT_FETCH = 8 /* + kind */, CNT_NEE = 12, CNT_RETIRE = 13,
+                   CNT_FREE = 14, CNT_CLS = 16 /* + 8 x parity + class */, kCounterSlots = 32 };
+ORION_HD constexpr int cnt_rays(int kind, int parity) { return CNT_RAYS + 2 * kind + parity; }
+ORION_HD constexpr int cnt_cls(int sc, int parity) { return CNT_CLS + 8 * parity + sc; }
+static_assert(kShadeClasses <= 8, "two parities of class counters");
 
-// Ray kinds of one trace launch (k_trace), as bits.
+// Ray kinds of one trace launch, by number and as bits.
+enum RayKind { RK_EXT = 0, RK_MIS = 1, RK_SHADOW = 2, RK_MIS_ENV = 3, kRayKinds = 4 };
 enum TraceKinds { TK_EXT = 1, TK_MIS = 2, TK_SHADOW = 4, TK_MIS_ENV = 8, TK_ALL = 15 };
 
 // ------------------------------------------------------------ batched mode
@@ -185,22 +194,25 @@ struct RaySet {
   unsigned long long* work;  // counting kernels: node visits at [0], triangle tests at [3]
 };
 
-// The rays of a wave at the start of a bounce, by TraceKinds bit: extension
-// (queue `cur`), MIS, shadow, environment MIS.
-inline void wave_ray_sets(const WaveView& w, int cur, RaySet set[4]) {
+// The rays of a wave of parity `cur`, by RayKind. marks: the shading classes
+// go to the slots' flag bytes.
+inline void wave_ray_sets(const WaveView& w, int cur, bool marks, RaySet set[kRayKinds]) {
   constexpr int kRec = sizeof(PathRec) / sizeof(float4), kNee = sizeof(NeeRec) / sizeof(float4);
-  set[0] = RaySet{w.q_ext[cur], w.counters + CNT_EXT0 + cur, w.counters + CNT_FETCH_EXT, w.ray_o.p, w.ray_d.p,
-                  w.hit.p, nullptr, kRec, kRec, w.qflags, w.q_cls, w.counters + CNT_CLS0, w.capacity, w.ray_stats,
-                  w.trace_work};
-  set[1] = RaySet{w.q_mis, w.counters + CNT_MIS, w.counters + CNT_FETCH_MIS, w.mis_o.p, w.mis_d.p,
-                  w.mis_hit, nullptr, kNee, 1, nullptr, nullptr, nullptr, 0, w.ray_stats + 2,
-                  w.trace_work ? w.trace_work + 2 : nullptr};
-  set[2] = RaySet{w.q_sh, w.counters + CNT_SH, w.counters + CNT_FETCH_SH, w.sh_o.p, w.sh_d.p,
-                  nullptr, w.occluded, kNee, 0, nullptr, nullptr, nullptr, 0, w.ray_stats + 1,
-                  w.trace_work ? w.trace_work + 1 : nullptr};
-  set[3] = RaySet{w.q_mis_env, w.counters + CNT_MIS_ENV, w.counters + CNT_FETCH_MIS_ENV, w.mis_o.p, w.mis_d.p,
-                  nullptr, w.mis_occluded, kNee, 0, nullptr, nullptr, nullptr, 0, w.ray_stats + 2,
-                  w.trace_work ? w.trace_work + 2 : nullptr};
+  unsigned long long* work = w.trace_work;
+  auto of = [&](int kind, const int* q, const float4* o, const float4* d, int stride, float4* hit, int hit_stride,
+                int* occluded, int stat) {
+    set[kind] = RaySet{q, w.counters + cnt_rays(kind, cur), w.counters + CNT_FETCH + kind, o, d, hit, occluded,
+                       stride, hit_stride, nullptr, nullptr, nullptr, 0, w.ray_stats + stat,
+                       work ? work + stat : nullptr};
+  };
+  of(RK_EXT, w.q_ext[cur], w.ray_o.p, w.ray_d.p, kRec, w.hit.p, kRec, nullptr, 0);
+  of(RK_MIS, w.q_mis, w.mis_o.p, w.mis_d.p, kNee, w.mis_hit, 1, nullptr, 2);
+  of(RK_SHADOW, w.q_sh, w.sh_o.p, w.sh_d.p, kNee, nullptr, 0, w.occluded, 1);
+  of(RK_MIS_ENV, w.q_mis_env, w.mis_o.p, w.mis_d.p, kNee, nullptr, 0, w.mis_occluded, 2);
+  set[RK_EXT].cls_flags = marks ? w.qflags : nullptr;
+  set[RK_EXT].q_cls = w.q_cls;
+  set[RK_EXT].cls_counters = w.counters + cnt_cls(0, cur);
+  set[RK_EXT].cls_stride = w.capacity;
 }
 
 // Refill threshold of any-hit warps: their rays end early and unevenly, so
@@ -232,8 +244,17 @@ struct WaveArgs {
   int width, height;
   int max_depth;
   int rr_depth;
+  int append;           // 1: queues are appended to directly (small waves), 0: listed by k_compact_queues
   unsigned class_mask;  // shading classes present in the scene (bit ShadeClass), SC_MISS always
 };
+
+// Waves of at most this many paths append to their queues directly: two
+// compaction launches fewer a bounce, for queues out of slot order. Medians of
+// a render, compacted / appended: Cornell 64x64 x 1 spp (4K paths a wave)
+// 0.515 / 0.404 ms; displaced 720p x 1 spp (461K) 1.76 / 1.56; Cornell 512x512 x
+// 4 spp (524K) 2.23 / 2.12, zoo the same 2.05 / 2.07; zoo 768x768 x 4 spp (1.2M)
+// 3.32 / 3.60; zoo 333x217 x 48 spp (1.7M) 4.11 / 4.72.
+constexpr int kAppendPaths = 1 << 19;
 
 struct FilmView {
   float* sum;        // W*H*3

@@ -542,13 +542,13 @@ __device__ __forceinline__ void trace_persistent(const SceneOf& scene_of, const 
 // Against a launch per kind: Cornell 64x64, 1 spp 0.90 -> 0.66 ms a render,
 // displaced sphere 1280x720, 1 spp 3.24 -> 2.49 ms; 1024x1024, 64 spp
 // unchanged (64.9 ms; 68.7 ms when it takes the kinds in the mixed order).
-// Also empties the class counters (CNT_CLS0..) of `counters`, which the last
-// shading read and the next compaction fills.
+// Also empties the other parity's counters (CounterSlot): `cur` is the parity
+// that this launch traces.
 constexpr float kSpreadRays = 4.f;
 
 template <int SMEM, bool COUNT, int CAP, class SceneOf>
 __device__ __forceinline__ void trace_kinds(const SceneOf& scene_of, const RaySet* set, int kinds, int* counters,
-                                            int2* stack_smem, int refill_closest, int refill_any, int* err) {
+                                            int cur, int2* stack_smem, int refill_closest, int refill_any, int* err) {
   float n[4], total = 0.f;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
@@ -556,7 +556,8 @@ __device__ __forceinline__ void trace_kinds(const SceneOf& scene_of, const RaySe
     total += n[k];
   }
   if (blockIdx.x == 0) {
-    if (threadIdx.x < kShadeClasses && set[0].cls_flags) counters[CNT_CLS0 + threadIdx.x] = 0;
+    if (threadIdx.x < kShadeClasses) counters[cnt_cls(threadIdx.x, cur ^ 1)] = 0;
+    if (threadIdx.x < kRayKinds) counters[cnt_rays(threadIdx.x, cur ^ 1)] = 0;
     if (threadIdx.x < 4 && ((kinds >> threadIdx.x) & 1))
       atomicAdd(set[threadIdx.x].stat, (unsigned long long)*set[threadIdx.x].count);
   }

@@ -110,3 +110,20 @@ def test_pixel_order_at_ragged_sizes(ctx, width, height, spp):
             assert np.array_equal(img.view(np.uint32), ref.view(np.uint32)), f"wave {wave}"
     finally:
         ctx.release(sid)
+
+
+@pytest.mark.parametrize("paths", [(1 << 19) - 4096, 1 << 19, (1 << 19) + 4096])
+def test_appended_and_compacted_queues_agree(ctx, paths):
+    """Waves of up to 2^19 paths append to their queues, larger ones list them in slot order; the order
+    of a queue never changes a path's result."""
+    from orion_gb300 import scenegen
+    s = scenegen.zoo(subdiv=2, spp=paths // 4096, max_depth=4)
+    s.width = s.height = 64
+    sid = ctx.upload(scenegen.to_host_scene(s))
+    try:
+        one, cnt = ctx.render(sid, 64, 64, wave_paths=paths)
+        many, c = ctx.render(sid, 64, 64, wave_paths=1 << 16)
+        assert np.array_equal(c, cnt) and (cnt == paths // 4096).all()
+        assert np.array_equal(one.view(np.uint32), many.view(np.uint32))
+    finally:
+        ctx.release(sid)
