@@ -1,25 +1,25 @@
-// Batched wavefront path tracing: many render jobs per device-side loop.
+// Batched wavefront path tracing: many render jobs per launch.
 //
-// The jobs' sample ranges are concatenated into one work list. One
-// iteration of the device-side loop
+// The jobs' sample ranges are concatenated into one work list, which runs in
+// one of two ways. Wave mode takes a wave of contiguous work items onto slots
+// 0..n-1 and runs the plain render's pipeline on them, each path against its
+// job's scene (k_wb_camera, then k_b_trace, k_wb_compact, k_b_shade per bounce,
+// then k_wb_film). Pooled mode shares one pool of slots among all jobs and
+// refills finished slots every iteration of a loop inside a CUDA graph
+// while-node:
 //
 //   k_b_plan     take = min(free slots, work left); reset this iteration's queues
-//   k_b_regen    pooled mode: start `take` new camera paths in free slots
+//   k_b_regen    start `take` new camera paths in free slots
 //   k_b_trace    closest hit for every live path (each against its job's scene)
 //   k_b_shade    one bounce of PathTracing::Li per path (shared shade_one)
-//   k_b_trace    shadow rays (any hit) and MIS rays (closest hit)
+//   k_b_trace    shadow rays (any hit) and MIS rays
 //   k_b_resolve  direct-light estimate into the path radiance
-//   k_b_retire   pooled mode: finished paths' radiance into the job's FP64
-//                film, slot freed
+//   k_b_retire   finished paths' radiance into the job's FP64 film, slot freed
 //   k_b_control  flip queues; keep looping while work or live paths remain
 //
-// runs inside a CUDA graph while-node. Pooled mode shares one pool of path
-// slots among all jobs and refills finished slots every iteration. Wave mode
-// starts a wave of contiguous work items on slots 0..n-1
-// (k_b_wave_begin / k_b_wave_camera), loops until none is alive and writes
-// the film once (k_b_wave_film). Paths of different jobs, depths and bounces
-// share every launch. Each path runs the plain path's device functions on
-// the same samples; the film's order of accumulation differs (FP64 atomics).
+// Paths of different jobs and depths share every launch. Each path runs the
+// plain path's device functions on the same samples; the film's order of
+// accumulation differs (FP64 atomics).
 #include <cuda_runtime.h>
 
 #include "kernels.h"
@@ -43,7 +43,7 @@ __global__ void k_b_plan(BatchView b) {
   c.take_base = c.cursor;
   c.cursor += (unsigned long long)take;
   c.counters[CNT_FREE] = nfree - take;
-  c.counters[CNT_NEE] = 0;
+  c.counters[CNT_NEE] = c.counters[CNT_NEE + 1] = 0;
   c.counters[CNT_RETIRE] = 0;
   c.counters[cnt_rays(RK_EXT, c.cur ^ 1)] = 0;
   for (int k = 1; k < kRayKinds; ++k) c.counters[cnt_rays(k, 0)] = c.counters[cnt_rays(k, 1)] = 0;
@@ -92,14 +92,16 @@ __global__ void k_b_regen(WaveView w, BatchView b, const uint32_t* sobol) {
   }
 }
 
-// Rays of the kinds in `kinds` (trace_kinds); the extension queue is that of
-// the current parity, which only the device knows inside a graph.
+// Rays of the kinds in `kinds` (trace_kinds). parity: that of the queues to
+// trace; pooled mode, whose current parity only the device knows inside a
+// graph: kCurrent, or kNext for the rays that this iteration's shading sent out.
+constexpr int kCurrent = 2, kNext = 3;
+
 struct BTraceArgs {
-  RaySet set[2][4];  // [parity][TraceKinds bit]
+  RaySet set[2][kRayKinds];  // [parity][RayKind]
   BatchView b;
   RecI job;
-  int kinds;
-  int flip;  // 1: the rays that this iteration's shading sent out (the other parity)
+  int kinds, parity;
   int refill_closest, refill_any;
 };
 
@@ -107,21 +109,24 @@ template <int SMEM>
 __global__ void __launch_bounds__(512, 2) k_b_trace(const __grid_constant__ BTraceArgs a) {
   extern __shared__ int2 stack_smem[];
   BatchCtl& c = *a.b.ctl;
-  const int cur = c.cur ^ a.flip;
+  const int cur = a.parity == kCurrent ? c.cur : a.parity == kNext ? c.cur ^ 1 : a.parity;
   trace_kinds<SMEM, false, kMaxStack>(JobScene{a.b.jobs, a.job}, a.set[cur], a.kinds, c.counters, cur, stack_smem,
                                       a.refill_closest, a.refill_any, &c.error);
 }
 
 // Shading of the slots whose extension ray hit a material of class SC (or
 // missed, SC_MISS), each against its job's scene.
-// waves: a wave's paths are never retired one by one, and the queues they go
-// to are marked in the slots' qflags bytes for k_b_compact (slot order, as in
-// plain renders); pooled mode appends to the queues directly.
+// Waves (parity 0 or 1): paths are never retired one by one; the queues they go
+// to are marked in the slots' qflags bytes (`marks`, for a compaction) or
+// appended to. As in plain renders the classes' launches overlap (k_shade). One
+// kernel serves both modes so that a path's arithmetic is compiled once.
 template <int SC>
-__global__ void __launch_bounds__(128, 5) k_b_shade(WaveView w, BatchView b, const uint32_t* sobol,
-                                                    int waves) {
+__global__ void __launch_bounds__(128, 5) k_b_shade(WaveView w, BatchView b, const uint32_t* sobol, int parity,
+                                                    int marks) {
+  asm volatile("griddepcontrol.launch_dependents;");
   BatchCtl& c = *b.ctl;
-  const int cur = c.cur;
+  const bool waves = parity != kCurrent;
+  const int cur = waves ? parity : c.cur;
   const int n = c.counters[cnt_cls(SC, cur)];
   const int* in_q = w.q_cls + (size_t)SC * w.capacity;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
@@ -132,45 +137,27 @@ __global__ void __launch_bounds__(128, 5) k_b_shade(WaveView w, BatchView b, con
     ShadeResult r = shade_one<lobes_of_class(SC), SC == SC_TEXTURED>(
         J.scene, w, sobol, pid, (uint64_t)slot_index(w, pid), meta.x, bounce, J.max_depth, J.rr_depth);
     if (r.alive) w.bounce[pid] = bounce + 1;
-    if (waves) {
+    if (marks) {
       w.qflags[pid] = (uint8_t)((r.alive ? kQfExt : 0) | (r.did_nee ? kQfNee : 0) | (r.want_sh ? kQfShadow : 0) |
                                 (r.want_mis ? kQfMis : 0) | (r.want_mis_env ? kQfMisEnv : 0));
       continue;
     }
-    queue_append(&c.counters[CNT_NEE], w.q_nee, pid, r.did_nee);
+    queue_append(&c.counters[CNT_NEE + (cur ^ 1)], w.q_nee, pid, r.did_nee);
     queue_append(&c.counters[cnt_rays(RK_SHADOW, cur ^ 1)], w.q_sh, pid, r.want_sh);
     queue_append(&c.counters[cnt_rays(RK_MIS, cur ^ 1)], w.q_mis, pid, r.want_mis);
     queue_append(&c.counters[cnt_rays(RK_MIS_ENV, cur ^ 1)], w.q_mis_env, pid, r.want_mis_env);
     queue_append(&c.counters[cnt_rays(RK_EXT, cur ^ 1)], w.q_ext[cur ^ 1], pid, r.alive);
-    queue_append(&c.counters[CNT_RETIRE], b.q_retire, pid, !r.alive);
+    if (!waves) queue_append(&c.counters[CNT_RETIRE], b.q_retire, pid, !r.alive);
+  }
+  if (waves) {
+    if (blockIdx.x == 0 && threadIdx.x < kRayKinds) c.counters[CNT_FETCH + threadIdx.x] = 0;  // for the next trace
+    if (blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
   }
 }
 
-// Wave mode: the slots' qflags bytes into queues in slot order (plain
-// renders' compaction, compact_queues). which 0: shading classes, after the
-// extension trace; 1: the queues the shading sent paths to (next extension
-// queue by the current parity, which only the device knows inside a graph).
-__global__ void __launch_bounds__(kCompactThreads) k_b_compact(WaveView w, BatchView b, int which) {
-  BatchCtl& c = *b.ctl;
-  const int cur = c.cur;
-  CompactTargets tg{};
-  if (which == 0) {
-    for (int k = 0; k < kShadeClasses; ++k) {
-      tg.queue[k] = w.q_cls + (size_t)k * w.capacity;
-      tg.counter[k] = &c.counters[cnt_cls(k, cur)];
-    }
-    compact_queues<kShadeClasses>(w.qflags, w.q_ext[cur], &c.counters[cnt_rays(RK_EXT, cur)], tg);
-  } else {
-    const int next = cur ^ 1;
-    int* qs[5] = {w.q_ext[next], w.q_mis, w.q_sh, w.q_mis_env, w.q_nee};  // as the QueueFlag bits
-    for (int k = 0; k < 5; ++k)
-      tg.queue[k] = qs[k], tg.counter[k] = &c.counters[k < kRayKinds ? cnt_rays(k, next) : (int)CNT_NEE];
-    compact_queues<5>(w.qflags, w.q_ext[cur], &c.counters[cnt_rays(RK_EXT, cur)], tg);
-  }
-}
-
-__global__ void k_b_resolve(WaveView w, BatchView b) {
-  const int n = b.ctl->counters[CNT_NEE];
+// parity: that of the paths to resolve, or kNext (pooled mode).
+__global__ void k_b_resolve(WaveView w, BatchView b, int parity) {
+  const int n = b.ctl->counters[CNT_NEE + (parity == kNext ? b.ctl->cur ^ 1 : parity)];
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
     const int pid = w.q_nee[q];
     resolve_one(b.jobs[w.job[pid]].scene, w, pid);
@@ -207,67 +194,130 @@ __global__ void k_b_retire(WaveView w, BatchView b) {
 // A batch can also run as waves over its concatenated work list: wave k
 // takes work items [base, base + n) onto slots 0..n-1 in order, its paths
 // bounce until none is alive (no refills), and the radiance of all n paths
-// goes to the jobs' films at the end, slot after slot, so neighbouring slots
-// add to neighbouring pixels of one job.
+// goes to the jobs' films at the end. A job's work items run pixel after
+// pixel in tile order, each pixel's passes in order, so neighbouring slots
+// hold neighbouring paths, as in plain waves, whose pipeline (fused trace,
+// overlapping shading classes) this is, with a launch that adds the light
+// samples once their rays are traced.
 
-// Resets the per-wave control fields (rays, paths and iterations stay
-// cumulative over the batch's waves).
-__global__ void k_b_wave_begin(BatchView b, int n, int iteration_cap) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  BatchCtl& c = *b.ctl;
-  c.cursor = c.total = c.take_base = 0ULL;
-  c.take = 0;
-  c.cur = 0;
-  for (int k = 0; k < kCounterSlots; ++k) c.counters[k] = 0;
-  c.counters[cnt_rays(RK_EXT, 0)] = n;
-  c.max_iterations = c.iterations + iteration_cap;
-  c.more = 1;
+// Work item `work`: its job, and the pixel and pass within the job.
+struct WorkItem {
+  int job, pass;
+  long long pixel;  // in tile order
+};
+
+__device__ __forceinline__ WorkItem work_item(const DevJob* jobs, int njobs, unsigned long long work) {
+  WorkItem it;
+  it.job = job_of_work(jobs, njobs, work);
+  const DevJob& J = jobs[it.job];
+  const long long k = (long long)(work - (unsigned long long)J.work_begin);
+  it.pixel = k >> 32 ? k / J.spp : (long long)((uint32_t)k / (uint32_t)J.spp);
+  it.pass = (int)(k - it.pixel * J.spp);
+  return it;
 }
 
-__global__ void k_b_wave_camera(WaveView w, BatchView b, const uint32_t* sobol, unsigned long long base, int n) {
-  const int njobs = b.ctl->njobs;
+__global__ void k_wb_camera(WaveView w, BatchView b, const uint32_t* sobol, unsigned long long base, int n) {
+  BatchCtl& c = *b.ctl;
+  if (blockIdx.x == 0 && threadIdx.x < kCounterSlots)
+    c.counters[threadIdx.x] = threadIdx.x == cnt_rays(RK_EXT, 0) ? n : 0;
+  const int njobs = c.njobs;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const unsigned long long work = base + (unsigned long long)i;
-    const int job = job_of_work(b.jobs, njobs, work);
-    const DevJob& J = b.jobs[job];
-    const long long index = J.first_index + (long long)(work - (unsigned long long)J.work_begin);
+    const WorkItem it = work_item(b.jobs, njobs, base + (unsigned long long)i);
+    const DevJob& J = b.jobs[it.job];
+    int px, py;
+    tile_pixel(it.pixel, J.width, J.height, &px, &py);
     const long long wh = (long long)J.width * J.height;
-    const long long pix = index % wh;
+    const long long index = J.first_index + it.pass * wh + (long long)py * J.width + px;
     V3 o, d;
-    const uint32_t dim = camera_ray_block(J.scene.cam, sobol, (uint64_t)index, (int)(pix % J.width),
-                                          (int)(pix / J.width), &o, &d);
-    PathRec r;
+    const uint32_t dim = camera_ray_block(J.scene.cam, sobol, (uint64_t)index, px, py, &o, &d);
+    PathRec& r = w.rec[i];
     r.o = f4(o, 0.f);
     r.d = f4(d, 0.f);
     r.beta = make_float4(1.f, 1.f, 1.f, 0.f);
     r.L = make_float4(0.f, 0.f, 0.f, __uint_as_float((uint32_t)(unsigned long long)index));
     r.hit = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-    r.meta = make_int4((int)dim, job, 0, (int)((unsigned long long)index >> 32));
-    w.rec[i] = r;
+    r.meta = make_int4((int)dim, it.job, 0, (int)((unsigned long long)index >> 32));
     w.q_ext[0][i] = i;
     w.qflags[i] = 0;
   }
 }
 
-__global__ void k_b_wave_film(WaveView w, BatchView b, int n) {
-  for (int pid = blockIdx.x * blockDim.x + threadIdx.x; pid < n; pid += gridDim.x * blockDim.x) {
-    const float4 l = w.L[pid];
-    const int4 meta = w.rec[pid].meta;
-    const DevJob& J = b.jobs[meta.y];
-    const long long index =
-        (long long)(((unsigned long long)(unsigned)meta.w << 32) | (unsigned long long)__float_as_uint(l.w));
-    const long long pix = index % ((long long)J.width * J.height);
-    atomicAdd(&J.sum[3 * pix], (double)l.x);
-    atomicAdd(&J.sum[3 * pix + 1], (double)l.y);
-    atomicAdd(&J.sum[3 * pix + 2], (double)l.z);
-    if (J.sumsq) {
-      atomicAdd(&J.sumsq[3 * pix], (double)l.x * l.x);
-      atomicAdd(&J.sumsq[3 * pix + 1], (double)l.y * l.y);
-      atomicAdd(&J.sumsq[3 * pix + 2], (double)l.z * l.z);
-    }
-    if (J.count) atomicAdd(&J.count[pix], 1u);
+template <int NQ>
+__global__ void __launch_bounds__(kCompactThreads) k_wb_compact(uint8_t* flags, const int* list, const int* count,
+                                                                CompactTargets tg) {
+  compact_queues<NQ>(flags, list, count, tg);
+}
+
+// unfinished: -1, or the parity of the extension queue that must be empty.
+// The wave's radiance into the jobs' films. A block takes 256 slots at a time
+// into shared memory; slots of one pixel are neighbours, so one thread per run of equal pixels and channel
+// adds up the run and issues its FP64 atomics (a pixel's samples may go on in
+// the next 256 slots or another wave): one atomic per run instead of one per
+// path.
+constexpr int kWbFilmThreads = 256;
+
+__global__ void __launch_bounds__(kWbFilmThreads) k_wb_film(WaveView w, BatchView b, unsigned long long base, int n,
+                                                            int unfinished) {
+  __shared__ float buf[3][kWbFilmThreads];
+  __shared__ int run_start[kWbFilmThreads + 1];
+  __shared__ int warp_runs[kWbFilmThreads / 32];
+  __shared__ long long run_pix[kWbFilmThreads];
+  __shared__ int run_job[kWbFilmThreads];
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  BatchCtl& c = *b.ctl;
+  if (blockIdx.x == 0 && t == 0) {
+    c.paths_done += (unsigned long long)n;
+    if (unfinished >= 0 && c.counters[cnt_rays(RK_EXT, unfinished)] > 0) c.error |= kErrIterationCap;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&b.ctl->paths_done, (unsigned long long)n);
+  const int njobs = c.njobs;
+  for (int from = blockIdx.x * kWbFilmThreads; from < n; from += gridDim.x * kWbFilmThreads) {
+    const int pid = from + t;
+    bool head = false;
+    WorkItem it{0, 0, 0};
+    if (pid < n) {
+      it = work_item(b.jobs, njobs, base + (unsigned long long)pid);
+      head = t == 0 || it.pass == 0;
+      const float4 l = w.L[pid];
+      buf[0][t] = l.x;
+      buf[1][t] = l.y;
+      buf[2][t] = l.z;
+    }
+    const unsigned heads = __ballot_sync(0xffffffffu, head);
+    if (lane == 0) warp_runs[wid] = __popc(heads);
+    __syncthreads();
+    int before = 0, runs = 0;
+#pragma unroll
+    for (int k = 0; k < kWbFilmThreads / 32; ++k) {
+      if (k < wid) before += warp_runs[k];
+      runs += warp_runs[k];
+    }
+    if (head) {
+      const DevJob& J = b.jobs[it.job];
+      const int r = before + __popc(heads & ((1u << lane) - 1u));
+      int x, y;
+      tile_pixel(it.pixel, J.width, J.height, &x, &y);
+      run_start[r] = t;
+      run_job[r] = it.job;
+      run_pix[r] = (long long)y * J.width + x;
+    }
+    if (t == 0) run_start[runs] = min(kWbFilmThreads, n - from);
+    __syncthreads();
+    for (int u = t; u < 3 * runs; u += kWbFilmThreads) {
+      const int r = u / 3, ch = u - 3 * r;
+      const DevJob& J = b.jobs[run_job[r]];
+      const float* v = buf[ch];
+      const int s0 = run_start[r], s1 = run_start[r + 1];
+      double sum = 0, sq = 0;
+      for (int i = s0; i < s1; ++i) sum += (double)v[i];
+      atomicAdd(&J.sum[3 * run_pix[r] + ch], sum);
+      if (J.sumsq) {
+        for (int i = s0; i < s1; ++i) sq += (double)v[i] * v[i];
+        atomicAdd(&J.sumsq[3 * run_pix[r] + ch], sq);
+      }
+      if (J.count && ch == 0) atomicAdd(&J.count[run_pix[r]], (unsigned)(s1 - s0));
+    }
+    __syncthreads();
+  }
 }
 
 // in_graph: sets the while-node's condition; otherwise leaves the decision in
@@ -288,21 +338,16 @@ __global__ void k_b_control(BatchView b, cudaGraphConditionalHandle cond, int in
     c.more = more ? 1 : 0;
 }
 
-// marks (wave mode): extension hits mark their slot's shading class in qflags
-// for k_b_compact instead of appending to the class queues.
-void b_trace(const LaunchConfig& cfg, const WaveView& w, const BatchView& b, int kinds, int grid, bool marks,
-             cudaStream_t s) {
+// marks: extension hits mark their slot's shading class in qflags for a
+// compaction instead of appending to the class queues.
+void b_trace(const LaunchConfig& cfg, const WaveView& bw, const BatchView& b, int kinds, int parity, int grid,
+             bool marks, cudaStream_t s) {
   BTraceArgs a;
-  WaveView bw = w;  // the batch's queues, rays and errors are counted in its control block
-  bw.counters = b.ctl->counters;
-  bw.ray_stats = b.ctl->rays;
-  for (int cur = 0; cur < 2; ++cur) {
-    wave_ray_sets(bw, cur, marks, a.set[cur]);
-  }
+  for (int cur = 0; cur < 2; ++cur) wave_ray_sets(bw, cur, marks, a.set[cur]);
   a.b = b;
-  a.job = w.job;
+  a.job = bw.job;
   a.kinds = kinds;
-  a.flip = kinds & TK_EXT ? 0 : 1;
+  a.parity = parity;
   a.refill_closest = cfg.refill_below < 1 ? 1 : (cfg.refill_below > 32 ? 32 : cfg.refill_below);
   a.refill_any = a.refill_closest;  // (the batch loop lost 9-13% of its requests/s at the plain renders' threshold)
   const int block = cfg.trace_block;
@@ -313,6 +358,16 @@ void b_trace(const LaunchConfig& cfg, const WaveView& w, const BatchView& b, int
     case 32: k_b_trace<32><<<grid, block, trace_smem_bytes(32, block), s>>>(a); break;
     default: k_b_trace<16><<<grid, block, trace_smem_bytes(16, block), s>>>(a); break;
   }
+}
+
+// The wave as the batch's kernels see it: queues and rays are counted in the
+// batch's control block.
+WaveView batch_view(const WaveView& w, const BatchView& b) {
+  WaveView v = w;
+  v.counters = b.ctl->counters;
+  v.ray_stats = b.ctl->rays;
+  v.trace_work = nullptr;
+  return v;
 }
 
 cudaError_t batch_limit_of(const void* f, int smem_bytes, int* max_block) {
@@ -360,11 +415,12 @@ void launch_batch_init(const WaveView& w, const BatchView& b, int capacity, cuda
 
 namespace {
 
-// One loop iteration's kernels on `stream`, optionally timed per stage.
+// One pooled loop iteration's kernels on `stream`, optionally timed per stage.
 void enqueue_iteration(const WaveView& w, const BatchView& b, const uint32_t* sobol,
-                       const LaunchConfig& cfg, unsigned class_mask, bool waves, cudaGraphConditionalHandle cond,
+                       const LaunchConfig& cfg, unsigned class_mask, cudaGraphConditionalHandle cond,
                        int in_graph, cudaStream_t stream, StageTimer* timer) {
   const int cap = w.capacity;
+  const WaveView bw = batch_view(w, b);
   const int persistent = cfg.num_sms * cfg.blocks_per_sm;
   const int tgrid = grid_cap(cap, cfg.trace_block, persistent);
   const int sgrid = grid_cap(cap, cfg.shade_block, persistent * 2);
@@ -375,65 +431,81 @@ void enqueue_iteration(const WaveView& w, const BatchView& b, const uint32_t* so
     if (timer) timer->end(stream);
   };
   begin(ST_CAMERA);
-  k_b_plan<<<1, 32, 0, stream>>>(b);  // wave mode: counters reset, nothing to take
-  if (!waves) k_b_regen<<<grid_cap(cap, 256, persistent * 4), 256, 0, stream>>>(w, b, sobol);
+  k_b_plan<<<1, 32, 0, stream>>>(b);
+  k_b_regen<<<grid_cap(cap, 256, persistent * 4), 256, 0, stream>>>(w, b, sobol);
   end();
-  const int cgrid = grid_cap(cap, kCompactSpan, cfg.num_sms * 8);
   begin(ST_TRACE_EXT);
-  b_trace(cfg, w, b, TK_EXT, tgrid, waves, stream);
+  b_trace(cfg, bw, b, TK_EXT, kCurrent, tgrid, false, stream);
   end();
-  if (waves) {  // the trace marked the slots' shading classes: list them in slot order
-    begin(ST_OTHER);
-    k_b_compact<<<cgrid, kCompactThreads, 0, stream>>>(w, b, 0);
-    end();
-  }
   begin(ST_SHADE);
   for (int sc = 0; sc < kShadeClasses; ++sc) {
     if (!((class_mask >> sc) & 1u)) continue;
     switch (sc) {
-      case SC_DIFFUSE: k_b_shade<SC_DIFFUSE><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, waves); break;
-      case SC_CONDUCTOR: k_b_shade<SC_CONDUCTOR><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, waves); break;
-      case SC_SPECULAR: k_b_shade<SC_SPECULAR><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, waves); break;
-      case SC_DIELECTRIC: k_b_shade<SC_DIELECTRIC><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, waves); break;
-      case SC_PLASTIC: k_b_shade<SC_PLASTIC><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, waves); break;
-      case SC_GENERAL: k_b_shade<SC_GENERAL><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, waves); break;
-      case SC_TEXTURED: k_b_shade<SC_TEXTURED><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, waves); break;
-      case SC_MISS: k_b_shade<SC_MISS><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, waves); break;
+      case SC_DIFFUSE: k_b_shade<SC_DIFFUSE><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
+      case SC_CONDUCTOR: k_b_shade<SC_CONDUCTOR><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
+      case SC_SPECULAR: k_b_shade<SC_SPECULAR><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
+      case SC_DIELECTRIC: k_b_shade<SC_DIELECTRIC><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
+      case SC_PLASTIC: k_b_shade<SC_PLASTIC><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
+      case SC_GENERAL: k_b_shade<SC_GENERAL><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
+      case SC_TEXTURED: k_b_shade<SC_TEXTURED><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
+      case SC_MISS: k_b_shade<SC_MISS><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
     }
   }
   end();
-  if (waves) {  // the shading marked the queues its paths go to
-    begin(ST_OTHER);
-    k_b_compact<<<cgrid, kCompactThreads, 0, stream>>>(w, b, 1);
-    end();
-  }
   begin(ST_TRACE_SHADOW);
-  b_trace(cfg, w, b, TK_SHADOW, tgrid, false, stream);
+  b_trace(cfg, bw, b, TK_SHADOW, kNext, tgrid, false, stream);
   end();
   begin(ST_TRACE_MIS);
-  b_trace(cfg, w, b, TK_MIS | TK_MIS_ENV, tgrid, false, stream);
+  b_trace(cfg, bw, b, TK_MIS | TK_MIS_ENV, kNext, tgrid, false, stream);
   end();
   begin(ST_RESOLVE);
-  k_b_resolve<<<sgrid, cfg.shade_block, 0, stream>>>(w, b);
+  k_b_resolve<<<sgrid, cfg.shade_block, 0, stream>>>(w, b, kNext);
   end();
-  if (!waves) {  // wave mode: the film is written once the wave is done
-    begin(ST_FILM);
-    k_b_retire<<<sgrid, cfg.shade_block, 0, stream>>>(w, b);
-    end();
-  }
+  begin(ST_FILM);
+  k_b_retire<<<sgrid, cfg.shade_block, 0, stream>>>(w, b);
+  end();
   begin(ST_OTHER);
   k_b_control<<<1, 32, 0, stream>>>(b, cond, in_graph);
   end();
 }
 
+// Shading of one bounce of a batch wave, as launch_shading (kernels.cu).
+int launch_wb_shading(const WaveView& bw, const BatchView& b, const uint32_t* sobol, unsigned class_mask, int cur,
+                      int append, int grid, int block, cudaStream_t stream) {
+  using Kernel = void (*)(WaveView, BatchView, const uint32_t*, int, int);
+  static const struct {
+    int sc;
+    Kernel kernel;
+  } kOrder[kShadeClasses] = {{SC_TEXTURED, k_b_shade<SC_TEXTURED>},     {SC_GENERAL, k_b_shade<SC_GENERAL>},
+                             {SC_PLASTIC, k_b_shade<SC_PLASTIC>},       {SC_DIELECTRIC, k_b_shade<SC_DIELECTRIC>},
+                             {SC_CONDUCTOR, k_b_shade<SC_CONDUCTOR>},   {SC_DIFFUSE, k_b_shade<SC_DIFFUSE>},
+                             {SC_SPECULAR, k_b_shade<SC_SPECULAR>},     {SC_MISS, k_b_shade<SC_MISS>}};
+  cudaLaunchAttribute early;
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.stream = stream;
+  c.attrs = &early;
+  int n = 0;
+  for (const auto& k : kOrder) {
+    if (!((class_mask >> k.sc) & 1u)) continue;
+    c.numAttrs = n > 0 ? 1 : 0;
+    cudaLaunchKernelEx(&c, k.kernel, bw, b, sobol, cur, append ? 0 : 1);
+    ++n;
+  }
+  return n;
+}
+
 }  // namespace
 
 cudaError_t capture_batch_iteration(const WaveView& w, const BatchView& b, const uint32_t* sobol,
-                                    const LaunchConfig& cfg, unsigned class_mask, bool waves, cudaGraphConditionalHandle cond, cudaStream_t stream,
-                                    cudaGraph_t body) {
+                                    const LaunchConfig& cfg, unsigned class_mask, cudaGraphConditionalHandle cond,
+                                    cudaStream_t stream, cudaGraph_t body) {
   cudaError_t e = cudaStreamBeginCaptureToGraph(stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return e;
-  enqueue_iteration(w, b, sobol, cfg, class_mask, waves, cond, 1, stream, nullptr);
+  enqueue_iteration(w, b, sobol, cfg, class_mask, cond, 1, stream, nullptr);
   cudaGraph_t out = body;
   cudaError_t e2 = cudaStreamEndCapture(stream, &out);
   cudaError_t e3 = cudaGetLastError();
@@ -441,14 +513,77 @@ cudaError_t capture_batch_iteration(const WaveView& w, const BatchView& b, const
 }
 
 void launch_batch_iteration(const WaveView& w, const BatchView& b, const uint32_t* sobol, const LaunchConfig& cfg,
-                            unsigned class_mask, bool waves, cudaStream_t stream, StageTimer* timer) {
-  enqueue_iteration(w, b, sobol, cfg, class_mask, waves, cudaGraphConditionalHandle{}, 0, stream, timer);
+                            unsigned class_mask, cudaStream_t stream, StageTimer* timer) {
+  enqueue_iteration(w, b, sobol, cfg, class_mask, cudaGraphConditionalHandle{}, 0, stream, timer);
 }
 
-void launch_batch_wave_begin(const WaveView& w, const BatchView& b, const uint32_t* sobol,
-                             unsigned long long base, int n, int iteration_cap, int num_sms, cudaStream_t stream) {
-  k_b_wave_begin<<<1, 32, 0, stream>>>(b, n, iteration_cap);
-  k_b_wave_camera<<<grid_cap(n, 256, num_sms * 32), 256, 0, stream>>>(w, b, sobol, base, n);
+void launch_batch_wave(const WaveView& w, const BatchView& b, const uint32_t* sobol, const LaunchConfig& cfg,
+                       unsigned class_mask, unsigned long long base, int n, int bounces, bool complete,
+                       cudaStream_t stream, int64_t* launches, StageTimer* timer) {
+  const WaveView bw = batch_view(w, b);
+  const bool append = n <= kAppendPaths;
+  const int persistent = cfg.num_sms * cfg.blocks_per_sm;
+  const int tgrid = grid_cap(n, cfg.trace_block, persistent);
+  const int sgrid = grid_cap(n, cfg.shade_block, persistent * 2);
+  const int cgrid = grid_cap(n, kCompactSpan, cfg.num_sms * 8);
+  int64_t nl = 0;
+  auto timed = [&](int st, auto&& launch) {
+    if (timer) timer->begin(st, stream);
+    nl += launch();
+    if (timer) timer->end(stream);
+  };
+  timed(ST_CAMERA, [&] {
+    k_wb_camera<<<grid_cap(n, 256, cfg.num_sms * 32), 256, 0, stream>>>(bw, b, sobol, base, n);
+    return 1;
+  });
+  int cur = 0;
+  for (int bounce = 0; bounce < bounces; ++bounce, cur ^= 1) {
+    if (!timer) {
+      b_trace(cfg, bw, b, bounce > 0 ? TK_ALL : TK_EXT, cur, tgrid, !append, stream);
+      ++nl;
+    } else {  // timed: kind by kind
+      const int stage[3] = {ST_TRACE_EXT, ST_TRACE_SHADOW, ST_TRACE_MIS};
+      const int kinds[3] = {TK_EXT, TK_SHADOW, TK_MIS | TK_MIS_ENV};
+      for (int k = 0; k < (bounce > 0 ? 3 : 1); ++k)
+        timed(stage[k], [&] {
+          b_trace(cfg, bw, b, kinds[k], cur, tgrid, !append, stream);
+          return 1;
+        });
+    }
+    if (bounce > 0)
+      timed(ST_RESOLVE, [&] {
+        k_b_resolve<<<sgrid, cfg.shade_block, 0, stream>>>(bw, b, cur);
+        return 1;
+      });
+    const int* list = bw.q_ext[cur];
+    const int* count = bw.counters + cnt_rays(RK_EXT, cur);
+    if (!append)
+      timed(ST_OTHER, [&] {
+        CompactTargets tg{};
+        for (int c = 0; c < kShadeClasses; ++c)
+          tg.queue[c] = bw.q_cls + (size_t)c * bw.capacity, tg.counter[c] = bw.counters + cnt_cls(c, cur);
+        k_wb_compact<kShadeClasses><<<cgrid, kCompactThreads, 0, stream>>>(bw.qflags, list, count, tg);
+        return 1;
+      });
+    timed(ST_SHADE, [&] {
+      return launch_wb_shading(bw, b, sobol, class_mask, cur, append, sgrid, cfg.shade_block, stream);
+    });
+    if (!append && !(complete && bounce + 1 == bounces))  // no path goes on after the last bounce
+      timed(ST_OTHER, [&] {
+        CompactTargets tg{};
+        int* qs[5] = {bw.q_ext[cur ^ 1], bw.q_mis, bw.q_sh, bw.q_mis_env, bw.q_nee};  // as the QueueFlag bits
+        for (int k = 0; k < 5; ++k)
+          tg.queue[k] = qs[k],
+          tg.counter[k] = bw.counters + (k < kRayKinds ? cnt_rays(k, cur ^ 1) : CNT_NEE + (cur ^ 1));
+        k_wb_compact<5><<<cgrid, kCompactThreads, 0, stream>>>(bw.qflags, list, count, tg);
+        return 1;
+      });
+  }
+  timed(ST_FILM, [&] {
+    k_wb_film<<<grid_cap(n, kWbFilmThreads, cfg.num_sms * 8), kWbFilmThreads, 0, stream>>>(bw, b, base, n, complete ? -1 : cur);
+    return 1;
+  });
+  if (launches) *launches += nl;
 }
 
 // FP64 film sums rounded to FP32 (orion_job.sum32).
@@ -460,10 +595,6 @@ __global__ void k_film_to_f32(const double* __restrict__ src, float* __restrict_
 void launch_film_to_f32(const double* src, float* dst, long long n, int num_sms, cudaStream_t stream) {
   const long long blocks = std::min<long long>((n + 255) / 256, (long long)num_sms * 8);
   k_film_to_f32<<<(int)std::max<long long>(blocks, 1), 256, 0, stream>>>(src, dst, n);
-}
-
-void launch_batch_wave_film(const WaveView& w, const BatchView& b, int n, int num_sms, cudaStream_t stream) {
-  k_b_wave_film<<<grid_cap(n, 256, num_sms * 32), 256, 0, stream>>>(w, b, n);
 }
 
 }  // namespace orion_gb300

@@ -29,9 +29,9 @@ static cudaStream_t engine_stream(orion_gpu_ctx* ctx, int e) { return e == 0 ? c
 // The captured loop launches the shading kernels of the classes in `mask`;
 // a graph that launches a superset is reused (an absent class's kernel
 // finds an empty queue), so the mask of a long-lived context only grows.
-static int build_batch_graph(orion_gpu_ctx* ctx, int e, int mode, const BatchView& bv, int slots, unsigned mask) {
+static int build_batch_graph(orion_gpu_ctx* ctx, int e, const BatchView& bv, int slots, unsigned mask) {
   BatchEngine& eng = ctx->beng[e];
-  BatchGraph& be = eng.loop[mode];
+  BatchGraph& be = eng.loop;
   Wave& wave = engine_wave(ctx, e);
   const void* key[4] = {wave.block.p, eng.jobs.p, eng.retire.p, eng.ctl.p};
   bool same = be.exec && be.slots == slots && std::memcmp(key, be.key, sizeof(key)) == 0 &&
@@ -53,7 +53,8 @@ static int build_batch_graph(orion_gpu_ctx* ctx, int e, int mode, const BatchVie
   cudaGraphNode_t node;
   CUDA_TRY(cudaGraphAddNode(&node, be.graph, nullptr, nullptr, 0, &np));
   cudaGraph_t body = np.conditional.phGraph_out[0];
-  cudaError_t ce = capture_batch_iteration(wave.view, bv, ctx->sobol.as<uint32_t>(), ctx->cfg, mask, mode == ORION_BATCH_WAVES, cond, engine_stream(ctx, e), body);
+  cudaError_t ce =
+      capture_batch_iteration(wave.view, bv, ctx->sobol.as<uint32_t>(), ctx->cfg, mask, cond, engine_stream(ctx, e), body);
   if (ce != cudaSuccess) {
     // A graph whose loop-body capture was invalidated is dropped, not
     // destroyed: nothing is assumed about its state after the failure.
@@ -157,7 +158,7 @@ static int run_batch_pooled_locked(orion_gpu_ctx* ctx, std::vector<DevJob>& dj, 
                                                          std::max<unsigned long long>(gtotal[e], 1024ULL));
     if ((rc = prepare_engine(ctx, e, (int)group[e].size(), slots, &bvs[e], &caps[e])) != ORION_OK) return rc;
     for (const DevJob& J : group[e]) masks[e] |= J.scene.class_mask;
-    if (!ctx->profiling && (rc = build_batch_graph(ctx, e, ORION_BATCH_POOLED, bvs[e], caps[e], masks[e])) != ORION_OK)
+    if (!ctx->profiling && (rc = build_batch_graph(ctx, e, bvs[e], caps[e], masks[e])) != ORION_OK)
       return rc;
   }
   cudaStream_t s = ctx->stream;
@@ -192,8 +193,7 @@ static int run_batch_pooled_locked(orion_gpu_ctx* ctx, std::vector<DevJob>& dj, 
     StageTimer timer{ctx->prof_events.data(), ctx->prof_stage.data(), need, 0};
     int more = 1;
     for (int it = 0; more && it < init[0].max_iterations; ++it) {
-      launch_batch_iteration(ctx->wave.view, bvs[0], ctx->sobol.as<uint32_t>(), ctx->cfg, masks[0], false, s,
-                             &timer);
+      launch_batch_iteration(ctx->wave.view, bvs[0], ctx->sobol.as<uint32_t>(), ctx->cfg, masks[0], s, &timer);
       CUDA_TRY(cudaGetLastError());
       CUDA_TRY(cudaMemcpyAsync(&more, &bvs[0].ctl->more, sizeof(int), cudaMemcpyDeviceToHost, s));
       CUDA_TRY(cudaStreamSynchronize(s));
@@ -208,7 +208,7 @@ static int run_batch_pooled_locked(orion_gpu_ctx* ctx, std::vector<DevJob>& dj, 
     }
   } else {
     for (int e = 0; e < ng; ++e)
-      CUDA_TRY(cudaGraphLaunch(ctx->beng[e].loop[ORION_BATCH_POOLED].exec, engine_stream(ctx, e)));
+      CUDA_TRY(cudaGraphLaunch(ctx->beng[e].loop.exec, engine_stream(ctx, e)));
     for (int e = 1; e < ng; ++e) {
       CUDA_TRY(cudaEventRecord(ctx->ev_join[e - 1], engine_stream(ctx, e)));
       CUDA_TRY(cudaStreamWaitEvent(s, ctx->ev_join[e - 1], 0));
@@ -235,7 +235,7 @@ static int run_batch_pooled_locked(orion_gpu_ctx* ctx, std::vector<DevJob>& dj, 
     }
     error_bits |= o.error;
     // Per iteration: plan, regen, 4 traces, one shade per class, resolve, retire, control; plus the init.
-    const unsigned launched = ctx->profiling ? masks[e] : ctx->beng[e].loop[ORION_BATCH_POOLED].mask;
+    const unsigned launched = ctx->profiling ? masks[e] : ctx->beng[e].loop.mask;
     launches += (9LL + __builtin_popcount(launched)) * o.iterations + 1;
   }
   out.error = error_bits;
@@ -260,18 +260,22 @@ static int run_batch_waves_locked(orion_gpu_ctx* ctx, std::vector<DevJob>& dj, u
                                   int max_depth_all, BatchCtl* out_ctl, float* ms_out) {
   const int njobs = (int)dj.size();
   int rc;
-  const int64_t wave = std::max<int64_t>(1024, std::min<int64_t>(ctx->default_batch_slots, (int64_t)total));
+  // As many waves as the slots ask for, and at least one per engine (none
+  // under 256K paths), all of about the same size, so that the engines'
+  // waves overlap to the end.
+  const int engines = std::min(ctx->batch_engines, (int)orion_gpu_ctx::kBatchEngines);
+  const int64_t slots = std::max<int64_t>(1024, ctx->default_batch_slots);
+  const int64_t want = ctx->profiling ? 1 : std::min<int64_t>(engines, std::max<int64_t>(1, (int64_t)total >> 18));
+  const int64_t pieces = std::max<int64_t>(((int64_t)total + slots - 1) / slots, want);
+  const int64_t wave = std::max<int64_t>(1024, ((int64_t)total + pieces - 1) / pieces);
   const int64_t nwaves = std::max<int64_t>(1, ((int64_t)total + wave - 1) / wave);
-  const int ne = ctx->profiling ? 1 : (int)std::min<int64_t>(std::min(ctx->batch_engines, (int)orion_gpu_ctx::kBatchEngines),
-                                                            nwaves);
+  const int ne = ctx->profiling ? 1 : (int)std::min<int64_t>(engines, nwaves);
   std::vector<BatchView> bvs(ne);
   std::vector<int> caps(ne);
   unsigned mask = 1u << SC_MISS;
   for (const DevJob& J : dj) mask |= J.scene.class_mask;
   for (int e = 0; e < ne; ++e) {
     if ((rc = prepare_engine(ctx, e, njobs, (int)wave, &bvs[e], &caps[e])) != ORION_OK) return rc;
-    if (!ctx->profiling && (rc = build_batch_graph(ctx, e, ORION_BATCH_WAVES, bvs[e], caps[e], mask)) != ORION_OK)
-      return rc;
   }
   cudaStream_t s = ctx->stream;
   std::memset(&ctx->stage_times, 0, sizeof(ctx->stage_times));
@@ -287,15 +291,14 @@ static int run_batch_waves_locked(orion_gpu_ctx* ctx, std::vector<DevJob>& dj, u
     cudaStream_t es = engine_stream(ctx, e);
     CUDA_TRY(cudaMemcpyAsync(bvs[e].jobs, dj.data(), (size_t)njobs * sizeof(DevJob), cudaMemcpyHostToDevice, es));
     CUDA_TRY(cudaMemcpyAsync(bvs[e].ctl, &zero, sizeof(BatchCtl), cudaMemcpyHostToDevice, es));
-    // The queue-compaction bytes start clear (other entry points share the slots' memory).
-    CUDA_TRY(cudaMemsetAsync(engine_wave(ctx, e).view.qflags, 0, (size_t)caps[e], es));
   }
-  // Every live path advances one bounce per iteration: a bound on each wave's loop.
-  const int iteration_cap =
-      ctx->cfg.test_batch_iterations > 0 ? ctx->cfg.test_batch_iterations : 2 * (max_depth_all + 2) + 8;
+  // Bounces 0 .. the deepest job's depth end every path (the test limit cuts waves short).
+  const int all_bounces = max_depth_all + 1;
+  const int bounces =
+      ctx->cfg.test_batch_iterations > 0 ? std::min(ctx->cfg.test_batch_iterations, all_bounces) : all_bounces;
   StageTimer timer{nullptr, nullptr, 0, 0};
   if (ctx->profiling) {
-    const int need = (int)std::min<int64_t>(nwaves * iteration_cap * 10, 200000);
+    const int need = (int)std::min<int64_t>(nwaves * (bounces + 1) * 8, 200000);
     while ((int)ctx->prof_events.size() < 2 * need) {
       cudaEvent_t e;
       CUDA_TRY(cudaEventCreate(&e));
@@ -304,29 +307,15 @@ static int run_batch_waves_locked(orion_gpu_ctx* ctx, std::vector<DevJob>& dj, u
     ctx->prof_stage.resize(need);
     timer = StageTimer{ctx->prof_events.data(), ctx->prof_stage.data(), need, 0};
   }
+  int64_t launches = 0;
   for (int64_t k = 0; k < nwaves; ++k) {
     const int e = (int)(k % ne);
     cudaStream_t es = engine_stream(ctx, e);
     const WaveView& wv = engine_wave(ctx, e).view;
     const unsigned long long base = (unsigned long long)(k * wave);
     const int n = (int)std::min<unsigned long long>((unsigned long long)wave, total - base);
-    if (ctx->profiling) timer.begin(ST_CAMERA, es);
-    launch_batch_wave_begin(wv, bvs[e], ctx->sobol.as<uint32_t>(), base, n, iteration_cap, ctx->num_sms, es);
-    if (ctx->profiling) timer.end(es);
-    if (ctx->profiling) {
-      int more = 1;
-      for (int it = 0; more && it < iteration_cap; ++it) {
-        launch_batch_iteration(wv, bvs[e], ctx->sobol.as<uint32_t>(), ctx->cfg, mask, true, es, &timer);
-        CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(cudaMemcpyAsync(&more, &bvs[e].ctl->more, sizeof(int), cudaMemcpyDeviceToHost, es));
-        CUDA_TRY(cudaStreamSynchronize(es));
-      }
-    } else {
-      CUDA_TRY(cudaGraphLaunch(ctx->beng[e].loop[ORION_BATCH_WAVES].exec, es));
-    }
-    if (ctx->profiling) timer.begin(ST_FILM, es);
-    launch_batch_wave_film(wv, bvs[e], n, ctx->num_sms, es);
-    if (ctx->profiling) timer.end(es);
+    launch_batch_wave(wv, bvs[e], ctx->sobol.as<uint32_t>(), ctx->cfg, mask, base, n, bounces, bounces == all_bounces, es,
+                      &launches, ctx->profiling ? &timer : nullptr);
     CUDA_TRY(cudaGetLastError());
   }
   for (int e = 1; e < ne; ++e) {
@@ -349,21 +338,16 @@ static int run_batch_waves_locked(orion_gpu_ctx* ctx, std::vector<DevJob>& dj, u
   }
   BatchCtl& out = *out_ctl;
   out = outs[0];
-  int64_t launches = 0;
   int error_bits = 0;
   for (int e = 0; e < ne; ++e) {
     const BatchCtl& o = outs[e];
     if (e > 0) {
       out.paths_done += o.paths_done;
       for (int j = 0; j < 3; ++j) out.rays[j] += o.rays[j];
-      out.iterations += o.iterations;
     }
     error_bits |= o.error;
-    // Per iteration: plan, 4 traces, 2 queue compactions, one shade per class, resolve, control.
-    const unsigned launched = ctx->profiling ? mask : ctx->beng[e].loop[ORION_BATCH_WAVES].mask;
-    launches += (9LL + __builtin_popcount(launched)) * o.iterations;
   }
-  launches += 3 * nwaves;  // begin, camera, film per wave
+  out.iterations = (int)std::min<int64_t>(nwaves * bounces, INT32_MAX);
   out.error = error_bits;
   ctx->last.paths = (int64_t)out.paths_done;
   ctx->last.ext_rays = (int64_t)out.rays[0];
@@ -418,6 +402,7 @@ static int plan_batch(orion_gpu_ctx* ctx, int32_t njobs, const orion_job* jobs, 
     const long long wh = (long long)J.width * J.height;
     J.first_index = p.first_pass * wh;
     J.num_paths = wh * spp;
+    J.spp = spp;
     J.work_begin = (long long)total;
     total += (unsigned long long)J.num_paths;
     max_depth_all = std::max(max_depth_all, J.max_depth);
@@ -640,6 +625,7 @@ int ctx_run_device_jobs(orion_gpu_ctx* ctx, const DeviceFilmJob* jobs, int njobs
     const long long wh = (long long)J.width * J.height;
     J.first_index = p.first_pass * wh;
     J.num_paths = wh * spp;
+    J.spp = spp;
     J.work_begin = (long long)total;
     total += (unsigned long long)J.num_paths;
     max_depth_all = std::max(max_depth_all, J.max_depth);

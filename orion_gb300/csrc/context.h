@@ -134,7 +134,7 @@ struct DeviceScene {
 
 constexpr int kMaxWaveStreams = 4;  // plain-render waves in flight at once
 
-// A captured device-side loop of one batch mode (pooled or waves).
+// The captured device-side loop of pooled batches.
 struct BatchGraph {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -151,14 +151,12 @@ struct BatchGraph {
 };
 
 // One batch engine: its free and retire lists, control block, job table and
-// captured device-side loops (the path slots are a Wave).
+// captured device-side loop (the path slots are a Wave).
 struct BatchEngine {
   DevBuf retire, free_list, ctl, jobs;
   int slots_alloc = 0, jobs_alloc = 0;
-  BatchGraph loop[2];  // [ORION_BATCH_POOLED], [ORION_BATCH_WAVES]
-  void drop_graph() {
-    for (BatchGraph& g : loop) g.drop();
-  }
+  BatchGraph loop;  // pooled mode
+  void drop_graph() { loop.drop(); }
 };
 
 struct Wave {

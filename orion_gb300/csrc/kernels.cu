@@ -30,19 +30,10 @@ namespace orion_gb300 {
 
 namespace {
 
-// The pixel of a wave's local pixel `lp` (WaveArgs): its place in the render's
-// pixel order, which runs through tiles of 8 x 4 pixels, tile row after tile
-// row, row by row within a tile (edge tiles are smaller).
+// The pixel of a wave's local pixel `lp` (WaveArgs).
 __device__ __forceinline__ void wave_pixel(const WaveArgs& a, int lp, int* x, int* y) {
-  const int64_t pos = (((int64_t)(lp >> a.chunk_log2) * a.waves + a.wave) << a.chunk_log2) +
-                      (lp & ((1 << a.chunk_log2) - 1));
-  const uint32_t band_pixels = 4u * (uint32_t)a.width;
-  const int band = pos >> 32 ? (int)(pos / band_pixels) : (int)((uint32_t)pos / band_pixels), y0 = 4 * band;
-  const int rows = min(4, a.height - y0), in_band = (int)(pos - (int64_t)band * band_pixels);
-  const int tile = in_band / (8 * rows), x0 = 8 * tile, cols = min(8, a.width - x0);
-  const int in_tile = in_band - 8 * rows * tile, row = in_tile / cols;
-  *x = x0 + in_tile - row * cols;
-  *y = y0 + row;
+  tile_pixel((((int64_t)(lp >> a.chunk_log2) * a.waves + a.wave) << a.chunk_log2) + (lp & ((1 << a.chunk_log2) - 1)),
+             a.width, a.height, x, y);
 }
 
 __global__ void k_camera(SceneView s, WaveView w, WaveArgs a) {

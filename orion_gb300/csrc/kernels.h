@@ -119,8 +119,8 @@ constexpr int kTestStackEntries = 2;
 // bounce b's trace reads the ray counters of parity b & 1, counts classes
 // under the same parity, and empties the other parity's for the next shading
 // and trace to fill.
-enum CounterSlot { CNT_RAYS = 0 /* + 2 x kind + parity */, CNT_FETCH = 8 /* + kind */, CNT_NEE = 12, CNT_RETIRE = 13,
-                   CNT_FREE = 14, CNT_CLS = 16 /* + 8 x parity + class */, kCounterSlots = 32 };
+enum CounterSlot { CNT_RAYS = 0 /* + 2 x kind + parity */, CNT_FETCH = 8 /* + kind */, CNT_NEE = 12 /* + parity */,
+                   CNT_RETIRE = 14, CNT_FREE = 15, CNT_CLS = 16 /* + 8 x parity + class */, kCounterSlots = 32 };
 ORION_HD constexpr int cnt_rays(int kind, int parity) { return CNT_RAYS + 2 * kind + parity; }
 ORION_HD constexpr int cnt_cls(int sc, int parity) { return CNT_CLS + 8 * parity + sc; }
 static_assert(kShadeClasses <= 8, "two parities of class counters");
@@ -132,7 +132,7 @@ enum TraceKinds { TK_EXT = 1, TK_MIS = 2, TK_SHADOW = 4, TK_MIS_ENV = 8, TK_ALL 
 // ------------------------------------------------------------ batched mode
 //
 // Many render jobs (scenes, views, resolutions, spp, depths) share one pool
-// of path slots. Each loop iteration refills free slots from the global work
+// of path slots (pooled mode; wave mode runs their work list in waves). Each loop iteration refills free slots from the global work
 // list (job by job, sample index by sample index), runs one bounce for every
 // live path, and retires finished paths into their job's FP64 film.
 
@@ -142,6 +142,7 @@ struct DevJob {
   int max_depth, rr_depth;
   long long first_index;  // sample index of the job's first path: k0 * W * H
   long long num_paths;    // W * H * spp
+  int spp;
   long long work_begin;   // offset of the job in the global work list
   double* sum;            // W*H*3
   double* sumsq;          // W*H*3
@@ -314,24 +315,24 @@ struct KernelLimits {
 cudaError_t configure_kernels(int smem_bytes, KernelLimits* lim);
 cudaError_t configure_batch_kernels(int smem_bytes, KernelLimits* lim);
 
-// Batched mode: builds the body of the device-side loop (one iteration)
+// Pooled batches: builds the body of the device-side loop (one iteration)
 // into `body` by stream capture on `stream`. The loop keeps running while
 // work or live paths remain; `cond` is the graph's while-condition handle.
 // Shading kernels are launched for the classes in `class_mask` only.
-// waves: the iteration of wave mode (no refills, no per-iteration film).
 cudaError_t capture_batch_iteration(const WaveView& w, const BatchView& b, const uint32_t* sobol,
-                                    const LaunchConfig& cfg, unsigned class_mask, bool waves,
-                                    cudaGraphConditionalHandle cond, cudaStream_t stream, cudaGraph_t body);
+                                    const LaunchConfig& cfg, unsigned class_mask, cudaGraphConditionalHandle cond,
+                                    cudaStream_t stream, cudaGraph_t body);
 // The same iteration launched directly (a host-driven loop reading ctl->more),
-// each stage timed by `timer`: the profiling path of the batched engine.
+// each stage timed by `timer`: the profiling path of the pooled engine.
 void launch_batch_iteration(const WaveView& w, const BatchView& b, const uint32_t* sobol, const LaunchConfig& cfg,
-                            unsigned class_mask, bool waves, cudaStream_t stream, StageTimer* timer);
-// Wave mode: starts a wave of work items [base, base + n) on slots 0..n-1
-// (at most `iteration_cap` more loop iterations), and after its loop adds
-// the n paths' radiance to their jobs' films.
-void launch_batch_wave_begin(const WaveView& w, const BatchView& b, const uint32_t* sobol,
-                             unsigned long long base, int n, int iteration_cap, int num_sms, cudaStream_t stream);
-void launch_batch_wave_film(const WaveView& w, const BatchView& b, int n, int num_sms, cudaStream_t stream);
+                            unsigned class_mask, cudaStream_t stream, StageTimer* timer);
+// Wave mode: renders the work items [base, base + n) on slots 0..n-1, a plain
+// wave's launches with `bounces` bounces, and adds the radiance of the n paths
+// to their jobs' films. complete: `bounces` is one more than the deepest job's
+// depth, which ends every path (else paths left report kErrIterationCap).
+void launch_batch_wave(const WaveView& w, const BatchView& b, const uint32_t* sobol, const LaunchConfig& cfg,
+                       unsigned class_mask, unsigned long long base, int n, int bounces, bool complete,
+                       cudaStream_t stream, int64_t* launches, StageTimer* timer);
 // dst[i] = (float)src[i] for i < n.
 void launch_film_to_f32(const double* src, float* dst, long long n, int num_sms, cudaStream_t stream);
 // Resets the batch control block and the free-slot list for `capacity` slots.

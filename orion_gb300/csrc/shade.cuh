@@ -43,6 +43,18 @@ __device__ __forceinline__ void class_append(int* counters, int* queues, int str
   queues[(size_t)cls * stride + base + __popc(peers & ((1u << lane) - 1u))] = value;
 }
 
+// Pixel `pos` of a film in tile order: tiles of 8 x 4 pixels, tile row after
+// tile row, row by row within a tile (edge tiles are smaller).
+__device__ __forceinline__ void tile_pixel(int64_t pos, int width, int height, int* x, int* y) {
+  const uint32_t band_pixels = 4u * (uint32_t)width;
+  const int band = pos >> 32 ? (int)(pos / band_pixels) : (int)((uint32_t)pos / band_pixels), y0 = 4 * band;
+  const int rows = min(4, height - y0), in_band = (int)(pos - (int64_t)band * band_pixels);
+  const int tile = in_band / (8 * rows), x0 = 8 * tile, cols = min(8, width - x0);
+  const int in_tile = in_band - 8 * rows * tile, row = in_tile / cols;
+  *x = x0 + in_tile - row * cols;
+  *y = y0 + row;
+}
+
 struct Hit {
   V3 p, ng, ns, su, sv;
 };
@@ -470,12 +482,14 @@ __device__ __forceinline__ void trace_persistent(const SceneOf& scene_of, const 
         const int my = base + __popc(idle & ((1u << lane) - 1u));
         if (my < n) {
           pid = rs.queue[my];
-          const SceneView& s = scene_of(pid);
-          ts = TraceScene{s.nodes, s.woop, s.tri_prim, s.tri_class};
           // The ray and its result pass through once: streaming (evict-first) accesses
           // leave L1 and L2 to the BVH nodes and triangles (displaced sphere +1.2%).
           const int64_t at = (int64_t)pid * rs.stride;
           const float4 o4 = __ldcs(rs.o + at), d4 = __ldcs(rs.d + at);
+          if constexpr (!kUniform) {
+            const SceneView& s = scene_of(pid);
+            ts = TraceScene{s.nodes, s.woop, s.tri_prim, s.tri_class};
+          }
           st.sp = 0;
           lane_start(r, o4, d4, ANY ? o4.w : kFloatMax, ANY);
           active = true;
@@ -558,6 +572,7 @@ __device__ __forceinline__ void trace_kinds(const SceneOf& scene_of, const RaySe
   if (blockIdx.x == 0) {
     if (threadIdx.x < kShadeClasses) counters[cnt_cls(threadIdx.x, cur ^ 1)] = 0;
     if (threadIdx.x < kRayKinds) counters[cnt_rays(threadIdx.x, cur ^ 1)] = 0;
+    if (threadIdx.x == 0) counters[CNT_NEE + (cur ^ 1)] = 0;
     if (threadIdx.x < 4 && ((kinds >> threadIdx.x) & 1))
       atomicAdd(set[threadIdx.x].stat, (unsigned long long)*set[threadIdx.x].count);
   }
