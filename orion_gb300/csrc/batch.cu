@@ -476,10 +476,10 @@ int launch_wb_shading(const WaveView& bw, const BatchView& b, const uint32_t* so
   static const struct {
     int sc;
     Kernel kernel;
-  } kOrder[kShadeClasses] = {{SC_TEXTURED, k_b_shade<SC_TEXTURED>},     {SC_GENERAL, k_b_shade<SC_GENERAL>},
-                             {SC_PLASTIC, k_b_shade<SC_PLASTIC>},       {SC_DIELECTRIC, k_b_shade<SC_DIELECTRIC>},
-                             {SC_CONDUCTOR, k_b_shade<SC_CONDUCTOR>},   {SC_DIFFUSE, k_b_shade<SC_DIFFUSE>},
-                             {SC_SPECULAR, k_b_shade<SC_SPECULAR>},     {SC_MISS, k_b_shade<SC_MISS>}};
+  } kOrder[kShadeClasses] = {{SC_MISS, k_b_shade<SC_MISS>},             {SC_SPECULAR, k_b_shade<SC_SPECULAR>},
+                             {SC_DIFFUSE, k_b_shade<SC_DIFFUSE>},       {SC_CONDUCTOR, k_b_shade<SC_CONDUCTOR>},
+                             {SC_DIELECTRIC, k_b_shade<SC_DIELECTRIC>}, {SC_PLASTIC, k_b_shade<SC_PLASTIC>},
+                             {SC_GENERAL, k_b_shade<SC_GENERAL>},       {SC_TEXTURED, k_b_shade<SC_TEXTURED>}};
   cudaLaunchAttribute early;
   early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   early.val.programmaticStreamSerializationAllowed = 1;
