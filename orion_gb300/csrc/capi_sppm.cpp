@@ -56,7 +56,9 @@ extern "C" int orion_gpu_render_sppm(orion_gpu_ctx* ctx, orion_scene_id id, cons
   pieces.push_back({(void**)&v.film, sizeof(float) * 3 * (size_t)npix});
   pieces.push_back({(void**)&v.film_count, sizeof(unsigned) * (size_t)npix});
   pieces.push_back({(void**)&v.rays, sizeof(unsigned long long)});
-  pieces.push_back({(void**)&v.hit_count, sizeof(int)});
+  pieces.push_back({(void**)&v.hit_count, 2 * sizeof(int)});  // and photon_next
+  const int num_mats = (int)(d.mats.bytes / sizeof(DevMaterial));
+  pieces.push_back({(void**)&v.photon_mats, sizeof(DevMaterial) * (size_t)num_mats});
   size_t total = 0;
   for (const Piece& pc : pieces) total += (pc.bytes + 255) & ~(size_t)255;
   if (ctx->sppm_block.bytes < total) RC(ctx->sppm_block.alloc(total));
@@ -69,6 +71,8 @@ extern "C" int orion_gpu_render_sppm(orion_gpu_ctx* ctx, orion_scene_id id, cons
   }
   v.vp_pr = f4s[0], v.vp_wo = f4s[1], v.vp_beta = f4s[2], v.vp_ns = f4s[3], v.vp_ng = f4s[4];
   v.vp_su = f4s[5], v.vp_sv = f4s[6], v.ld = f4s[7], v.tau = f4s[8];
+  v.photon_next = v.hit_count + 1;
+  v.num_sms = ctx->num_sms;
   v.width = W;
   v.height = H;
   v.npix = (int)npix;
@@ -83,7 +87,7 @@ extern "C" int orion_gpu_render_sppm(orion_gpu_ctx* ctx, orion_scene_id id, cons
   v.by_cell = reinterpret_cast<float4*>(static_cast<char*>(ctx->sppm_hits.p) + hit_bytes);
   v.hits_cap = (int)hits_cap;
 
-  launch_sppm_init(v, p.initial_radius, st);
+  launch_sppm_init(v, p.initial_radius, d.view.mats, num_mats, st);
   CUDA_TRY(cudaMemsetAsync(v.rays, 0, sizeof(unsigned long long), st));
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaEventRecord(ctx->ev0, st));

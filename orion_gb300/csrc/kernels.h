@@ -376,6 +376,9 @@ struct SppmView {
   float4* hits;
   int hits_cap;     // photons x (max depth - 1): every hit after a photon's first
   int* hit_count;
+  DevMaterial* photon_mats;  // the scene's materials with DevLobe::photon set
+  int* photon_next;  // next photon to start (beside hit_count: cleared together)
+  int num_sms;
   // hash cell -> photon hits: cell h holds records [cell_start[h], cell_start[h + 1]) of by_cell
   int* cell_start;  // npix + 1 (counts, then their exclusive scan)
   int* cell_fill;   // npix
@@ -389,8 +392,9 @@ struct SppmView {
 constexpr int kSppmBoundsBlocks = 1024;  // blocks of the bounds pass (part_lo / part_hi entries)
 constexpr int kScanBlock = 1024;         // elements per block of the cell-count scan
 
-// Resets per-pixel state (radius r0, no visible point) and the film.
-void launch_sppm_init(const SppmView& v, float radius0, cudaStream_t stream);
+// Resets per-pixel state (radius r0, no visible point) and the film, and
+// fills photon_mats from the scene's materials.
+void launch_sppm_init(const SppmView& v, float radius0, const DevMaterial* mats, int num_mats, cudaStream_t stream);
 // Camera pass and the grid over the visible points of iteration `iter`.
 void launch_sppm_visible_points(const SceneView& s, const SppmView& v, int iter, cudaStream_t stream);
 // Exclusive scan of the cell counts (cell_start).

@@ -516,4 +516,34 @@ __device__ __forceinline__ bool warp_triangles(LaneRay& r, const TraceScene& s, 
   return found;
 }
 
+// One ray per lane, traced by the whole warp to the end (all 32 lanes call it;
+// lanes without a ray pass on = false): closest hit in (0, FLT_MAX], or ANY,
+// whether anything lies in (0, tmax] (tri >= 0). For kernels that follow a path
+// per lane: out of line, so that their several trace sites share two copies of
+// the traversal. smem: the block's dynamic shared memory, as
+// trace_smem_bytes(SMEM, blockDim.x) lays it out.
+template <bool ANY, int SMEM>
+static __device__ __noinline__ RayHit warp_trace(const float4* nodes, const float4* woop, const int* tri_prim,
+                                                 int2* smem, bool on, V3 o, V3 d, float tmax) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const TraceScene ts{nodes, woop, tri_prim, nullptr};
+  TraversalStack<SMEM> st;
+  st.smem = smem + threadIdx.x;
+  st.stride = blockDim.x;
+  st.sp = 0;
+  TriScratch* sc = reinterpret_cast<TriScratch*>(smem + (size_t)SMEM * blockDim.x) + (threadIdx.x >> 5);
+  LaneRay r;
+  lane_start(r, make_float4(o.x, o.y, o.z, 0.f), make_float4(d.x, d.y, d.z, 0.f), ANY ? tmax : kFloatMax, ANY);
+  __syncwarp();
+  while (__any_sync(kFull, on)) {
+    if (on) lane_visit<ANY, SMEM>(r, ts, st, nullptr);
+    const bool occl = warp_triangles<ANY, false, true>(r, ts, sc, nullptr);
+    if (on && ((ANY && occl) || lane_pop(r, st))) {
+      on = false;
+      r.tg.y = 0u;
+    }
+  }
+  return RayHit{r.tmax, r.u, r.v, r.tri};
+}
+
 }  // namespace orion_gb300
