@@ -577,7 +577,7 @@ struct WideCollapser {
         e = std::max(-126, std::min(112, m == 0.5 ? ex - 1 : ex));
       }
       while (e < 112 && std::ldexp(255.0, e) < ext) ++e;  // guards the rounding of ext / 255
-      w.e[k] = (uint8_t)(e + 127);
+      w.e[k] = (uint8_t)(e + 127 + 15);
       cell[k] = std::ldexp(1.0, e);
     }
     // Internal children first (their node slots), then leaf triangles.
@@ -694,7 +694,7 @@ void build_bvh(const float* positions, int64_t num_tris, const BvhBuildOptions& 
     WideNode empty;
     std::memset(&empty, 0, sizeof(empty));  // no slot in use, inverted boxes: nothing hits
     std::memset(empty.qlo, 0xff, sizeof(empty.qlo));
-    for (int k = 0; k < 3; ++k) empty.e[k] = 127;
+    for (int k = 0; k < 3; ++k) empty.e[k] = 127 + 15;
     out->wide.push_back(empty);
     return;
   }

@@ -196,7 +196,9 @@ struct BvhNode {
 
 // One node of the 8-wide BVH the kernels traverse: 80 bytes = 5 x float4.
 // Child boxes are quantised to 8 bits per bound on a per-axis grid of
-// power-of-two cells anchored at `p`: bound = p + q * 2^(e - 127).
+// power-of-two cells anchored at `p`: bound = p + q * cell, cell = 2^(e - 142)
+// (e is the float exponent of 2^15 cells, which is what the traversal scales
+// the ray by).
 // Internal children are stored contiguously from child_base in slot order;
 // the triangles of all leaf children contiguously from tri_base.
 // meta[s]: 0 = empty slot; internal child: 0x80; leaf child:
@@ -207,7 +209,7 @@ struct BvhNode {
 // roughly near to far.
 struct WideNode {
   float p[3];
-  uint8_t e[3];        // biased exponent of the cell size per axis
+  uint8_t e[3];        // biased exponent of 2^15 x the cell size per axis
   uint8_t imask;       // bit s: slot s holds an internal child
   int32_t child_base;
   int32_t tri_base;
