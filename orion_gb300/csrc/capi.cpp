@@ -864,6 +864,38 @@ extern "C" int orion_gpu_sobol(orion_gpu_ctx* ctx, int64_t n, const uint64_t* in
   return ORION_OK;
 }
 
+namespace {
+// A ray query's rays (8 floats each) and results (4 words) on the device, in
+// one piece, up to 64 MB of it from the context's pool: no device-wide
+// cudaMalloc / cudaFree per query.
+struct QueryBuffers {
+  DevBuf ws;
+  float *rays = nullptr, *t = nullptr, *u = nullptr, *v = nullptr;
+  int* prim = nullptr;
+  int load(orion_gpu_ctx* ctx, int64_t n, const float* host) {
+    const size_t bytes = 48 * (size_t)n;
+    if (bytes <= ((size_t)64 << 20))
+      RC(ws.alloc_pooled(bytes, ctx->scene_pool, ctx->stream));
+    else
+      RC(ws.alloc(bytes));
+    rays = ws.as<float>();
+    t = rays + 8 * n, u = t + n, v = u + n;
+    prim = reinterpret_cast<int*>(v + n);
+    if (n) CUDA_TRY(cudaMemcpyAsync(rays, host, 32 * (size_t)n, cudaMemcpyHostToDevice, ctx->stream));
+    return ORION_OK;
+  }
+  int store(orion_gpu_ctx* ctx, int64_t n, float* ht, float* hu, float* hv, int32_t* hp) {
+    if (n == 0) return ORION_OK;
+    const size_t bytes = 4 * (size_t)n;
+    CUDA_TRY(cudaMemcpyAsync(ht, t, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    CUDA_TRY(cudaMemcpyAsync(hu, u, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    CUDA_TRY(cudaMemcpyAsync(hv, v, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    CUDA_TRY(cudaMemcpyAsync(hp, prim, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    return ORION_OK;
+  }
+};
+}  // namespace
+
 extern "C" int orion_gpu_trace(orion_gpu_ctx* ctx, orion_scene_id id, int64_t n, const float* rays, int32_t any_hit,
                                float* t, float* u, float* v, int32_t* prim) {
   if (!ctx || n < 0 || (n > 0 && (!rays || !t || !u || !v || !prim))) return fail(ORION_ERR_INVALID, "bad argument");
@@ -871,19 +903,11 @@ extern "C" int orion_gpu_trace(orion_gpu_ctx* ctx, orion_scene_id id, int64_t n,
   CUDA_TRY(cudaSetDevice(ctx->device));
   auto it = ctx->scenes.find(id);
   if (it == ctx->scenes.end()) return fail(ORION_ERR_INVALID, "unknown scene id");
-  DevBuf dr, dt, du, dv, dp;
-  RC(to_device(dr, rays, 8 * (size_t)n, ctx->stream));
-  RC(dt.alloc(n * 4));
-  RC(du.alloc(n * 4));
-  RC(dv.alloc(n * 4));
-  RC(dp.alloc(n * 4));
-  launch_trace(it->second->view, n, dr.as<float>(), any_hit, dt.as<float>(), du.as<float>(), dv.as<float>(),
-               dp.as<int>(), ctx->cfg, ctx->stream);
+  QueryBuffers q;
+  RC(q.load(ctx, n, rays));
+  launch_trace(it->second->view, n, q.rays, any_hit, q.t, q.u, q.v, q.prim, ctx->cfg, ctx->stream);
   CUDA_TRY(cudaGetLastError());
-  RC(to_host(t, dt, n, ctx->stream));
-  RC(to_host(u, du, n, ctx->stream));
-  RC(to_host(v, dv, n, ctx->stream));
-  RC(to_host(prim, dp, n, ctx->stream));
+  RC(q.store(ctx, n, t, u, v, prim));
   CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   return ORION_OK;
 }
@@ -902,21 +926,13 @@ extern "C" int orion_gpu_trace_wave(orion_gpu_ctx* ctx, orion_scene_id id, int64
   if (n == 0) return ORION_OK;
   RC(ensure_wave(ctx, (int)n));
   const WaveView& w = ctx->wave.view;
-  DevBuf dr, dt, du, dv, dp;
-  RC(to_device(dr, rays, 8 * (size_t)n, ctx->stream));
-  RC(dt.alloc(n * 4));
-  RC(du.alloc(n * 4));
-  RC(dv.alloc(n * 4));
-  RC(dp.alloc(n * 4));
+  QueryBuffers q;
+  RC(q.load(ctx, n, rays));
   CUDA_TRY(cudaMemsetAsync(w.error_word, 0, sizeof(int), ctx->stream));
-  launch_trace_wave(it->second->view, w, (int)n, dr.as<float>(), any_hit, dt.as<float>(), du.as<float>(),
-                    dv.as<float>(), dp.as<int>(), ctx->cfg, ctx->stream);
+  launch_trace_wave(it->second->view, w, (int)n, q.rays, any_hit, q.t, q.u, q.v, q.prim, ctx->cfg, ctx->stream);
   CUDA_TRY(cudaGetLastError());
   int err_word = 0;
-  RC(to_host(t, dt, n, ctx->stream));
-  RC(to_host(u, du, n, ctx->stream));
-  RC(to_host(v, dv, n, ctx->stream));
-  RC(to_host(prim, dp, n, ctx->stream));
+  RC(q.store(ctx, n, t, u, v, prim));
   CUDA_TRY(cudaMemcpyAsync(&err_word, w.error_word, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   if (err_word) return fail(ORION_ERR_DEVICE, kernel_error(err_word));

@@ -340,6 +340,7 @@ struct LaneRay {
   int tri, best_prim;
   uint32_t oct;
   uint2 ng, tg;
+  float tnear;  // ray queries only (TNEAR)
 };
 
 // any: an occlusion ray (its node groups list children far to near, lane_visit).
@@ -365,7 +366,8 @@ struct TraceWork {
 // and the triangles of its hit leaves (r.tg). COUNT adds the visit to `wk`.
 // A push beyond the stack's capacity poisons the ray (r.tmax = -1; see the
 // file comment): the caller reports it when the ray is done.
-template <bool ANY, int SMEM, bool COUNT = false, int CAP = kMaxStack>
+// TNEAR: hits begin beyond r.tnear, not 0.
+template <bool ANY, int SMEM, bool COUNT = false, int CAP = kMaxStack, bool TNEAR = false>
 __device__ __forceinline__ void lane_visit(LaneRay& r, const TraceScene& s, TraversalStack<SMEM, CAP>& st,
                                            TraceWork* wk) {
   if (r.ng.y > 0x00ffffffu) {
@@ -376,7 +378,7 @@ __device__ __forceinline__ void lane_visit(LaneRay& r, const TraceScene& s, Trav
     const uint32_t ord = ANY ? (r.oct ^ 7u) : r.oct;
     const int child = take_child(r.ng, ord);
     if (r.ng.y && !st.push(make_int2((int)r.ng.x, (int)r.ng.y))) r.tmax = -1.f;
-    wide_node(s.nodes, child, r.o, r.idir, r.oct, 0.f, r.tmax, r.ng, r.tg, ord);
+    wide_node(s.nodes, child, r.o, r.idir, r.oct, TNEAR ? r.tnear : 0.f, r.tmax, r.ng, r.tg, ord);
     if (COUNT) ++wk->nodes;
   } else {
     r.tg = r.ng;
@@ -440,41 +442,49 @@ constexpr int kDealClosest = 4, kDealAny = 3;
 // each owner keeps the least (t, primID) of its hits in (0, tmax] or, ANY,
 // any hit. UNIFORM: every lane traces the same scene (otherwise each pair
 // uses its owner's triangle arrays). Returns true for an ANY lane whose ray
-// hit.
-template <bool ANY, bool COUNT, bool UNIFORM>
+// hit. TNEAR: hits begin beyond r.tnear; a lane whose r.tnear is negative tests
+// its triangles itself (the packed keys order non-negative distances only).
+template <bool ANY, bool COUNT, bool UNIFORM, bool TNEAR = false>
 __device__ __forceinline__ bool warp_triangles(LaneRay& r, const TraceScene& s, TriScratch* sc, TraceWork* wk) {
   constexpr unsigned kFull = 0xffffffffu;
   constexpr int kDeal = ANY ? kDealAny : kDealClosest;
   const int lane = threadIdx.x & 31;
   bool found = false;
+  auto one_by_one = [&]() {
+    while (r.tg.y != 0u) {
+      const int k = (int)r.tg.x + __ffs(r.tg.y) - 1;
+      r.tg.y &= r.tg.y - 1u;
+      float t, u, v;
+      if (COUNT) ++wk->tris;
+      if (woop_hit(s.woop, k, r.o, r.d, TNEAR ? r.tnear : 0.f, r.tmax, &t, &u, &v)) {
+        if (ANY) {
+          r.tri = k;
+          r.tg.y = 0u;
+          found = true;
+          break;
+        }
+        const int prim = __ldg(s.tri_prim + k);
+        if (t < r.tmax || r.tri < 0 || prim < r.best_prim) {
+          r.tmax = t;
+          r.u = u;
+          r.v = v;
+          r.tri = k;
+          r.best_prim = prim;
+        }
+      }
+    }
+  };
+  if constexpr (TNEAR) {
+    if (r.tnear < 0.f) one_by_one();
+    __syncwarp();
+  }
   while (true) {
     if (!__any_sync(kFull, r.tg.y != 0u)) break;
     const int c = __popc(r.tg.y);
     const int total = (int)__reduce_add_sync(kFull, (unsigned)c);
     if (total == 0) break;
     if ((int)__reduce_max_sync(kFull, (unsigned)c) < kDeal * ((total + 31) >> 5)) {
-      while (r.tg.y != 0u) {  // one by one
-        const int k = (int)r.tg.x + __ffs(r.tg.y) - 1;
-        r.tg.y &= r.tg.y - 1u;
-        float t, u, v;
-        if (COUNT) ++wk->tris;
-        if (woop_hit(s.woop, k, r.o, r.d, 0.f, r.tmax, &t, &u, &v)) {
-          if (ANY) {
-            r.tri = k;
-            r.tg.y = 0u;
-            found = true;
-            break;
-          }
-          const int prim = __ldg(s.tri_prim + k);
-          if (t < r.tmax || r.tri < 0 || prim < r.best_prim) {
-            r.tmax = t;
-            r.u = u;
-            r.v = v;
-            r.tri = k;
-            r.best_prim = prim;
-          }
-        }
-      }
+      one_by_one();
       break;
     }
     // Dealt: this lane's pairs are [first, first + c) of the warp's list.
@@ -498,6 +508,8 @@ __device__ __forceinline__ bool warp_triangles(LaneRay& r, const TraceScene& s, 
     const float oz = __shfl_sync(kFull, r.o.z, ow), dx = __shfl_sync(kFull, r.d.x, ow);
     const float dy = __shfl_sync(kFull, r.d.y, ow), dz = __shfl_sync(kFull, r.d.z, ow);
     const float tmax = __shfl_sync(kFull, r.tmax, ow);
+    float tnear = 0.f;
+    if constexpr (TNEAR) tnear = __shfl_sync(kFull, r.tnear, ow);
     const uint32_t obase = __shfl_sync(kFull, r.tg.x, ow), omask = __shfl_sync(kFull, r.tg.y, ow);
     const float4* woop = s.woop;
     const int* tri_prim = s.tri_prim;
@@ -510,7 +522,7 @@ __device__ __forceinline__ bool warp_triangles(LaneRay& r, const TraceScene& s, 
     int k = 0;
     if (lane < total) {
       k = (int)(obase + nth_set_bit(omask, (uint32_t)(lane - seg)));
-      hit = woop_hit(woop, k, V3{ox, oy, oz}, V3{dx, dy, dz}, 0.f, tmax, &t, &u, &v);
+      hit = woop_hit(woop, k, V3{ox, oy, oz}, V3{dx, dy, dz}, tnear, tmax, &t, &u, &v);
     }
     const unsigned span = dealt == 32 ? kFull : (((1u << dealt) - 1u) << (first & 31));
     if (ANY) {
