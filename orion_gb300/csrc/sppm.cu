@@ -127,7 +127,7 @@ __device__ V3 sppm_direct(const SceneView& s, const Tracer& tr, bool on, const D
     const bool occ = tr.occluded(want, o, dir, 1.f - kShadowEpsilon);
     if (want && !occ) Ld = part;
   }
-  bool want_env = false, want_area = false;
+  bool want_mis = false, env = false;
   V3 fb = V3{0, 0, 0};
   float mis_pdf = 0.f, wgt = 0.f;
   if (on && !is_delta_light(lt.kind)) {
@@ -136,37 +136,38 @@ __device__ V3 sppm_direct(const SceneView& s, const Tracer& tr, bool on, const D
     fb = fb * absdot(dir, h.ns);
     if (!is_black(fb) && mis_pdf > 0.f) {
       o = offset_ray_origin(h.p, h.ng, dir);
-      if (lt.kind == DL_ENV) {
+      env = lt.kind == DL_ENV;
+      want_mis = true;
+      if (env) {
         const float lpdf = env_pdf_li(lt, s.envmaps, dir);
-        if (lpdf != 0.f) {
+        if (lpdf != 0.f)
           wgt = power_heuristic(mis_pdf, lpdf);
-          want_env = true;
-          ++*rays;
-        }
-      } else {
-        want_area = true;
-        ++*rays;
+        else
+          want_mis = false;
       }
+      *rays += want_mis ? 1u : 0u;
     }
   }
-  if (__syncthreads_or(want_env)) {
-    const bool occ = tr.occluded(want_env, o, dir, kFloatMax);
-    if (want_env && !occ) Ld = Ld + sdiv(mul(fb, env_le(lt, s.envmaps, dir)) * wgt, mis_pdf);
-  }
-  if (__syncthreads_or(want_area)) {
-    const RayHit mh = tr.closest(want_area, o, dir);
-    const int prim = want_area && mh.tri >= 0 ? __ldg(s.tri_prim + mh.tri) : -1;
-    if (prim >= 0 && prim == lt.prim) {
-      // Triangle::pdf (src/core/triangle.cpp:123-135) on the traced hit.
-      const PrimShade& sh = s.prims[prim];
-      const V3 ip = point_on(sh, mh.u, mh.v);
-      const V3 ing = geometric_normal(sh);
-      float lpdf = length_sq(h.p - ip) / (absdot(ing, -dir) * lt.area);
-      if (isinf(lpdf)) lpdf = 0.f;
-      if (lpdf != 0.f) {
-        const float w = power_heuristic(mis_pdf, lpdf);
-        const V3 Li = dot(ing, -dir) > 0.f ? ld3(lt.L) : V3{0, 0, 0};
-        if (!is_black(Li)) Ld = Ld + sdiv(mul(fb, Li) * w, mis_pdf);
+  // Towards an area light the closest hit is needed; rays towards the
+  // environment, for which any hit would do, go along.
+  if (__syncthreads_or(want_mis)) {
+    const RayHit mh = tr.closest(want_mis, o, dir);
+    if (want_mis && env) {
+      if (mh.tri < 0) Ld = Ld + sdiv(mul(fb, env_le(lt, s.envmaps, dir)) * wgt, mis_pdf);
+    } else if (want_mis) {
+      const int prim = mh.tri >= 0 ? __ldg(s.tri_prim + mh.tri) : -1;
+      if (prim >= 0 && prim == lt.prim) {
+        // Triangle::pdf (src/core/triangle.cpp:123-135) on the traced hit.
+        const PrimShade& sh = s.prims[prim];
+        const V3 ip = point_on(sh, mh.u, mh.v);
+        const V3 ing = geometric_normal(sh);
+        float lpdf = length_sq(h.p - ip) / (absdot(ing, -dir) * lt.area);
+        if (isinf(lpdf)) lpdf = 0.f;
+        if (lpdf != 0.f) {
+          const float w = power_heuristic(mis_pdf, lpdf);
+          const V3 Li = dot(ing, -dir) > 0.f ? ld3(lt.L) : V3{0, 0, 0};
+          if (!is_black(Li)) Ld = Ld + sdiv(mul(fb, Li) * w, mis_pdf);
+        }
       }
     }
   }
@@ -532,9 +533,24 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_parts(int* part, int nparts
   }
 }
 
-__global__ void __launch_bounds__(kScanBlock) k_scan_add(int* a, int n, const int* part) {
+// raw: `part` holds the blocks' sums, not their scan: each block adds up those
+// before it itself (one launch less, while there are few).
+constexpr int kScanRaw = 4 * kScanBlock;
+
+__global__ void __launch_bounds__(kScanBlock) k_scan_add(int* a, int n, const int* part, int raw) {
+  __shared__ int warp_sum[32];
   const int i = blockIdx.x * kScanBlock + threadIdx.x;
-  if (i < n) a[i] += part[blockIdx.x];
+  int before = 0;
+  if (raw) {
+    for (int k = threadIdx.x; k < blockIdx.x; k += kScanBlock) before += part[k];
+    before = (int)__reduce_add_sync(0xffffffffu, (unsigned)before);
+    if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = before;
+    __syncthreads();
+    before = (int)__reduce_add_sync(0xffffffffu, (unsigned)warp_sum[threadIdx.x & 31]);
+  } else {
+    before = part[blockIdx.x];
+  }
+  if (i < n) a[i] += before;
 }
 
 // Photons (sppm.cpp:197-270). Warps stay in the loop: each turn traces one
@@ -648,6 +664,17 @@ __global__ void __launch_bounds__(kPhotonBlock, 2) k_sppm_photons(SceneView s, S
   count_rays(v.rays, rays);
 }
 
+// Empties hash cell `pix` (there are as many as pixels) and the photon counters.
+__device__ __forceinline__ void clear_cells(const SppmView& v, int pix) {
+  v.cell_start[pix] = 0;
+  v.cell_fill[pix] = 0;
+  if (pix == 0) {
+    v.cell_start[v.npix] = 0;
+    *v.hit_count = 0;
+    *v.photon_next = 0;
+  }
+}
+
 // Pixel update and film (sppm.cpp:272-320), in the reference's operation
 // order without contraction.
 __global__ void __launch_bounds__(256) k_sppm_update(SppmView v) {
@@ -685,6 +712,7 @@ __global__ void __launch_bounds__(256) k_sppm_update(SppmView v) {
   f[1] = __fadd_rn(f[1], __fadd_rn(__fdiv_rn(ld4.y, fi), __fdiv_rn(tau4.y, den)));
   f[2] = __fadd_rn(f[2], __fadd_rn(__fdiv_rn(ld4.z, fi), __fdiv_rn(tau4.z, den)));
   v.film_count[pix] += 1u;
+  clear_cells(v, pix);  // for the next iteration's photons
 }
 
 // Also the materials as photons see them (TransportMode::Photon).
@@ -703,6 +731,7 @@ __global__ void k_sppm_init(SppmView v, float radius0, const DevMaterial* mats, 
     v.m[pix] = 0;
     v.film[3 * (size_t)pix] = v.film[3 * (size_t)pix + 1] = v.film[3 * (size_t)pix + 2] = 0.f;
     v.film_count[pix] = 0u;
+    clear_cells(v, pix);
   }
 }
 
@@ -714,28 +743,38 @@ void launch_sppm_init(const SppmView& v, float radius0, const DevMaterial* mats,
   k_sppm_init<<<std::min(blocks_for(v.npix, 256), 4096), 256, 0, stream>>>(v, radius0, mats, num_mats);
 }
 
+// Threads per block for n paths: as few (whole warps) as spread them over all
+// SMs four times, at most `most`. Full launches want large blocks (few places
+// in the code at a time), small ones many: 512x512 pixels 4.8 ms at 256 threads
+// against 5.6 at 64, 128x128 pixels 3.5 against 3.1.
+static int sppm_block(int64_t n, int num_sms, int most) {
+  const int64_t per_sm = (n + 4LL * num_sms - 1) / (4LL * num_sms);
+  return (int)std::min<int64_t>(most, (per_sm + 31) / 32 * 32);
+}
+
 void launch_sppm_visible_points(const SceneView& s, const SppmView& v, int iter, cudaStream_t stream) {
-  const size_t smem = trace_smem_bytes(kSppmStack, kSppmBlock);
-  k_sppm_camera<<<blocks_for(v.npix, kSppmBlock), kSppmBlock, smem, stream>>>(s, v, iter);
-  k_sppm_bounds<<<kSppmBoundsBlocks, 256, 0, stream>>>(v);
-  k_sppm_grid<<<1, 256, 0, stream>>>(v, kSppmBoundsBlocks);
+  const int block = sppm_block(v.npix, v.num_sms, kSppmBlock);
+  k_sppm_camera<<<blocks_for(v.npix, block), block, trace_smem_bytes(kSppmStack, block), stream>>>(s, v, iter);
+  const int parts = std::min(blocks_for(v.npix, 256), kSppmBoundsBlocks);
+  k_sppm_bounds<<<parts, 256, 0, stream>>>(v);
+  k_sppm_grid<<<1, 256, 0, stream>>>(v, parts);
 }
 
 void launch_sppm_scan(const SppmView& v, cudaStream_t stream) {
   const int n = v.npix + 1;
   const int nb = blocks_for(n, kScanBlock);
   k_scan_blocks<<<nb, kScanBlock, 0, stream>>>(v.cell_start, n, v.scan_part);
-  k_scan_parts<<<1, kScanBlock, 0, stream>>>(v.scan_part, nb);
-  k_scan_add<<<nb, kScanBlock, 0, stream>>>(v.cell_start, n, v.scan_part);
+  const bool raw = nb <= kScanRaw;
+  if (!raw) k_scan_parts<<<1, kScanBlock, 0, stream>>>(v.scan_part, nb);
+  if (nb > 1) k_scan_add<<<nb, kScanBlock, 0, stream>>>(v.cell_start, n, v.scan_part, raw ? 1 : 0);
 }
 
 void launch_sppm_photons(const SceneView& s, const SppmView& v, int iter, cudaStream_t stream) {
-  cudaMemsetAsync(v.cell_start, 0, sizeof(int) * ((size_t)v.npix + 1), stream);
-  cudaMemsetAsync(v.cell_fill, 0, sizeof(int) * (size_t)v.npix, stream);
-  cudaMemsetAsync(v.hit_count, 0, 2 * sizeof(int), stream);  // and photon_next
-  const size_t smem = trace_smem_bytes(kSppmStack, kPhotonBlock);
-  if (v.photons > 0)
-    k_sppm_photons<<<std::min(blocks_for(v.photons, kPhotonBlock), 2 * v.num_sms), kPhotonBlock, smem, stream>>>(s, v, iter);
+  if (v.photons > 0) {
+    const int block = sppm_block(v.photons, v.num_sms, kPhotonBlock);
+    const int grid = std::min(blocks_for(v.photons, block), 1024 / block * v.num_sms);
+    k_sppm_photons<<<grid, block, trace_smem_bytes(kSppmStack, block), stream>>>(s, v, iter);
+  }
   launch_sppm_scan(v, stream);
   k_sppm_fill<<<std::min(blocks_for(v.hits_cap, 256), 8192), 256, 0, stream>>>(v);
   k_sppm_gather<<<blocks_for(v.npix, kGatherWarps), 32 * kGatherWarps, 0, stream>>>(s, v);
