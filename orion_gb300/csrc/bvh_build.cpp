@@ -10,16 +10,19 @@
 //     the rest of each subtree follows depth-first for locality;
 //   * Woop unit-triangle records (3 x float4 = 48 bytes) in leaf order, and
 //     the leaf-order -> primID map.
-// Subtrees below the top levels are built on worker threads.
+// Subtrees are built on worker threads.
 #include "bvh_build.h"
+
+#include "host_parallel.h"
 
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <condition_variable>
 #include <cstring>
 #include <deque>
-#include <future>
 #include <limits>
+#include <memory>
 #include <mutex>
 #include <thread>
 
@@ -78,106 +81,158 @@ struct TmpNode {
   int depth = 0;
 };
 
+// Four floats worked on together (the compiler's vector type, SSE or NEON).
+// vmin / vmax pick lane by lane exactly what std::min / std::max (box, x) do.
+typedef float V4 __attribute__((vector_size(16)));
+typedef int32_t I4 __attribute__((vector_size(16)));
+
+inline V4 vmin(V4 box, V4 x) { return x < box ? x : box; }
+inline V4 vmax(V4 box, V4 x) { return box < x ? x : box; }
+inline V4 splat(float f) { return V4{f, f, f, f}; }
+
 // One triangle's box and id, 32 bytes. The build partitions these records
 // themselves (not indices into per-triangle arrays), so every scan of a
-// range reads memory in order.
+// range reads memory in order. The id sits in the fourth lanes as two exact
+// small floats, so that no lane ever holds a denormal or a NaN of its own.
 struct PrimRef {
-  float lo[3];
-  int32_t id;
-  float hi[3];
-  float pad;
+  V4 lo, hi;
+  void set_id(int32_t id) {
+    lo[3] = (float)(id & 0x7fffff);
+    hi[3] = (float)(id >> 23);
+  }
+  int32_t id() const { return (int32_t)lo[3] | ((int32_t)hi[3] << 23); }
+  V4 centroids() const { return splat(0.5f) * (lo + hi); }
   float centroid(int k) const { return 0.5f * (lo[k] + hi[k]); }
 };
 
+// Boxes of a range of triangles and of their centroids.
+struct RangeBox {
+  V4 lo = splat(std::numeric_limits<float>::infinity()), hi = -lo;
+  V4 clo = lo, chi = hi;
+  void add(const PrimRef& r) {
+    lo = vmin(lo, r.lo);
+    hi = vmax(hi, r.hi);
+    const V4 c = r.centroids();
+    clo = vmin(clo, c);
+    chi = vmax(chi, c);
+  }
+  void add(const RangeBox& o) {
+    lo = vmin(lo, o.lo);
+    hi = vmax(hi, o.hi);
+    clo = vmin(clo, o.clo);
+    chi = vmax(chi, o.chi);
+  }
+};
+
+// Nodes of one thread, in pieces (a node never moves).
+struct Arena {
+  static constexpr int kPiece = 1024;
+  std::vector<std::unique_ptr<TmpNode[]>> pieces;
+  int used = kPiece;
+  TmpNode* alloc() {
+    if (used == kPiece) {
+      pieces.emplace_back(new TmpNode[kPiece]);
+      used = 0;
+    }
+    return &pieces.back()[used++];
+  }
+};
+
+// A fixed set of threads (the caller's among them) takes subtrees from one
+// queue, largest first; whoever splits a large one leaves its right child there
+// and goes on with the left. Nobody waits for a subtree: the build is done when
+// none is queued or being built.
 struct Builder {
   const BvhBuildOptions& opt;
   PrimRef* refs;
-  std::mutex arena_mu;
-  std::vector<std::unique_ptr<std::deque<TmpNode>>> arenas;
+  int threads;
+  std::vector<Arena> arenas;  // one per thread
   std::atomic<int> max_depth{0};
   std::atomic<int> leaves{0};
-  int spawn_depth;
-  int threads;
-  std::atomic<int> running{0};  // subtrees building on threads of their own
+  struct Task {
+    int begin, end, depth;
+    TmpNode** slot;
+  };
+  std::mutex mu;
+  std::condition_variable wake;
+  std::deque<Task> queue;
+  int unfinished = 0;  // tasks queued or being built
 
-  Builder(const BvhBuildOptions& o, PrimRef* r, int nthreads) : opt(o), refs(r), threads(nthreads) {
-    spawn_depth = 0;
-    while ((1 << spawn_depth) < 4 * threads) ++spawn_depth;
+  Builder(const BvhBuildOptions& o, PrimRef* r, int nthreads) : opt(o), refs(r), threads(nthreads) {}
+
+  TmpNode* run(int count) {
+    // As many threads as the triangles can keep busy.
+    const int n = std::max(1, std::min(threads, count / kSpawn));
+    arenas.resize(n);
+    TmpNode* root = nullptr;
+    queue.push_back(Task{0, count, 0, &root});
+    unfinished = 1;
+    std::vector<std::thread> th;
+    for (int t = 1; t < n; ++t) th.emplace_back([this, t] { work(arenas[t]); });
+    work(arenas[0]);
+    for (std::thread& x : th) x.join();
+    return root;
   }
 
-  std::deque<TmpNode>* new_arena() {
-    std::lock_guard<std::mutex> g(arena_mu);
-    arenas.emplace_back(new std::deque<TmpNode>());
-    return arenas.back().get();
+  void work(Arena& arena) {
+    std::unique_lock<std::mutex> g(mu);
+    while (true) {
+      wake.wait(g, [this] { return !queue.empty() || unfinished == 0; });
+      if (queue.empty()) return;
+      const Task t = queue.front();
+      queue.pop_front();
+      g.unlock();
+      *t.slot = build(t.begin, t.end, t.depth, arena);
+      g.lock();
+      if (--unfinished == 0) wake.notify_all();
+    }
   }
 
   static float half_area(const float* a, const float* b) {
     float dx = b[0] - a[0], dy = b[1] - a[1], dz = b[2] - a[2];
     return dx * dy + dy * dz + dz * dx;
   }
+  static float half_area(V4 a, V4 b) {
+    const V4 d = b - a;
+    return d[0] * d[1] + d[1] * d[2] + d[2] * d[0];
+  }
 
   // Ranges above this many primitives are scanned by several threads (the
   // top levels of the tree, which would otherwise run on one thread).
   static constexpr int kParallelScan = 1 << 16;
 
-  // Runs f(b, e, part) over `parts` contiguous pieces of [begin, end) in parallel.
-  template <class F>
-  static void parallel_parts(int begin, int end, int parts, F f) {
-    std::vector<std::thread> th;
-    const int64_t n = end - begin;
-    for (int t = 0; t < parts; ++t) {
-      const int b = begin + (int)(n * t / parts), e = begin + (int)(n * (t + 1) / parts);
-      th.emplace_back(f, b, e, t);
-    }
-    for (auto& x : th) x.join();
-  }
+  // Subtrees of more primitives than this go to the queue (one takes about 0.1
+  // ms to build).
+  static constexpr int kSpawn = 512;
 
   int scan_parts(int count) const {
     if (count < kParallelScan) return 1;
     return std::max(1, std::min(threads, count / (kParallelScan / 4)));
   }
 
-  // Box of the primitives (centroids: the box of their centres) over [begin, end).
-  void bounds_range(bool centroids, int begin, int end, float* bl, float* bh) const {
-    for (int k = 0; k < 3; ++k) {
-      bl[k] = std::numeric_limits<float>::infinity();
-      bh[k] = -std::numeric_limits<float>::infinity();
-    }
-    for (int i = begin; i < end; ++i) {
-      const PrimRef& r = refs[i];
-      for (int k = 0; k < 3; ++k) {
-        const float a = centroids ? r.centroid(k) : r.lo[k], b = centroids ? a : r.hi[k];
-        bl[k] = std::min(bl[k], a);
-        bh[k] = std::max(bh[k], b);
-      }
-    }
-  }
-
-  // bounds_range, in parallel for large ranges.
-  void box_of(bool centroids, int begin, int end, float* bl, float* bh) const {
+  // Boxes over [begin, end), in parallel for large ranges.
+  RangeBox boxes(int begin, int end) const {
     const int parts = scan_parts(end - begin);
-    if (parts == 1) return bounds_range(centroids, begin, end, bl, bh);
-    std::vector<float> r(6 * (size_t)parts);
-    parallel_parts(begin, end, parts,
-                   [&](int s, int e, int t) { bounds_range(centroids, s, e, &r[6 * t], &r[6 * t + 3]); });
-    for (int k = 0; k < 3; ++k) {
-      bl[k] = std::numeric_limits<float>::infinity();
-      bh[k] = -std::numeric_limits<float>::infinity();
+    RangeBox all;
+    if (parts == 1) {
+      for (int i = begin; i < end; ++i) all.add(refs[i]);
+      return all;
     }
-    for (int t = 0; t < parts; ++t)
-      for (int k = 0; k < 3; ++k) {
-        bl[k] = std::min(bl[k], r[6 * t + k]);
-        bh[k] = std::max(bh[k], r[6 * t + 3 + k]);
-      }
+    std::vector<RangeBox> part(parts);
+    parallel_parts(begin, end, parts, [&](int s, int e, int t) {
+      RangeBox b;
+      for (int i = s; i < e; ++i) b.add(refs[i]);
+      part[t] = b;
+    });
+    for (const RangeBox& b : part) all.add(b);
+    return all;
   }
 
-  void bounds(int begin, int end, float* bl, float* bh) const { box_of(false, begin, end, bl, bh); }
-
-  TmpNode* build(int begin, int end, int depth, std::deque<TmpNode>* arena) {
-    arena->emplace_back();
-    TmpNode* n = &arena->back();
+  TmpNode* build(int begin, int end, int depth, Arena& arena) {
+    TmpNode* n = arena.alloc();
     n->depth = depth;
-    bounds(begin, end, n->lo, n->hi);
+    const RangeBox box = boxes(begin, end);
+    for (int k = 0; k < 3; ++k) n->lo[k] = box.lo[k], n->hi[k] = box.hi[k];
     int count = end - begin;
     n->first = begin;
     n->total = count;
@@ -193,30 +248,21 @@ struct Builder {
     if (!forced_median) {
       float cost_leaf = (float)count;
       float split_cost;
-      mid = sah_split(begin, end, n, &split_cost);
+      mid = sah_split(begin, end, box, &split_cost);
       if (mid < 0 || (count <= opt.max_leaf && cost_leaf <= split_cost)) {
         if (count <= opt.max_leaf) return make_leaf(n, begin, count);
         mid = -1;
       }
     }
-    if (mid < 0) mid = median_split(begin, end);
-    // A subtree goes to a new thread while fewer than 2 x threads are busy, so
-    // uneven SAH splits still keep every core working.
-    bool spawn = false;
-    if (count > 8192) {
-      int live = running.load();
-      while (live < 2 * threads && !(spawn = running.compare_exchange_weak(live, live + 1))) {
+    if (mid < 0) mid = median_split(begin, end, box);
+    if (end - mid > kSpawn && arenas.size() > 1) {
+      {
+        std::lock_guard<std::mutex> g(mu);
+        queue.push_back(Task{mid, end, depth + 1, &n->child[1]});
+        ++unfinished;
       }
-    }
-    if (spawn) {
-      auto fut = std::async(std::launch::async, [=] {
-        std::deque<TmpNode>* a2 = new_arena();
-        TmpNode* r = build(begin, mid, depth + 1, a2);
-        running.fetch_sub(1);
-        return r;
-      });
-      n->child[1] = build(mid, end, depth + 1, arena);
-      n->child[0] = fut.get();
+      wake.notify_one();
+      n->child[0] = build(begin, mid, depth + 1, arena);
     } else {
       n->child[0] = build(begin, mid, depth + 1, arena);
       n->child[1] = build(mid, end, depth + 1, arena);
@@ -231,64 +277,70 @@ struct Builder {
     return n;
   }
 
-  int median_split(int begin, int end) {
-    float cl[3], ch[3];
-    centroid_bounds(begin, end, cl, ch);
+  int median_split(int begin, int end, const RangeBox& box) {
     int axis = 0;
     for (int k = 1; k < 3; ++k)
-      if (ch[k] - cl[k] > ch[axis] - cl[axis]) axis = k;
+      if (box.chi[k] - box.clo[k] > box.chi[axis] - box.clo[axis]) axis = k;
     int mid = begin + (end - begin) / 2;
     std::nth_element(refs + begin, refs + mid, refs + end,
                      [&](const PrimRef& a, const PrimRef& b) { return a.centroid(axis) < b.centroid(axis); });
     return mid;
   }
 
-  void centroid_bounds(int begin, int end, float* cl, float* ch) const { box_of(true, begin, end, cl, ch); }
-
   struct Bins {
     int cnt[3][64];
-    float blo[3][64][3], bhi[3][64][3];
+    V4 blo[3][64], bhi[3][64];
     void clear(int B) {
+      const V4 inf = splat(std::numeric_limits<float>::infinity());
       for (int axis = 0; axis < 3; ++axis)
         for (int b = 0; b < B; ++b) {
           cnt[axis][b] = 0;
-          for (int k = 0; k < 3; ++k) {
-            blo[axis][b][k] = std::numeric_limits<float>::infinity();
-            bhi[axis][b][k] = -std::numeric_limits<float>::infinity();
-          }
+          blo[axis][b] = inf;
+          bhi[axis][b] = -inf;
         }
     }
   };
 
-  void bin_range(int begin, int end, int B, const float* cl, const float* scale, Bins& bins) const {
+  void bin_range(int begin, int end, int B, V4 cl, V4 scale, Bins& bins) const {
     bins.clear(B);
     for (int i = begin; i < end; ++i) {
       const PrimRef& r = refs[i];
+      const I4 at = __builtin_convertvector((r.centroids() - cl) * scale, I4);
       for (int axis = 0; axis < 3; ++axis) {
         if (scale[axis] == 0.f) continue;
-        int b = std::min(B - 1, (int)((r.centroid(axis) - cl[axis]) * scale[axis]));
+        const int b = std::min(B - 1, (int)at[axis]);
         bins.cnt[axis][b]++;
-        for (int k = 0; k < 3; ++k) {
-          bins.blo[axis][b][k] = std::min(bins.blo[axis][b][k], r.lo[k]);
-          bins.bhi[axis][b][k] = std::max(bins.bhi[axis][b][k], r.hi[k]);
-        }
+        bins.blo[axis][b] = vmin(bins.blo[axis][b], r.lo);
+        bins.bhi[axis][b] = vmax(bins.bhi[axis][b], r.hi);
       }
     }
   }
 
   // Returns the partition point of the best binned SAH split, or -1.
-  int sah_split(int begin, int end, const TmpNode* n, float* best_cost_out) {
+  int sah_split(int begin, int end, const RangeBox& box, float* best_cost_out) {
+    const float parent_area = half_area(box.lo, box.hi);
+    if (end - begin == 2) {
+      // Two primitives part on every axis along which their centres differ,
+      // always the same way: the first such axis is the one binning finds.
+      for (int axis = 0; axis < 3; ++axis) {
+        if (!(box.chi[axis] - box.clo[axis] > 0.f)) continue;
+        PrimRef *a = refs + begin, *b = a + 1;
+        if (!(a->centroid(axis) < b->centroid(axis))) std::swap(*a, *b);
+        const float cost = half_area(a->lo, a->hi) + half_area(b->lo, b->hi);
+        *best_cost_out = parent_area > 0.f ? 1.f + cost / parent_area : 1.f;
+        return cost < std::numeric_limits<float>::infinity() ? begin + 1 : -1;
+      }
+      return -1;
+    }
     // Small ranges get as many bins as primitives (at least 4): the per-bin
     // clear and sweep would otherwise dominate near the leaves.
     const int B = std::max(2, std::min(std::min(opt.bins, 64), std::max(4, end - begin)));
-    float cl[3], ch[3];
-    centroid_bounds(begin, end, cl, ch);
-    float parent_area = half_area(n->lo, n->hi);
     int best_axis = -1, best_bin = -1;
     float best_cost = std::numeric_limits<float>::infinity();
-    float scale[3];
+    V4 cl = box.clo, scale = splat(0.f);
+    cl[3] = 0.f;
     for (int axis = 0; axis < 3; ++axis) {
-      float ext = ch[axis] - cl[axis];
+      float ext = box.chi[axis] - box.clo[axis];
       scale[axis] = ext > 0.f ? B / ext : 0.f;
     }
     Bins all;
@@ -303,46 +355,37 @@ struct Builder {
         for (int axis = 0; axis < 3; ++axis)
           for (int b = 0; b < B; ++b) {
             all.cnt[axis][b] += pb.cnt[axis][b];
-            for (int k = 0; k < 3; ++k) {
-              all.blo[axis][b][k] = std::min(all.blo[axis][b][k], pb.blo[axis][b][k]);
-              all.bhi[axis][b][k] = std::max(all.bhi[axis][b][k], pb.bhi[axis][b][k]);
-            }
+            all.blo[axis][b] = vmin(all.blo[axis][b], pb.blo[axis][b]);
+            all.bhi[axis][b] = vmax(all.bhi[axis][b], pb.bhi[axis][b]);
           }
     }
-    auto& cnt = all.cnt;
-    auto& blo = all.blo;
-    auto& bhi = all.bhi;
+    const V4 inf = splat(std::numeric_limits<float>::infinity());
     for (int axis = 0; axis < 3; ++axis) {
       if (scale[axis] == 0.f) continue;
+      const int* cnt = all.cnt[axis];
       float rarea[64];
       int rcnt[64];
-      float al[3], ah[3];
-      for (int k = 0; k < 3; ++k) {
-        al[k] = std::numeric_limits<float>::infinity();
-        ah[k] = -std::numeric_limits<float>::infinity();
-      }
+      V4 al = inf, ah = -inf;
       int ac = 0;
-      for (int b = B - 1; b > 0; --b) {
-        ac += cnt[axis][b];
-        for (int k = 0; k < 3; ++k) {
-          al[k] = std::min(al[k], blo[axis][b][k]);
-          ah[k] = std::max(ah[k], bhi[axis][b][k]);
+      for (int b = B - 1; b > 0; --b) {  // an empty bin leaves the sums as they are
+        if (cnt[b]) {
+          ac += cnt[b];
+          al = vmin(al, all.blo[axis][b]);
+          ah = vmax(ah, all.bhi[axis][b]);
+          rarea[b] = half_area(al, ah);
+        } else {
+          rarea[b] = ac ? rarea[b + 1] : 0.f;
         }
         rcnt[b] = ac;
-        rarea[b] = ac ? half_area(al, ah) : 0.f;
       }
-      for (int k = 0; k < 3; ++k) {
-        al[k] = std::numeric_limits<float>::infinity();
-        ah[k] = -std::numeric_limits<float>::infinity();
-      }
+      al = inf, ah = -inf;
       ac = 0;
       for (int b = 0; b < B - 1; ++b) {
-        ac += cnt[axis][b];
-        for (int k = 0; k < 3; ++k) {
-          al[k] = std::min(al[k], blo[axis][b][k]);
-          ah[k] = std::max(ah[k], bhi[axis][b][k]);
-        }
-        if (ac == 0 || rcnt[b + 1] == 0) continue;
+        if (cnt[b] == 0) continue;  // the split before it again, or no primitive yet
+        ac += cnt[b];
+        al = vmin(al, all.blo[axis][b]);
+        ah = vmax(ah, all.bhi[axis][b]);
+        if (rcnt[b + 1] == 0) break;
         float cost = half_area(al, ah) * ac + rarea[b + 1] * rcnt[b + 1];
         if (cost < best_cost) {
           best_cost = cost;
@@ -664,7 +707,7 @@ struct WideCollapser {
         for (int r = 0; r < nk; ++r) fill(tk.root.child_base + r, kids[r], tk.nodes, tk.tris);
       }
     };
-    if (!tasks.empty()) Builder::parallel_parts(0, threads, std::max(1, std::min(threads, (int)tasks.size())), worker);
+    if (!tasks.empty()) parallel_parts(0, threads, std::max(1, std::min(threads, (int)tasks.size())), worker);
     for (Task& tk : tasks) {
       const int node_off = (int)out.size(), tri_off = (int)tris.size();
       for (WideNode& w : tk.nodes) {
@@ -710,7 +753,7 @@ void build_bvh(const float* positions, int64_t num_tris, const BvhBuildOptions& 
   }
   int threads = opt.threads > 0 ? opt.threads : (int)std::max(1u, std::thread::hardware_concurrency());
   std::vector<PrimRef> refs(T);
-  Builder::parallel_parts(0, T, std::max(1, std::min(threads, T / 4096)), [&](int s, int e, int) {
+  parallel_parts(0, T, std::max(1, std::min(threads, T / 4096)), [&](int s, int e, int) {
     for (int i = s; i < e; ++i) {
       const float* p = positions + 9 * (size_t)i;
       PrimRef& r = refs[i];
@@ -718,20 +761,18 @@ void build_bvh(const float* positions, int64_t num_tris, const BvhBuildOptions& 
         r.lo[k] = std::min(std::min(p[k], p[3 + k]), p[6 + k]);
         r.hi[k] = std::max(std::max(p[k], p[3 + k]), p[6 + k]);
       }
-      r.id = i;
-      r.pad = 0.f;
+      r.set_id(i);
     }
   });
   Builder b(opt, refs.data(), threads);
-  std::deque<TmpNode>* arena = b.new_arena();
-  TmpNode* root = b.build(0, T, 0, arena);
+  TmpNode* root = b.run(T);
   out->depth = b.max_depth.load();
   out->leaves = b.leaves.load();
   std::vector<int32_t> order(T);  // binary leaf order -> primID
-  for (int i = 0; i < T; ++i) order[i] = refs[i].id;
+  for (int i = 0; i < T; ++i) order[i] = refs[i].id();
   // Woop records of triangles in `ids` order, in parallel.
   auto records = [&](const std::vector<int32_t>& ids) {
-    Builder::parallel_parts(0, T, std::max(1, std::min(threads, T / 4096)), [&](int s, int e, int) {
+    parallel_parts(0, T, std::max(1, std::min(threads, T / 4096)), [&](int s, int e, int) {
       for (int i = s; i < e; ++i) {
         out->tri_prim[i] = ids[i];
         woop_record(positions + 9 * (size_t)ids[i], &out->woop[12 * (size_t)i]);

@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "context.h"
+#include "host_parallel.h"
 
 using namespace orion_gb300;
 
@@ -342,10 +343,16 @@ extern "C" int orion_gpu_scene_upload(orion_gpu_ctx* ctx, const orion_host_scene
       if (b->depth >= kMaxBvhDepth) return fail(ORION_ERR_UNSUPPORTED, "BVH deeper than the traversal stack bound");
       hsm->tri_class.resize(b->tri_prim.size());
       hsm->class_mask = 1u << SC_MISS;
-      for (size_t i = 0; i < hsm->tri_class.size(); ++i) {
-        hsm->tri_class[i] = (uint8_t)hsm->prep->mats[hsm->prep->prims[b->tri_prim[i]].material].shade_class;
-        hsm->class_mask |= 1u << hsm->tri_class[i];
-      }
+      const int64_t nt = (int64_t)hsm->tri_class.size();
+      const int parts = parts_for(nt, 16384);
+      std::vector<unsigned> masks(parts, 0u);
+      parallel_parts(0, nt, parts, [&](int64_t begin, int64_t end, int t) {
+        for (int64_t i = begin; i < end; ++i) {
+          hsm->tri_class[i] = (uint8_t)hsm->prep->mats[hs.material_of_prim[b->tri_prim[i]]].shade_class;
+          masks[t] |= 1u << hsm->tri_class[i];
+        }
+      });
+      for (unsigned m : masks) hsm->class_mask |= m;
       hsm->bvh = std::move(b);
       pin(hsm, hsm->bvh->wide);
       pin(hsm, hsm->bvh->woop);

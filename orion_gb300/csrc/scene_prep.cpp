@@ -6,6 +6,8 @@
 // computes per hit or at preprocess time.
 #include "scene_prep.h"
 
+#include "host_parallel.h"
+
 #include "material_build.h"
 
 #include <cmath>
@@ -155,23 +157,40 @@ void prepare_envmap(const HostImage& im, const float L[3], PreparedScene* out, f
 
 bool prepare_scene(const HostScene& s, PreparedScene* out, std::string* err) {
   const int64_t T = s.num_prims();
-  out->prims.resize(T);
-  float lo[3] = {std::numeric_limits<float>::max(), std::numeric_limits<float>::max(),
-                 std::numeric_limits<float>::max()};
-  float hi[3] = {std::numeric_limits<float>::lowest(), std::numeric_limits<float>::lowest(),
-                 std::numeric_limits<float>::lowest()};
-  for (int64_t i = 0; i < T; ++i) {
-    PrimShade& p = out->prims[i];
-    std::memset(&p, 0, sizeof(p));
-    std::memcpy(p.p, &s.positions[9 * i], 9 * sizeof(float));
-    std::memcpy(p.n, &s.normals[9 * i], 9 * sizeof(float));
-    p.material = s.material_of_prim[i];
-    p.light = s.light_of_prim[i];
-    for (int c = 0; c < 3; ++c)
-      for (int k = 0; k < 3; ++k) {
-        lo[k] = std::min(lo[k], p.p[3 * c + k]);
-        hi[k] = std::max(hi[k], p.p[3 * c + k]);
-      }
+  out->prims.assign((size_t)T, PrimShade{});
+  struct Box {
+    float lo[3], hi[3];
+  };
+  const int parts = parts_for(T, 8192);
+  std::vector<Box> part(parts);
+  parallel_parts(0, T, parts, [&](int64_t begin, int64_t end, int t) {
+    Box b;
+    for (int k = 0; k < 3; ++k) {
+      b.lo[k] = std::numeric_limits<float>::max();
+      b.hi[k] = std::numeric_limits<float>::lowest();
+    }
+    for (int64_t i = begin; i < end; ++i) {
+      PrimShade& p = out->prims[i];
+      std::memcpy(p.p, &s.positions[9 * i], 9 * sizeof(float));
+      std::memcpy(p.n, &s.normals[9 * i], 9 * sizeof(float));
+      p.material = s.material_of_prim[i];
+      p.light = s.light_of_prim[i];
+      for (int c = 0; c < 3; ++c)
+        for (int k = 0; k < 3; ++k) {
+          b.lo[k] = std::min(b.lo[k], p.p[3 * c + k]);
+          b.hi[k] = std::max(b.hi[k], p.p[3 * c + k]);
+        }
+    }
+    part[t] = b;
+  });
+  float lo[3], hi[3];
+  for (int k = 0; k < 3; ++k) {
+    lo[k] = part[0].lo[k];
+    hi[k] = part[0].hi[k];
+    for (const Box& b : part) {
+      lo[k] = std::min(lo[k], b.lo[k]);
+      hi[k] = std::max(hi[k], b.hi[k]);
+    }
   }
   // Bounds3::boundingSphere (src/core/geometry.h:551-554).
   for (int k = 0; k < 3; ++k) out->world_center[k] = (lo[k] + hi[k]) * 0.5f;
