@@ -121,15 +121,18 @@ __global__ void __launch_bounds__(512, 2) k_b_trace(const __grid_constant__ BTra
 // appended to. As in plain renders the classes' launches overlap (k_shade). One
 // kernel serves both modes so that a path's arithmetic is compiled once.
 template <int SC>
-__global__ void __launch_bounds__(128, 5) k_b_shade(WaveView w, BatchView b, const uint32_t* sobol, int parity,
-                                                    int marks) {
+__global__ void __launch_bounds__(shade_threads(SC), kShadeThreadsPerSm / shade_threads(SC))
+    k_b_shade(WaveView w, BatchView b, const uint32_t* sobol, int parity, int marks) {
   asm volatile("griddepcontrol.launch_dependents;");
   BatchCtl& c = *b.ctl;
   const bool waves = parity != kCurrent;
   const int cur = waves ? parity : c.cur;
   const int n = c.counters[cnt_cls(SC, cur)];
   const int* in_q = w.q_cls + (size_t)SC * w.capacity;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+  for (int q0 = blockIdx.x * blockDim.x; q0 < n; q0 += gridDim.x * blockDim.x) {
+    const int q = q0 + threadIdx.x;
+    __syncthreads();  // the block's warps go through the code together
+    if (q >= n) continue;
     const int pid = in_q[q];
     const int4 meta = w.rec[pid].meta;
     const DevJob& J = b.jobs[meta.y];
@@ -440,15 +443,16 @@ void enqueue_iteration(const WaveView& w, const BatchView& b, const uint32_t* so
   begin(ST_SHADE);
   for (int sc = 0; sc < kShadeClasses; ++sc) {
     if (!((class_mask >> sc) & 1u)) continue;
+    const ShadeShape shape = shade_shape(sc, cap, cfg);
     switch (sc) {
-      case SC_DIFFUSE: k_b_shade<SC_DIFFUSE><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
-      case SC_CONDUCTOR: k_b_shade<SC_CONDUCTOR><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
-      case SC_SPECULAR: k_b_shade<SC_SPECULAR><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
-      case SC_DIELECTRIC: k_b_shade<SC_DIELECTRIC><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
-      case SC_PLASTIC: k_b_shade<SC_PLASTIC><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
-      case SC_GENERAL: k_b_shade<SC_GENERAL><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
-      case SC_TEXTURED: k_b_shade<SC_TEXTURED><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
-      case SC_MISS: k_b_shade<SC_MISS><<<sgrid, cfg.shade_block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
+      case SC_DIFFUSE: k_b_shade<SC_DIFFUSE><<<shape.grid, shape.block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
+      case SC_CONDUCTOR: k_b_shade<SC_CONDUCTOR><<<shape.grid, shape.block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
+      case SC_SPECULAR: k_b_shade<SC_SPECULAR><<<shape.grid, shape.block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
+      case SC_DIELECTRIC: k_b_shade<SC_DIELECTRIC><<<shape.grid, shape.block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
+      case SC_PLASTIC: k_b_shade<SC_PLASTIC><<<shape.grid, shape.block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
+      case SC_GENERAL: k_b_shade<SC_GENERAL><<<shape.grid, shape.block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
+      case SC_TEXTURED: k_b_shade<SC_TEXTURED><<<shape.grid, shape.block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
+      case SC_MISS: k_b_shade<SC_MISS><<<shape.grid, shape.block, 0, stream>>>(w, b, sobol, kCurrent, 0); break;
     }
   }
   end();
@@ -471,7 +475,7 @@ void enqueue_iteration(const WaveView& w, const BatchView& b, const uint32_t* so
 
 // Shading of one bounce of a batch wave, as launch_shading (kernels.cu).
 int launch_wb_shading(const WaveView& bw, const BatchView& b, const uint32_t* sobol, unsigned class_mask, int cur,
-                      int append, int grid, int block, cudaStream_t stream) {
+                      int append, int n_paths, const LaunchConfig& cfg, cudaStream_t stream) {
   using Kernel = void (*)(WaveView, BatchView, const uint32_t*, int, int);
   static const struct {
     int sc;
@@ -484,13 +488,14 @@ int launch_wb_shading(const WaveView& bw, const BatchView& b, const uint32_t* so
   early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   early.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t c = {};
-  c.gridDim = dim3(grid);
-  c.blockDim = dim3(block);
   c.stream = stream;
   c.attrs = &early;
   int n = 0;
   for (const auto& k : kOrder) {
     if (!((class_mask >> k.sc) & 1u)) continue;
+    const ShadeShape shape = shade_shape(k.sc, n_paths, cfg);
+    c.blockDim = dim3(shape.block);
+    c.gridDim = dim3(shape.grid);
     c.numAttrs = n > 0 ? 1 : 0;
     cudaLaunchKernelEx(&c, k.kernel, bw, b, sobol, cur, append ? 0 : 1);
     ++n;
@@ -566,7 +571,7 @@ void launch_batch_wave(const WaveView& w, const BatchView& b, const uint32_t* so
         return 1;
       });
     timed(ST_SHADE, [&] {
-      return launch_wb_shading(bw, b, sobol, class_mask, cur, append, sgrid, cfg.shade_block, stream);
+      return launch_wb_shading(bw, b, sobol, class_mask, cur, append, n, cfg, stream);
     });
     if (!append && !(complete && bounce + 1 == bounces))  // no path goes on after the last bounce
       timed(ST_OTHER, [&] {

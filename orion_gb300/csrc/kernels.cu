@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(512, 2) k_trace(const __grid_constant__ TraceA
 
 // One bounce for every path whose extension ray hit a material of shading
 // class SC (or, for SC_MISS, left the scene), with that class's BSDF code only.
-// Launch bounds: at most 96 registers (5 blocks of 128 threads per SM).
+// Launch bounds: at most 96 registers (640 threads per SM).
 // The queues a path goes to next (light-sample resolution, shadow ray, MIS
 // rays, next extension ray) are recorded as bits of its qflags byte, and
 // k_compact_queues lists them in slot order: the next trace launches then
@@ -93,12 +93,15 @@ __global__ void __launch_bounds__(512, 2) k_trace(const __grid_constant__ TraceA
 // ones overlap; block 0 ends only when the launch before has, which makes the
 // end of the last one the end of all.
 template <int SC>
-__global__ void __launch_bounds__(128, 5) k_shade(SceneView s, WaveView w, WaveArgs a, int bounce, int cur) {
+__global__ void __launch_bounds__(shade_threads(SC), kShadeThreadsPerSm / shade_threads(SC)) k_shade(SceneView s, WaveView w, WaveArgs a, int bounce, int cur) {
   asm volatile("griddepcontrol.launch_dependents;");
   if (blockIdx.x == 0 && threadIdx.x < kRayKinds) w.counters[CNT_FETCH + threadIdx.x] = 0;  // for the next trace
   const int n = w.counters[cnt_cls(SC, cur)];
   const int* in_q = w.q_cls + (size_t)SC * w.capacity;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+  for (int q0 = blockIdx.x * blockDim.x; q0 < n; q0 += gridDim.x * blockDim.x) {
+    const int q = q0 + threadIdx.x;
+    __syncthreads();  // the block's warps go through the code together
+    if (q >= n) continue;
     const int pid = in_q[q];
     const int4 meta = w.rec[pid].meta;
     const uint64_t index = ((uint64_t)(uint32_t)meta.w << 32) | (uint32_t)meta.y;
@@ -406,8 +409,8 @@ void trace_dispatch(int kinds, const SceneView& s, const WaveView& w, int cur, b
 // 1 spp 0.66 -> 0.55 ms). One kernel for all classes was slower where it
 // matters (zoo 5.35 ms, displaced sphere 60.7 -> 63.1 ms: more spills) and
 // contracted other multiply-adds.
-int launch_shading(const SceneView& s, const WaveView& w, const WaveArgs& a, int bounce, int cur, int grid, int block,
-                   cudaStream_t stream) {
+int launch_shading(const SceneView& s, const WaveView& w, const WaveArgs& a, int bounce, int cur,
+                   const LaunchConfig& cfg, cudaStream_t stream) {
   using Kernel = void (*)(SceneView, WaveView, WaveArgs, int, int);
   static const struct {
     int sc;
@@ -420,13 +423,14 @@ int launch_shading(const SceneView& s, const WaveView& w, const WaveArgs& a, int
   early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   early.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t c = {};
-  c.gridDim = dim3(grid);
-  c.blockDim = dim3(block);
   c.stream = stream;
   c.attrs = &early;
   int n = 0;
   for (const auto& k : kOrder) {
     if (!((a.class_mask >> k.sc) & 1u)) continue;
+    const ShadeShape shape = shade_shape(k.sc, a.n_paths, cfg);
+    c.blockDim = dim3(shape.block);
+    c.gridDim = dim3(shape.grid);
     c.numAttrs = n > 0 ? 1 : 0;
     cudaLaunchKernelEx(&c, k.kernel, s, w, a, bounce, cur);
     ++n;
@@ -456,7 +460,6 @@ void launch_wave(const SceneView& s, const WaveView& w, const WaveArgs& a, const
   // Mpaths/s on the displaced sphere, 2433 -> 2525 on eight spheres, against
   // grids that fill the register file).
   const int tgrid = grid_for(a.n_paths, cfg.trace_block, persistent);
-  const int sgrid = grid_for(a.n_paths, cfg.shade_block, persistent * 2);
   const int compact_grid = grid_for(a.n_paths, kCompactSpan, cfg.num_sms * 8);
   int cur = 0;
   for (int bounce = 0; bounce <= a.max_depth; ++bounce) {
@@ -488,7 +491,7 @@ void launch_wave(const SceneView& s, const WaveView& w, const WaveArgs& a, const
       end();
     }
     begin(ST_SHADE);
-    nl += launch_shading(s, w, a, bounce, cur, sgrid, cfg.shade_block, stream) - 1;  // end() counts one of them
+    nl += launch_shading(s, w, a, bounce, cur, cfg, stream) - 1;  // end() counts one of them
     end();
     if (!a.append && bounce < a.max_depth) {  // after the last bounce no path goes on and no queue is read
       begin(ST_OTHER);

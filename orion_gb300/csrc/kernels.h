@@ -276,6 +276,33 @@ struct LaunchConfig {
   int test_batch_iterations;  // batch loops stop (with an error) after this many iterations
 };
 
+// Threads of a shading block. Shading waits for instructions about as much as
+// for memory, so a block's warps start each path together (a barrier), and the
+// classes with the most code run in large blocks: few places in the code at a
+// time on an SM. The others keep LaunchConfig::shade_block (at most 128), which
+// fits beside another wave's trace blocks. Against 128 threads for all, without
+// the barrier: zoo 985x726 x 20 spp 13.7 -> 11.9 ms, zoo 333x217 x 48 spp 4.0 ->
+// 3.6, textured 640x359 x 32 spp 4.8 -> 4.5; Cornell, displaced and eight spheres
+// unchanged (640 threads: Cornell 1% slower; for all classes: displaced 6%).
+constexpr int kShadeThreadsPerSm = 640;
+constexpr bool large_code(int sc) {
+  return sc == SC_GENERAL || sc == SC_TEXTURED || sc == SC_PLASTIC || sc == SC_DIELECTRIC;
+}
+constexpr int shade_threads(int sc) { return large_code(sc) ? 320 : 128; }
+
+struct ShadeShape {
+  int grid, block;
+};
+// For up to n paths of class sc: about twice the blocks that run at once.
+inline ShadeShape shade_shape(int sc, int64_t n, const LaunchConfig& cfg) {
+  const int block = large_code(sc) ? shade_threads(sc) : cfg.shade_block;
+  const int64_t most = large_code(sc) ? (int64_t)cfg.num_sms * 2 * (kShadeThreadsPerSm / shade_threads(sc))
+                                      : (int64_t)cfg.num_sms * cfg.blocks_per_sm * 2;
+  int64_t g = (n + block - 1) / block;
+  if (g > most) g = most;
+  return ShadeShape{(int)(g < 1 ? 1 : g), block};
+}
+
 enum Stage { ST_CAMERA = 0, ST_TRACE_EXT, ST_SHADE, ST_TRACE_SHADOW, ST_TRACE_MIS, ST_RESOLVE, ST_FILM, ST_OTHER,
              kNumStages };
 
