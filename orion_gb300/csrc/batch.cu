@@ -240,8 +240,6 @@ __global__ void k_wb_camera(WaveView w, BatchView b, const uint32_t* sobol, unsi
     r.L = make_float4(0.f, 0.f, 0.f, __uint_as_float((uint32_t)(unsigned long long)index));
     r.hit = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
     r.meta = make_int4((int)dim, it.job, 0, (int)((unsigned long long)index >> 32));
-    w.q_ext[0][i] = i;
-    w.qflags[i] = 0;
   }
 }
 
@@ -344,9 +342,9 @@ __global__ void k_b_control(BatchView b, cudaGraphConditionalHandle cond, int in
 // marks: extension hits mark their slot's shading class in qflags for a
 // compaction instead of appending to the class queues.
 void b_trace(const LaunchConfig& cfg, const WaveView& bw, const BatchView& b, int kinds, int parity, int grid,
-             bool marks, cudaStream_t s) {
+             bool marks, bool camera_rays, cudaStream_t s) {
   BTraceArgs a;
-  for (int cur = 0; cur < 2; ++cur) wave_ray_sets(bw, cur, marks, a.set[cur]);
+  for (int cur = 0; cur < 2; ++cur) wave_ray_sets(bw, cur, marks, camera_rays, a.set[cur]);
   a.b = b;
   a.job = bw.job;
   a.kinds = kinds;
@@ -438,7 +436,7 @@ void enqueue_iteration(const WaveView& w, const BatchView& b, const uint32_t* so
   k_b_regen<<<grid_cap(cap, 256, persistent * 4), 256, 0, stream>>>(w, b, sobol);
   end();
   begin(ST_TRACE_EXT);
-  b_trace(cfg, bw, b, TK_EXT, kCurrent, tgrid, false, stream);
+  b_trace(cfg, bw, b, TK_EXT, kCurrent, tgrid, false, false, stream);
   end();
   begin(ST_SHADE);
   for (int sc = 0; sc < kShadeClasses; ++sc) {
@@ -457,10 +455,10 @@ void enqueue_iteration(const WaveView& w, const BatchView& b, const uint32_t* so
   }
   end();
   begin(ST_TRACE_SHADOW);
-  b_trace(cfg, bw, b, TK_SHADOW, kNext, tgrid, false, stream);
+  b_trace(cfg, bw, b, TK_SHADOW, kNext, tgrid, false, false, stream);
   end();
   begin(ST_TRACE_MIS);
-  b_trace(cfg, bw, b, TK_MIS | TK_MIS_ENV, kNext, tgrid, false, stream);
+  b_trace(cfg, bw, b, TK_MIS | TK_MIS_ENV, kNext, tgrid, false, false, stream);
   end();
   begin(ST_RESOLVE);
   k_b_resolve<<<sgrid, cfg.shade_block, 0, stream>>>(w, b, kNext);
@@ -544,14 +542,14 @@ void launch_batch_wave(const WaveView& w, const BatchView& b, const uint32_t* so
   int cur = 0;
   for (int bounce = 0; bounce < bounces; ++bounce, cur ^= 1) {
     if (!timer) {
-      b_trace(cfg, bw, b, bounce > 0 ? TK_ALL : TK_EXT, cur, tgrid, !append, stream);
+      b_trace(cfg, bw, b, bounce > 0 ? TK_ALL : TK_EXT, cur, tgrid, !append, bounce == 0, stream);
       ++nl;
     } else {  // timed: kind by kind
       const int stage[3] = {ST_TRACE_EXT, ST_TRACE_SHADOW, ST_TRACE_MIS};
       const int kinds[3] = {TK_EXT, TK_SHADOW, TK_MIS | TK_MIS_ENV};
       for (int k = 0; k < (bounce > 0 ? 3 : 1); ++k)
         timed(stage[k], [&] {
-          b_trace(cfg, bw, b, kinds[k], cur, tgrid, !append, stream);
+          b_trace(cfg, bw, b, kinds[k], cur, tgrid, !append, bounce == 0, stream);
           return 1;
         });
     }
@@ -560,7 +558,7 @@ void launch_batch_wave(const WaveView& w, const BatchView& b, const uint32_t* so
         k_b_resolve<<<sgrid, cfg.shade_block, 0, stream>>>(bw, b, cur);
         return 1;
       });
-    const int* list = bw.q_ext[cur];
+    const int* list = bounce == 0 ? nullptr : bw.q_ext[cur];  // the slots traced this bounce
     const int* count = bw.counters + cnt_rays(RK_EXT, cur);
     if (!append)
       timed(ST_OTHER, [&] {

@@ -55,8 +55,6 @@ __global__ void k_camera(SceneView s, WaveView w, WaveArgs a) {
     r.d = f4(d, 0.f);
     r.hit = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
     r.meta = make_int4((int)dim, (int)(uint32_t)(uint64_t)index, 0, (int)((uint64_t)index >> 32));
-    w.q_ext[0][pid] = pid;
-    w.qflags[pid] = 0;
   }
 }
 
@@ -368,11 +366,11 @@ int grid_for(int64_t n, int block, int max_blocks) {
 }
 
 template <int SMEM, bool COUNT = false, int CAP = kMaxStack>
-void launch_trace_kernel(int kinds, const SceneView& s, const WaveView& w, int cur, bool marks, const LaunchConfig& cfg,
-                         int grid, cudaStream_t stream) {
+void launch_trace_kernel(int kinds, const SceneView& s, const WaveView& w, int cur, bool marks, bool camera_rays,
+                         const LaunchConfig& cfg, int grid, cudaStream_t stream) {
   TraceArgs a;
   a.scene = s;
-  wave_ray_sets(w, cur, marks, a.set);
+  wave_ray_sets(w, cur, marks, camera_rays, a.set);
   a.counters = w.counters;
   a.err = w.error_word;
   a.kinds = kinds;
@@ -383,22 +381,22 @@ void launch_trace_kernel(int kinds, const SceneView& s, const WaveView& w, int c
 }
 
 // kinds: TraceKinds bits.
-void trace_dispatch(int kinds, const SceneView& s, const WaveView& w, int cur, bool marks, const LaunchConfig& cfg,
-                    int grid, cudaStream_t stream) {
+void trace_dispatch(int kinds, const SceneView& s, const WaveView& w, int cur, bool marks, bool camera_rays,
+                    const LaunchConfig& cfg, int grid, cudaStream_t stream) {
   if (w.trace_work) {  // counting render: the stack's split between shared and local memory is irrelevant
-    launch_trace_kernel<0, true>(kinds, s, w, cur, marks, cfg, grid, stream);
+    launch_trace_kernel<0, true>(kinds, s, w, cur, marks, camera_rays, cfg, grid, stream);
     return;
   }
   if (cfg.test_stack_entries) {  // orion_gpu_set_test_limits: kernels with a kTestStackEntries-entry stack
-    launch_trace_kernel<0, false, kTestStackEntries>(kinds, s, w, cur, marks, cfg, grid, stream);
+    launch_trace_kernel<0, false, kTestStackEntries>(kinds, s, w, cur, marks, camera_rays, cfg, grid, stream);
     return;
   }
   switch (cfg.smem_stack) {
-    case 0: launch_trace_kernel<0>(kinds, s, w, cur, marks, cfg, grid, stream); break;
-    case 8: launch_trace_kernel<8>(kinds, s, w, cur, marks, cfg, grid, stream); break;
-    case 24: launch_trace_kernel<24>(kinds, s, w, cur, marks, cfg, grid, stream); break;
-    case 32: launch_trace_kernel<32>(kinds, s, w, cur, marks, cfg, grid, stream); break;
-    default: launch_trace_kernel<16>(kinds, s, w, cur, marks, cfg, grid, stream); break;
+    case 0: launch_trace_kernel<0>(kinds, s, w, cur, marks, camera_rays, cfg, grid, stream); break;
+    case 8: launch_trace_kernel<8>(kinds, s, w, cur, marks, camera_rays, cfg, grid, stream); break;
+    case 24: launch_trace_kernel<24>(kinds, s, w, cur, marks, camera_rays, cfg, grid, stream); break;
+    case 32: launch_trace_kernel<32>(kinds, s, w, cur, marks, camera_rays, cfg, grid, stream); break;
+    default: launch_trace_kernel<16>(kinds, s, w, cur, marks, camera_rays, cfg, grid, stream); break;
   }
 }
 
@@ -466,28 +464,29 @@ void launch_wave(const SceneView& s, const WaveView& w, const WaveArgs& a, const
     // The bounce's extension rays and the previous bounce's light rays. A
     // render that times its stages traces them kind by kind.
     if (!timer) {
-      trace_dispatch(bounce > 0 ? TK_ALL : TK_EXT, s, w, cur, !a.append, cfg, tgrid, stream);
+      trace_dispatch(bounce > 0 ? TK_ALL : TK_EXT, s, w, cur, !a.append, bounce == 0, cfg, tgrid, stream);
       ++nl;
     } else {
       begin(ST_TRACE_EXT);
-      trace_dispatch(TK_EXT, s, w, cur, !a.append, cfg, tgrid, stream);
+      trace_dispatch(TK_EXT, s, w, cur, !a.append, bounce == 0, cfg, tgrid, stream);
       end();
       if (bounce > 0) {
         begin(ST_TRACE_SHADOW);
-        trace_dispatch(TK_SHADOW, s, w, cur, !a.append, cfg, tgrid, stream);
+        trace_dispatch(TK_SHADOW, s, w, cur, !a.append, bounce == 0, cfg, tgrid, stream);
         end();
         begin(ST_TRACE_MIS);
-        trace_dispatch(TK_MIS | TK_MIS_ENV, s, w, cur, !a.append, cfg, tgrid, stream);
+        trace_dispatch(TK_MIS | TK_MIS_ENV, s, w, cur, !a.append, bounce == 0, cfg, tgrid, stream);
         end();
       }
     }
+    const int* list = bounce == 0 ? nullptr : w.q_ext[cur];  // the slots traced this bounce
     if (!a.append) {  // the trace marked each finished ray's shading class: list them by class in slot order
       begin(ST_OTHER);
       CompactTargets tg{};
       for (int c = 0; c < kShadeClasses; ++c)
         tg.queue[c] = w.q_cls + (size_t)c * w.capacity, tg.counter[c] = w.counters + cnt_cls(c, cur);
       k_compact_queues<kShadeClasses><<<compact_grid, kCompactThreads, 0, stream>>>(
-          w.qflags, w.q_ext[cur], w.counters + cnt_rays(RK_EXT, cur), tg);
+          w.qflags, list, w.counters + cnt_rays(RK_EXT, cur), tg);
       end();
     }
     begin(ST_SHADE);
@@ -499,7 +498,7 @@ void launch_wave(const SceneView& s, const WaveView& w, const WaveArgs& a, const
       int* qs[kRayKinds] = {w.q_ext[cur ^ 1], w.q_mis, w.q_sh, w.q_mis_env};  // as the QueueFlag bits
       for (int k = 0; k < kRayKinds; ++k) tg.queue[k] = qs[k], tg.counter[k] = w.counters + cnt_rays(k, cur ^ 1);
       k_compact_queues<kRayKinds><<<compact_grid, kCompactThreads, 0, stream>>>(
-          w.qflags, w.q_ext[cur], w.counters + cnt_rays(RK_EXT, cur), tg);
+          w.qflags, list, w.counters + cnt_rays(RK_EXT, cur), tg);
       end();
     }
     // No resolve pass: each path's light sample is added to its radiance by
@@ -538,7 +537,7 @@ void launch_trace_wave(const SceneView& s, const WaveView& w, int n, const float
   k_reset_counters<<<1, 32, 0, stream>>>(w.counters, kCounterSlots, cnt_rays(any_hit ? RK_SHADOW : RK_EXT, 0), n);
   k_load_rays<<<grid_for(n, 256, 4096), 256, 0, stream>>>(w, n, rays, any_hit);
   const int tgrid = grid_for(n, cfg.trace_block, cfg.num_sms * cfg.blocks_per_sm);
-  trace_dispatch(any_hit ? TK_SHADOW : TK_EXT, s, w, 0, true, cfg, tgrid, stream);
+  trace_dispatch(any_hit ? TK_SHADOW : TK_EXT, s, w, 0, true, false, cfg, tgrid, stream);
   k_store_hits<<<grid_for(n, 256, 4096), 256, 0, stream>>>(w, n, any_hit, t, u, v, prim);
 }
 

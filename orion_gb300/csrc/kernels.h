@@ -176,7 +176,7 @@ struct BatchView {
 // that of path slot queue[k], its origin and direction at o / d + slot x
 // stride (float4 units).
 struct RaySet {
-  const int* queue;
+  const int* queue;   // null: ray k is slot k's (a wave's camera rays)
   const int* count;
   int* fetch;         // next ray to take; zero at launch
   const float4* o;    // any hit: w = tmax
@@ -196,8 +196,9 @@ struct RaySet {
 };
 
 // The rays of a wave of parity `cur`, by RayKind. marks: the shading classes
-// go to the slots' flag bytes.
-inline void wave_ray_sets(const WaveView& w, int cur, bool marks, RaySet set[kRayKinds]) {
+// go to the slots' flag bytes. camera_rays: the extension rays are those of all
+// slots, in order, and no queue lists them.
+inline void wave_ray_sets(const WaveView& w, int cur, bool marks, bool camera_rays, RaySet set[kRayKinds]) {
   constexpr int kRec = sizeof(PathRec) / sizeof(float4), kNee = sizeof(NeeRec) / sizeof(float4);
   unsigned long long* work = w.trace_work;
   auto of = [&](int kind, const int* q, const float4* o, const float4* d, int stride, float4* hit, int hit_stride,
@@ -206,7 +207,7 @@ inline void wave_ray_sets(const WaveView& w, int cur, bool marks, RaySet set[kRa
                        stride, hit_stride, nullptr, nullptr, nullptr, 0, w.ray_stats + stat,
                        work ? work + stat : nullptr};
   };
-  of(RK_EXT, w.q_ext[cur], w.ray_o.p, w.ray_d.p, kRec, w.hit.p, kRec, nullptr, 0);
+  of(RK_EXT, camera_rays ? nullptr : w.q_ext[cur], w.ray_o.p, w.ray_d.p, kRec, w.hit.p, kRec, nullptr, 0);
   of(RK_MIS, w.q_mis, w.mis_o.p, w.mis_d.p, kNee, w.mis_hit, 1, nullptr, 2);
   of(RK_SHADOW, w.q_sh, w.sh_o.p, w.sh_d.p, kNee, nullptr, 0, w.occluded, 1);
   of(RK_MIS_ENV, w.q_mis_env, w.mis_o.p, w.mis_d.p, kNee, nullptr, 0, w.mis_occluded, 2);

@@ -447,7 +447,8 @@ struct JobScene {
 // their triangle tests to rs.work[3]. A ray whose traversal overflowed its
 // stack (capacity CAP) is reported as a miss (not occluded) and sets
 // kErrTraversalStack in *err.
-template <bool ANY, int SMEM, bool COUNT = false, int CAP = kMaxStack, class SceneOf>
+// UNLISTED: rs.queue may be null.
+template <bool ANY, bool UNLISTED, int SMEM, bool COUNT = false, int CAP = kMaxStack, class SceneOf>
 __device__ __forceinline__ void trace_persistent(const SceneOf& scene_of, const RaySet& rs, int n, int2* stack_smem,
                                                  int refill_below, int* err) {
   constexpr unsigned kFull = 0xffffffffu;
@@ -481,7 +482,7 @@ __device__ __forceinline__ void trace_persistent(const SceneOf& scene_of, const 
       if (!active) {
         const int my = base + __popc(idle & ((1u << lane) - 1u));
         if (my < n) {
-          pid = rs.queue[my];
+          pid = !UNLISTED || rs.queue ? rs.queue[my] : my;
           // The ray and its result pass through once: streaming (evict-first) accesses
           // leave L1 and L2 to the BVH nodes and triangles (displaced sphere +1.2%).
           const int64_t at = (int64_t)pid * rs.stride;
@@ -586,25 +587,27 @@ __device__ __forceinline__ void trace_kinds(const SceneOf& scene_of, const RaySe
       const int count = (kinds >> kind) & 1 ? *r.count : 0;
       if (count == 0) continue;
       if (kind < 2)
-        trace_persistent<false, SMEM, COUNT, CAP>(scene_of, r, count, stack_smem, refill_closest, err);
+        trace_persistent<false, true, SMEM, COUNT, CAP>(scene_of, r, count, stack_smem, refill_closest, err);
       else
-        trace_persistent<true, SMEM, COUNT, CAP>(scene_of, r, count, stack_smem, refill_any, err);
+        trace_persistent<true, false, SMEM, COUNT, CAP>(scene_of, r, count, stack_smem, refill_any, err);
     }
     return;
   }
-#pragma unroll  // four copies of the loop, each with its kind's pointers as constants (no spills)
-  for (int k = 0; k < 4; ++k) {
-    const int count = (kinds >> k) & 1 ? *set[k].count : 0;
-    if (count == 0) continue;
-    if (k < 2)
-      trace_persistent<false, SMEM, COUNT, CAP>(scene_of, set[k], count, stack_smem, refill_closest, err);
-    else
-      trace_persistent<true, SMEM, COUNT, CAP>(scene_of, set[k], count, stack_smem, refill_any, err);
-  }
+  // Four copies of the loop, each with its kind's pointers as constants.
+  auto kind_count = [&](int k) { return (kinds >> k) & 1 ? *set[k].count : 0; };
+  if (const int count = kind_count(RK_EXT))
+    trace_persistent<false, true, SMEM, COUNT, CAP>(scene_of, set[RK_EXT], count, stack_smem, refill_closest, err);
+  if (const int count = kind_count(RK_MIS))
+    trace_persistent<false, false, SMEM, COUNT, CAP>(scene_of, set[RK_MIS], count, stack_smem, refill_closest, err);
+  if (const int count = kind_count(RK_SHADOW))
+    trace_persistent<true, false, SMEM, COUNT, CAP>(scene_of, set[RK_SHADOW], count, stack_smem, refill_any, err);
+  if (const int count = kind_count(RK_MIS_ENV))
+    trace_persistent<true, false, SMEM, COUNT, CAP>(scene_of, set[RK_MIS_ENV], count, stack_smem, refill_any, err);
 }
 
 // Lists slots in queues from their qflags bytes: bit b of a slot's byte puts
-// the slot in queue b. The slots looked at are list[0 .. *count) (the bounce's
+// the slot in queue b. The slots looked at are list[0 .. *count), or slots 0 ..
+// *count without a list (the bounce's
 // extension queue: every slot traced and shaded this bounce), so the cost
 // follows the live paths, not the wave. Blocks of kCompactThreads threads take
 // spans of kCompactSpan list entries in turn: list order within a span (a
@@ -631,7 +634,10 @@ __device__ __forceinline__ void compact_queues(uint8_t* flags, const int* list, 
     const int p0 = span * kCompactSpan + t * kCompactItems;
     int slot[kCompactItems];
     uint32_t words[4] = {0u, 0u, 0u, 0u};
-    if (p0 + kCompactItems <= n) {  // p0 is a multiple of 16: four aligned 16-byte loads of the list
+    if (!list) {
+#pragma unroll
+      for (int j = 0; j < kCompactItems; ++j) slot[j] = p0 + j < n ? p0 + j : -1;
+    } else if (p0 + kCompactItems <= n) {  // p0 is a multiple of 16: four aligned 16-byte loads of the list
       const int4* l4 = reinterpret_cast<const int4*>(list + p0);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
