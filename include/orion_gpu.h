@@ -282,10 +282,9 @@ int orion_film_write_bmp(const char* path, int32_t width, int32_t height, const 
 /* ------------------------------------------------------------- batches */
 /* Many render() calls in one launch. There is no single reference call for
  * this: it runs PathTracing::render (src/integrator/path.cpp:15-37) for every
- * job, sharing one pool of path slots across jobs (finished slots are
- * refilled with the next job's paths), inside one CUDA graph launch whose
- * device-side loop runs until every job's paths are done. Per-path results
- * are the plain render's; films are accumulated in FP64. */
+ * job, the jobs' paths sharing launches: in waves of path slots, or in one
+ * pool of slots refilled by a device-side loop (orion_gpu_set_batch_mode).
+ * Per-path results are the plain render's; films are accumulated in FP64. */
 typedef struct orion_job {
   orion_scene_id scene;
   int32_t reserved;
@@ -301,9 +300,9 @@ typedef struct orion_job {
 typedef struct orion_batch_stats {
   int64_t paths;               /* camera paths traced */
   int64_t rays;                /* extension + shadow + MIS rays */
-  int64_t iterations;          /* device loop iterations */
+  int64_t iterations;          /* pooled: device loop iterations; waves: bounces launched, over all waves */
   int64_t capacity;            /* path slots in the pool */
-  double device_ms;            /* device time of the graph launch */
+  double device_ms;            /* device time of the launches */
 } orion_batch_stats;
 
 int orion_gpu_render_batch(orion_gpu_ctx* ctx, int32_t njobs, const orion_job* jobs, orion_batch_stats* stats);
@@ -326,7 +325,7 @@ typedef struct orion_launch_config {
 
 /* How orion_gpu_render_batch (and the server) run a batch:
  * ORION_BATCH_WAVES (default): the jobs' concatenated work list in waves of
- *   batch_slots paths, each wave's paths bouncing until none is alive;
+ *   batch_slots paths, each launched for as many bounces as the deepest job has;
  * ORION_BATCH_POOLED: a pool of batch_slots path slots refilled from the
  *   work list every bounce. */
 enum { ORION_BATCH_POOLED = 0, ORION_BATCH_WAVES = 1 };
@@ -410,7 +409,7 @@ int orion_gpu_trace(orion_gpu_ctx* ctx, orion_scene_id id, int64_t n, const floa
                     float* t, float* u, float* v, int32_t* prim);
 /* The same queries traced by the renderer's own persistent kernels: closest-hit
  * rays become a wave's extension rays (k_trace), any-hit rays its shadow rays
- * (k_trace_sh, occlusion within (0, tfar]). Every ray's tnear must be 0, as
+ * (k_trace, occlusion within (0, tfar]). Every ray's tnear must be 0, as
  * for the renderer's rays; closest-hit rays ignore tfar (extension rays are
  * unbounded). prim = -1 for a miss; for any_hit = 1, prim = 1 when occluded
  * and t, u, v are 0. Replaces rtcIntersect / rtcOccluded as the renderer calls

@@ -3,8 +3,8 @@
 // The jobs' sample ranges are concatenated into one work list, which runs in
 // one of two ways. Wave mode takes a wave of contiguous work items onto slots
 // 0..n-1 and runs the plain render's pipeline on them, each path against its
-// job's scene (k_wb_camera, then k_b_trace, k_wb_compact, k_b_shade per bounce,
-// then k_wb_film). Pooled mode shares one pool of slots among all jobs and
+// job's scene (k_wb_camera, then k_b_trace, k_b_resolve, k_wb_compact, k_b_shade
+// per bounce, then k_wb_film). Pooled mode shares one pool of slots among all jobs and
 // refills finished slots every iteration of a loop inside a CUDA graph
 // while-node:
 //

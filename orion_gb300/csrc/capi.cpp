@@ -1,11 +1,12 @@
 // C ABI (include/orion_gpu.h): context, resident scenes, render driver.
 //
 // PathTracing::render (src/integrator/path.cpp:15-37) loops over spp passes
-// and pixels, one CPU thread per row. Here the sample indices
-// [k0*W*H, (k0+spp)*W*H) are cut into waves of up to `wave_paths` paths; each
-// wave is one fixed sequence of kernels on the context's stream (no host
-// synchronisation inside a render), and the film is accumulated per pixel in
-// sample order so its FP32 sums follow the reference's addition order.
+// and pixels, one CPU thread per row. Here the film's pixels are cut into
+// waves of up to `wave_paths` paths, all samples of a pixel in one wave; each
+// wave is one fixed sequence of kernels (no host synchronisation inside a
+// render), waves take turns on up to four streams, and the film is accumulated
+// per pixel in sample order so its FP32 sums follow the reference's addition
+// order.
 #include <cuda_runtime.h>
 #include <dlfcn.h>
 

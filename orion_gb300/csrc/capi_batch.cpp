@@ -2,13 +2,14 @@
 // orion_gpu_set_batch_mode, orion_gpu_autotune_batch).
 //
 // PathTracing::render (src/integrator/path.cpp:15-37) renders one scene per
-// call. A batch renders many (scene, spp, film) jobs in one device-side loop,
-// captured once as a CUDA graph and replayed until every job's samples are
-// done. Two modes share the plain render's kernels:
+// call. A batch renders many (scene, spp, film) jobs together. Two modes share
+// the plain render's device functions:
 //   pooled - a fixed pool of path slots; finished paths retire their film
-//            sample and the slot takes the next sample index of any job;
+//            sample and the slot takes the next sample index of any job, in a
+//            device-side loop captured once as a CUDA graph;
 //   waves  - the jobs' sample indices are laid end to end and cut into waves
-//            of `batch_slots` paths, each wave run to completion.
+//            of `batch_slots` paths, each wave the plain render's launches for
+//            the deepest job's bounces, with no graph.
 // Up to two engines run a batch concurrently, engine e on the wave state and
 // stream of plain-render wave slot e.
 #include <cuda_runtime.h>

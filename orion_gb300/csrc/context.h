@@ -151,7 +151,7 @@ struct BatchGraph {
 };
 
 // One batch engine: its free and retire lists, control block, job table and
-// captured device-side loop (the path slots are a Wave).
+// pooled mode's captured loop (the path slots are a Wave).
 struct BatchEngine {
   DevBuf retire, free_list, ctl, jobs;
   int slots_alloc = 0, jobs_alloc = 0;
@@ -185,7 +185,7 @@ struct orion_gpu_ctx {
   Wave wave;
   // Plain renders overlap consecutive waves on up to kWaveStreams streams:
   // per extra stream its wave state, the stream, its join event; the events
-  // that order the film writes wave after wave.
+  // that order the film writes of waves with other passes of the same pixels.
   static constexpr int kWaveStreams = orion_gb300::kMaxWaveStreams;
   // Four: the eight-sphere 1080p render (eight waves) 2583 -> 2822 Mpaths/s
   // against two. Renders of fewer than two full waves are split two ways

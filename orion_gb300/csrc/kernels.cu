@@ -271,7 +271,7 @@ __global__ void k_trace_any(SceneView s, int64_t n, const float* rays, float* t,
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const float* r = rays + 8 * i;
     V3 o = V3{r[0], r[1], r[2]}, d = V3{r[3], r[4], r[5]};
-    RayHit h = traverse<true, SMEM>(ts, o, d, r[6], r[7], st);
+    RayHit h = traverse_any(ts, o, d, r[6], r[7], st);
     t[i] = h.tri >= 0 ? h.t : 0.f;
     u[i] = h.u;
     v[i] = h.v;

@@ -257,29 +257,26 @@ __device__ __forceinline__ int take_child(uint2& ng, uint32_t oct) {
   return child;
 }
 
-// ANY = false: closest hit over (tnear, tfar]. ANY = true: first hit found,
-// children visited far to near (see lane_visit). A stack overflow ends the
-// traversal with a miss (see the file comment).
-template <bool ANY, int SMEM, int CAP>
-__device__ __forceinline__ RayHit traverse(const TraceScene& s, V3 o, V3 d, float tnear, float tfar,
-                                           TraversalStack<SMEM, CAP>& st) {
+// First hit found over (tnear, tfar], one ray per thread, children visited far
+// to near (see lane_visit). A stack overflow ends the traversal with a miss
+// (see the file comment).
+template <int SMEM, int CAP>
+__device__ __forceinline__ RayHit traverse_any(const TraceScene& s, V3 o, V3 d, float tnear, float tfar,
+                                               TraversalStack<SMEM, CAP>& st) {
   RayHit h;
   h.t = tfar;
   h.u = h.v = 0.f;
   h.tri = -1;
   const V3 idir = V3{safe_inv(d.x), safe_inv(d.y), safe_inv(d.z)};
   const uint32_t oct = ray_octant(idir);
-  const uint32_t ord = ANY ? oct ^ 7u : oct;
-  int best_prim = 0x7fffffff;
+  const uint32_t ord = oct ^ 7u;
   st.sp = 0;
   uint2 ng = root_group(ord), tg = make_uint2(0u, 0u);
   while (true) {
     if (ng.y > 0x00ffffffu) {
       const int child = take_child(ng, ord);
-      if (ng.y && !st.push(make_int2((int)ng.x, (int)ng.y))) {
+      if (ng.y && !st.push(make_int2((int)ng.x, (int)ng.y)))
         h.t = -1.f;  // poisoned: nothing passes a test against tmax < tnear
-        h.tri = -1;
-      }
       wide_node(s.nodes, child, o, idir, oct, tnear, h.t, ng, tg, ord);
     } else {
       tg = ng;
@@ -290,21 +287,11 @@ __device__ __forceinline__ RayHit traverse(const TraceScene& s, V3 o, V3 d, floa
       tg.y &= tg.y - 1u;
       float t, u, v;
       if (woop_hit(s.woop, k, o, d, tnear, h.t, &t, &u, &v)) {
-        if (ANY) {
-          h.t = t;
-          h.u = u;
-          h.v = v;
-          h.tri = k;
-          return h;
-        }
-        const int prim = __ldg(s.tri_prim + k);
-        if (t < h.t || h.tri < 0 || prim < best_prim) {
-          h.t = t;
-          h.u = u;
-          h.v = v;
-          h.tri = k;
-          best_prim = prim;
-        }
+        h.t = t;
+        h.u = u;
+        h.v = v;
+        h.tri = k;
+        return h;
       }
     }
     if (ng.y == 0u) {
@@ -313,10 +300,7 @@ __device__ __forceinline__ RayHit traverse(const TraceScene& s, V3 o, V3 d, floa
       ng = make_uint2((uint32_t)e.x, (uint32_t)e.y);
     }
   }
-  if (h.t < 0.f) {  // stack overflow: reported as a miss
-    h.t = tfar;
-    h.tri = -1;
-  }
+  if (h.t < 0.f) h.t = tfar;  // stack overflow: reported as a miss
   return h;
 }
 
