@@ -91,8 +91,8 @@ def test_traversal_work_counts(ctx, scene):
 def test_pixel_order_at_ragged_sizes(ctx, width, height, spp):
     """Slots run pixel after pixel through tiles of 8 x 4 pixels, each pixel's passes in order, and the
     film adds up to 256 samples of a pixel at a go: films with cut-off tiles, chunks and sample runs
-    equal the batch engine's, which numbers its slots pass after pass (FP64 sums, 1e-5 as its tests:
-    the two engines' FP32 paths are compiled apart), and do not depend on the wave size."""
+    equal the batch engine's, which has kernels of its own (FP64 sums, 1e-5 as its tests: the two
+    engines' FP32 paths are compiled apart), and do not depend on the wave size."""
     from orion_gb300 import scenegen
     s = scenegen.zoo(subdiv=1, spp=spp, max_depth=3)
     s.width, s.height = width, height
@@ -125,5 +125,30 @@ def test_appended_and_compacted_queues_agree(ctx, paths):
         many, c = ctx.render(sid, 64, 64, wave_paths=1 << 16)
         assert np.array_equal(c, cnt) and (cnt == paths // 4096).all()
         assert np.array_equal(one.view(np.uint32), many.view(np.uint32))
+    finally:
+        ctx.release(sid)
+
+
+@pytest.mark.parametrize("spp", [1, 7, 8, 9, 31, 255, 256, 257])
+def test_batch_film_adds_every_run_of_samples(ctx, spp):
+    """A batch wave's film kernel takes 256 slots at a time and adds up each pixel's run of samples in
+    pieces of 8: runs of one sample to more than 256, cut at block ends and (behind a job of 3 samples
+    a pixel, 13 x 7 pixels) at odd slots, with squares and without. Sums and squares as
+    the plain FP64 render's to FP32 rounding (1e-5, as the batch tests), counts exactly."""
+    from orion_gb300 import scenegen
+    s = scenegen.zoo(subdiv=1, spp=spp, max_depth=2)
+    s.width, s.height = 13, 7
+    sid = ctx.upload(scenegen.to_host_scene(s))
+    try:
+        jobs = [dict(sid=sid, width=13, height=7, spp=3), dict(sid=sid, width=13, height=7, spp=spp, first_pass=2)]
+        films = ctx.render_batch(jobs)[0]
+        for job, (got, sq, count) in zip(jobs, films):
+            want, want_sq = ctx.render(sid, 13, 7, spp=job["spp"], first_pass=job.get("first_pass", 0), fp64=True)
+            assert (count == job["spp"]).all()
+            assert np.allclose(got, want, rtol=1e-5, atol=1e-7)
+            assert np.allclose(sq, want_sq, rtol=1e-5, atol=1e-7)
+        only_sums = ctx.render_batch(jobs, sumsq=False)[0]
+        for a, b in zip(films, only_sums):
+            assert np.allclose(a[0], b[0], rtol=1e-12, atol=1e-12)
     finally:
         ctx.release(sid)
