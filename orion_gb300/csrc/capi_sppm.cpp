@@ -71,7 +71,7 @@ extern "C" int orion_gpu_render_sppm(orion_gpu_ctx* ctx, orion_scene_id id, cons
   }
   v.vp_pr = f4s[0], v.vp_wo = f4s[1], v.vp_beta = f4s[2], v.vp_ns = f4s[3], v.vp_ng = f4s[4];
   v.vp_su = f4s[5], v.vp_sv = f4s[6], v.ld = f4s[7], v.tau = f4s[8];
-  v.photon_next = v.hit_count + 1;
+  v.photon_next = reinterpret_cast<unsigned*>(v.hit_count + 1);
   v.num_sms = ctx->num_sms;
   v.width = W;
   v.height = H;

@@ -405,7 +405,7 @@ struct SppmView {
   int hits_cap;     // photons x (max depth - 1): every hit after a photon's first
   int* hit_count;
   DevMaterial* photon_mats;  // the scene's materials with DevLobe::photon set
-  int* photon_next;  // next photon to start (beside hit_count: cleared together)
+  unsigned* photon_next;  // next photon to start (beside hit_count: cleared together)
   int num_sms;
   // hash cell -> photon hits: cell h holds records [cell_start[h], cell_start[h + 1]) of by_cell
   int* cell_start;  // npix + 1 (counts, then their exclusive scan)
@@ -416,6 +416,14 @@ struct SppmView {
   unsigned* film_count;
   unsigned long long* rays;
 };
+
+// Whether the photons [base, base + count) that a warp took from photon_next reach
+// the end of an iteration's `photons`. Every warp takes past the end once, at most 32
+// photons: the counter is unsigned, so that it holds INT32_MAX photons and that of
+// more warps than a launch has.
+ORION_HD inline bool photons_dealt(unsigned base, unsigned count, int photons) {
+  return base + count >= (unsigned)photons;
+}
 
 constexpr int kSppmBoundsBlocks = 1024;  // blocks of the bounds pass (part_lo / part_hi entries)
 constexpr int kScanBlock = 1024;         // elements per block of the cell-count scan

@@ -364,8 +364,8 @@ __device__ __forceinline__ unsigned cell_hash(int x, int y, int z, int size) {
 // each cell's first entry after the scan), so a gather reads a cell's hits
 // from consecutive records.
 __global__ void __launch_bounds__(256) k_sppm_fill(SppmView v) {
-  const int n = min(*v.hit_count, v.hits_cap);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  const unsigned n = (unsigned)min(*v.hit_count, v.hits_cap);  // up to INT32_MAX: i goes past it by a stride
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float4* src = v.hits + 3 * (size_t)i;
     const float4 a = src[0], b = src[1], c = src[2];
     const unsigned h = (unsigned)__float_as_int(a.w);
@@ -574,13 +574,13 @@ __global__ void __launch_bounds__(kPhotonBlock, 2) k_sppm_photons(SceneView s, S
   while (true) {
     const unsigned act = __ballot_sync(kFull, on);
     if (!exhausted && __popc(act) < kPhotonRefill) {
-      const int cnt = 32 - __popc(act);
-      int base = 0;
+      const unsigned cnt = 32 - __popc(act);
+      unsigned base = 0;
       if (lane == 0) base = atomicAdd(v.photon_next, cnt);
       base = __shfl_sync(kFull, base, 0);
-      exhausted = base + cnt >= v.photons;
-      const int k = base + __popc(~act & ((1u << lane) - 1u));
-      if (!on && k < v.photons) {
+      exhausted = photons_dealt(base, cnt, v.photons);
+      const unsigned k = base + __popc(~act & ((1u << lane) - 1u));
+      if (!on && k < (unsigned)v.photons) {
         smp.index = (uint64_t)v.iterations * v.npix + (uint64_t)iter * v.photons + (uint64_t)k;
         smp.dim = 5u;
         float light_pdf;
@@ -671,7 +671,7 @@ __device__ __forceinline__ void clear_cells(const SppmView& v, int pix) {
   if (pix == 0) {
     v.cell_start[v.npix] = 0;
     *v.hit_count = 0;
-    *v.photon_next = 0;
+    *v.photon_next = 0u;
   }
 }
 

@@ -1,0 +1,40 @@
+"""Host code and index arithmetic that the kernels share, compiled alone (g++, no GPU) and driven at
+its limits by small programs under tests/native."""
+from __future__ import annotations
+
+import os
+import subprocess
+
+import pytest
+
+from orion_gb300 import build
+
+NATIVE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "native")
+
+
+@pytest.fixture(scope="module")
+def native(tmp_path_factory):
+    """native(name, *sources): path of tests/native/<name>.cpp compiled with the library's `sources`."""
+    out = tmp_path_factory.mktemp("native")
+
+    def compile_one(name, *sources):
+        exe = str(out / name)
+        subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-I", build.CSRC, "-I",
+                        os.path.join(build.CUDA_HOME, "include"), os.path.join(NATIVE, name + ".cpp"),
+                        *(os.path.join(build.CSRC, s) for s in sources), "-o", exe, "-lpthread", "-ldl"], check=True)
+        return exe
+
+    return compile_one
+
+
+def _run(exe, *args):
+    p = subprocess.run([exe, *map(str, args)], capture_output=True, text=True, timeout=120)
+    assert p.returncode == 0 and p.stdout.strip().endswith("ok"), (p.returncode, p.stdout, p.stderr)
+
+
+@pytest.mark.parametrize("photons,dealt", [(2**31 - 1, 2**31 - 200_001), (2**31 - 155_000, 2**31 - 160_000),
+                                           (100_000, 0), (31, 0)])
+def test_photons_near_the_largest_count_are_dealt_once(native, photons, dealt):
+    """k_sppm_photons' warps overshoot the last photon by up to 32 each: all of them stop, and each photon
+    is started once, up to the largest count that orion_gpu_render_sppm accepts."""
+    _run(native("photon_deal"), photons, dealt)
