@@ -385,8 +385,12 @@ __global__ void __launch_bounds__(256) k_sppm_fill(SppmView v) {
 // in short cells nor over the hits outside the sphere (738 -> 337 us against cell
 // after cell, each hit's BSDF where it is found: 592M -> 239M instructions).
 // Every lane runs the same material's BSDF, inline for the diffuse class; the
-// lanes' sums are added at the end.
+// lanes' sums are added at the end. The counts of 32 cells are summed in an int:
+// where one is above kGatherTogether (films of few pixels, whose few hash cells hold
+// many hits and turn up several times in one sphere) the cells go one by one.
 constexpr int kGatherWarps = 4;
+constexpr int kGatherTogether = 1 << 14;
+static_assert(32LL * kGatherTogether <= INT32_MAX, "the counts of a warp's cells are added up in an int");
 
 template <unsigned KM>
 __device__ __forceinline__ void gather_photons(const SppmView& v, const DevMaterial& m, const Frame& fr, V3 p, V3 wo,
@@ -405,7 +409,7 @@ __device__ __forceinline__ void gather_photons(const SppmView& v, const DevMater
       ++count;
     }
   };
-  for (int c0 = 0; c0 < cells; c0 += 32) {
+  for (int c0 = 0; c0 < cells;) {
     const int c = c0 + lane;
     int start = 0, in_cell = 0;
     if (c < cells) {
@@ -414,22 +418,25 @@ __device__ __forceinline__ void gather_photons(const SppmView& v, const DevMater
       start = v.cell_start[h];
       in_cell = v.cell_start[h + 1] - start;
     }
+    const bool alone = __any_sync(kFull, in_cell > kGatherTogether);  // the first cell only
+    if (alone && lane > 0) in_cell = 0;
+    c0 += alone ? 1 : 32;
     int incl = in_cell;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int y = __shfl_up_sync(kFull, incl, o);
       if (lane >= o) incl += y;
     }
-    const int total = __shfl_sync(kFull, incl, 31), before = incl - in_cell;
-    for (int e0 = 0; e0 < total; e0 += 32) {
-      const int e = e0 + lane;
+    const unsigned total = __shfl_sync(kFull, incl, 31), before = incl - in_cell;
+    for (unsigned e0 = 0; e0 < total; e0 += 32) {
+      const unsigned e = e0 + lane;
       int cell = 0;  // the last lane whose hits begin at or before e
 #pragma unroll
       for (int step = 16; step > 0; step >>= 1) {
-        const int at = __shfl_sync(kFull, before, cell + step);
+        const unsigned at = __shfl_sync(kFull, before, cell + step);
         if (at <= e) cell += step;
       }
-      const int idx = __shfl_sync(kFull, start, cell) + e - __shfl_sync(kFull, before, cell);
+      const int idx = __shfl_sync(kFull, start, cell) + (int)(e - __shfl_sync(kFull, before, cell));
       const bool in = e < total && !(length_sq(p - xyz(v.by_cell[3 * (size_t)idx])) > rr);
       const unsigned hits = __ballot_sync(kFull, in);
       if (in) queue[queued + __popc(hits & ((1u << lane) - 1u))] = idx;

@@ -252,6 +252,25 @@ def test_sppm_at_ragged_sizes(ctx, port, width, height, iterations, photons, rad
     assert np.sqrt(np.mean((gpu - ref) ** 2)) <= 0.01 * np.sqrt(np.mean(ref ** 2))
 
 
+@pytest.mark.parametrize("width,height,photons", [(2, 2, 300_000), (4, 3, 500_000)])
+def test_sppm_hash_cells_of_many_hits(ctx, port, width, height, photons):
+    """A film of few pixels has as few hash cells, so each holds far more photon hits than the gather adds up
+    together (2^14) and turns up many times in one sphere: cells one by one, the image within 1% RMSE as above
+    (thousands of photons a pixel)."""
+    from orion_gb300 import scenegen
+    s = scenegen.caustics(64, subdiv=2)
+    s.width, s.height = width, height
+    host = scenegen.to_host_scene(s)
+    kw = dict(iterations=1, photons=photons, radius=0.4, max_depth=5)
+    ref, _ = port.Scene(host).render_sppm(**kw)
+    sid = ctx.upload(host)
+    gpu, cnt = ctx.render_sppm(sid, width, height, **kw)
+    ctx.release(sid)
+    assert (cnt == 1).all() and np.isfinite(gpu).all()
+    ref = ref.astype(np.float64).reshape(gpu.shape)
+    assert np.sqrt(np.mean((gpu - ref) ** 2)) <= 0.01 * np.sqrt(np.mean(ref ** 2))
+
+
 def test_sppm_parameters_and_errors(ctx, tmp_path):
     import orion_gb300 as og
     path = helpers.write_scene("caustics", str(tmp_path / "c"), res=24, iterations=2, photons=-1, radius=0.1)
