@@ -19,6 +19,7 @@
 
 #include "context.h"
 #include "host_parallel.h"
+#include "wave_plan.h"
 
 using namespace orion_gb300;
 
@@ -485,39 +486,19 @@ static int render_impl(orion_gpu_ctx* ctx, orion_scene_id id, const orion_render
     if (nw < want) nw = want;
     wave = std::max<int64_t>(1, (total + nw - 1) / nw);
   }
-  // A wave renders `passes` passes of some chunks of the film's pixels
-  // (WaveArgs). Only a wave smaller than a pixel's samples splits them: then
-  // several groups of passes follow one another.
-  const int64_t groups = (spp + wave - 1) / std::max<int64_t>(wave, 1);
-  const int passes = (int)((spp + groups - 1) / groups);
-  const int64_t wave_pixels = std::max<int64_t>(1, wave / passes);
-  int chunk_log2 = 8;  // at most a sixteenth of a wave's pixels
-  while (chunk_log2 > 0 && (int64_t)16 << chunk_log2 > wave_pixels) --chunk_log2;
-  const int64_t chunks = (wh + ((int64_t)1 << chunk_log2) - 1) >> chunk_log2;
-  // The film's waves: as few as `wave` allows, where the last chunk may take a
-  // wave over it (by a sixteenth at most) unless the caller set it.
-  const int64_t group_waves =
-      p.wave_paths > 0 ? (chunks + std::max<int64_t>(1, wave_pixels >> chunk_log2) - 1) /
-                             std::max<int64_t>(1, wave_pixels >> chunk_log2)
-                       : std::min<int64_t>(chunks, (wh + wave_pixels - 1) / wave_pixels);
-  // Wave k's chunks are k, k + group_waves, ...; the last chunk may be partial.
-  auto pixels_of = [&](int64_t k) {
-    const int64_t n = (chunks - k + group_waves - 1) / group_waves;
-    const bool has_last = (chunks - 1) % group_waves == k;
-    return (n << chunk_log2) - (has_last ? (chunks << chunk_log2) - wh : 0);
-  };
-  const int64_t capacity = std::min<int64_t>(((chunks + group_waves - 1) / group_waves) << chunk_log2, wh) * passes;
-  int rc = ensure_wave(ctx, (int)capacity);
+  const WavePlan plan = plan_waves(wh, spp, std::max<int64_t>(wave, 1), p.wave_paths > 0);
+  const int capacity = (int)plan.capacity();
+  int rc = ensure_wave(ctx, capacity);
   if (rc != ORION_OK) return rc;
   // Waves take turns on `ns` streams, each with its own path-state block, so
   // one wave's kernels fill the SMs that another's kernel tails leave idle.
   // Waves of other passes of the same pixels write the film one after the
   // other (events), so every pixel still sums its samples in sample order.
   // Profiled renders stay on one stream so that stage times add up.
-  const int64_t nwaves = groups * group_waves;
+  const int64_t nwaves = plan.groups * plan.group_waves;
   const int ns = ctx->profiling ? 1 : (int)std::min<int64_t>(ctx->wave_streams, nwaves);
   for (int i = 1; i < ns; ++i)
-    if ((rc = alloc_wave(ctx->xwave[i - 1], (int)capacity)) != ORION_OK) return rc;
+    if ((rc = alloc_wave(ctx->xwave[i - 1], capacity)) != ORION_OK) return rc;
   auto wave_view = [&](int i) -> const WaveView& { return i == 0 ? ctx->wave.view : ctx->xwave[i - 1].view; };
   auto wave_stream = [&](int i) { return i == 0 ? ctx->stream : ctx->xstream[i - 1]; };
   const bool fp64 = sum64 != nullptr;
@@ -549,23 +530,23 @@ static int render_impl(orion_gpu_ctx* ctx, orion_scene_id id, const orion_render
   }
   for (int64_t k = 0; k < nwaves; ++k) {
     const int slot = (int)(k % ns);
-    const int64_t group = k / group_waves;
+    const int64_t group = k / plan.group_waves;
     WaveArgs a;
     a.sobol = ctx->sobol.as<uint32_t>();
-    a.first_pass = p.first_pass + group * passes;
-    a.passes = (int)std::min<int64_t>(passes, spp - group * passes);
-    a.wave = (int)(k % group_waves);
-    a.waves = (int)group_waves;
-    a.chunk_log2 = chunk_log2;
+    a.first_pass = p.first_pass + group * plan.passes;
+    a.passes = (int)std::min<int64_t>(plan.passes, spp - group * plan.passes);
+    a.wave = (int)(k % plan.group_waves);
+    a.waves = (int)plan.group_waves;
+    a.chunk_log2 = plan.chunk_log2;
     a.add = group > 0;
-    a.n_paths = (int)(pixels_of(a.wave) * a.passes);
+    a.n_paths = (int)(plan.pixels_of(a.wave) * a.passes);
     a.width = d.width;
     a.height = d.height;
     a.max_depth = max_depth;
     a.rr_depth = rr_depth;
     a.append = a.n_paths <= kAppendPaths;
     a.class_mask = d.class_mask;
-    const bool ordered = ns > 1 && groups > 1;
+    const bool ordered = ns > 1 && plan.groups > 1;
     const cudaEvent_t film_wait = ordered && k > 0 ? ctx->ev_film[(k - 1) % ns] : nullptr;
     const cudaEvent_t film_done = ordered ? ctx->ev_film[k % ns] : nullptr;
     WaveView wv = wave_view(slot);

@@ -38,3 +38,15 @@ def test_photons_near_the_largest_count_are_dealt_once(native, photons, dealt):
     """k_sppm_photons' warps overshoot the last photon by up to 32 each: all of them stop, and each photon
     is started once, up to the largest count that orion_gpu_render_sppm accepts."""
     _run(native("photon_deal"), photons, dealt)
+
+
+INT32_MAX = 2**31 - 1
+
+
+@pytest.mark.parametrize("pixels,spp,wave,exact", [
+    (740 * 1451, 4000, INT32_MAX, 0),  # a wave rounded up to whole chunks would pass INT32_MAX paths
+    (740 * 1451, 4000, INT32_MAX, 1), (2 * 2**27 + 2, 8, INT32_MAX - 7, 0), (1, INT32_MAX, INT32_MAX, 0),
+    (1, 7, 3, 1), (33 * 6, 255, 64, 0), (33 * 6, 255, 1000, 1), (1920 * 1080, 128, 1 << 25, 0),
+    (1024 * 1024, 64, 1 << 25, 0), (257, 1, 100, 0), (7 * 41, 257, 7 * 41 * 257, 0)])
+def test_waves_cover_the_film_within_their_capacity(native, pixels, spp, wave, exact):
+    _run(native("wave_plan"), pixels, spp, wave, exact)
