@@ -504,6 +504,14 @@ static int render_impl(orion_gpu_ctx* ctx, orion_scene_id id, const orion_render
   const bool fp64 = sum64 != nullptr;
   if ((rc = ensure_film(ctx, wh, fp64)) != ORION_OK) return rc;
   cudaStream_t s = ctx->stream;
+  if (nwaves == 0) {  // no samples: no wave writes the film
+    CUDA_TRY(cudaMemsetAsync(ctx->film_sum.p, 0, wh * 3 * sizeof(float), s));
+    CUDA_TRY(cudaMemsetAsync(ctx->film_count.p, 0, wh * sizeof(uint32_t), s));
+    if (fp64) {
+      CUDA_TRY(cudaMemsetAsync(ctx->film64.p, 0, wh * 3 * sizeof(double), s));
+      CUDA_TRY(cudaMemsetAsync(ctx->filmsq64.p, 0, wh * 3 * sizeof(double), s));
+    }
+  }
   const bool count_work = ctx->count_work;
   for (int i = 0; i < ns; ++i) {
     CUDA_TRY(cudaMemsetAsync(wave_view(i).ray_stats, 0, 10 * sizeof(unsigned long long), s));

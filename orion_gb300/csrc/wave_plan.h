@@ -29,12 +29,13 @@ struct WavePlan {
 
 // `wave`: paths per wave (>= 1). exact: no wave is larger. Otherwise there are as few
 // waves as `wave` allows, and their last chunk may take one over it, by a sixteenth at
-// most; but never past INT32_MAX paths, which slots are numbered with.
+// most; but never past INT32_MAX paths, which slots are numbered with. No samples
+// (spp <= 0): no groups.
 inline WavePlan plan_waves(int64_t pixels, int spp, int64_t wave, bool exact) {
   WavePlan p;
   p.pixels = pixels;
-  p.groups = (spp + wave - 1) / wave;
-  p.passes = (int)((spp + p.groups - 1) / p.groups);
+  p.groups = spp > 0 ? (spp + wave - 1) / wave : 0;
+  p.passes = spp > 0 ? (int)((spp + p.groups - 1) / p.groups) : 1;
   const int64_t wave_pixels = std::max<int64_t>(1, wave / p.passes);
   p.chunk_log2 = 8;  // a chunk is at most a sixteenth of a wave's pixels
   while (p.chunk_log2 > 0 && (int64_t)16 << p.chunk_log2 > wave_pixels) --p.chunk_log2;

@@ -17,7 +17,8 @@ int main(int, char** argv) {
   if (p.capacity() < 1 || p.capacity() > INT32_MAX) return std::puts("capacity out of range"), 1;
   if (exact && p.capacity() > wave) return std::puts("larger than asked for"), 1;
   if (p.capacity() > wave + wave / 16) return std::puts("over by more than a sixteenth"), 1;
-  if ((int64_t)(p.groups - 1) * p.passes >= spp || (int64_t)p.groups * p.passes < spp)
+  if (p.passes < 1) return std::puts("no passes"), 1;
+  if (spp <= 0 ? p.groups != 0 : (int64_t)(p.groups - 1) * p.passes >= spp || (int64_t)p.groups * p.passes < spp)
     return std::puts("passes left out"), 1;
   int64_t sum = 0;
   for (int64_t k = 0; k < p.group_waves; ++k) {

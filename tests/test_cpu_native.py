@@ -50,3 +50,8 @@ INT32_MAX = 2**31 - 1
     (1024 * 1024, 64, 1 << 25, 0), (257, 1, 100, 0), (7 * 41, 257, 7 * 41 * 257, 0)])
 def test_waves_cover_the_film_within_their_capacity(native, pixels, spp, wave, exact):
     _run(native("wave_plan"), pixels, spp, wave, exact)
+
+
+@pytest.mark.parametrize("spp", [0, -3])
+def test_no_samples_make_no_waves(native, spp):
+    _run(native("wave_plan"), 64 * 48, spp, 1, 0)

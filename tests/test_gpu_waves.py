@@ -152,3 +152,26 @@ def test_batch_film_adds_every_run_of_samples(ctx, spp):
             assert np.allclose(a[0], b[0], rtol=1e-12, atol=1e-12)
     finally:
         ctx.release(sid)
+
+
+def test_a_render_of_no_samples_is_black(ctx):
+    """A scene of 0 samples a pixel renders to a film of zeros and no counts, whatever the context rendered
+    before."""
+    from orion_gb300 import scenegen
+    s = scenegen.zoo(subdiv=1, spp=2, max_depth=2)
+    s.width, s.height = 20, 12
+    some = ctx.upload(scenegen.to_host_scene(s))
+    s.spp = 0
+    none = ctx.upload(scenegen.to_host_scene(s))
+    try:
+        img, cnt = ctx.render(some, 20, 12)
+        assert img.any() and (cnt == 2).all()
+        ctx.render(some, 20, 12, fp64=True)
+        img, cnt = ctx.render(none, 20, 12)
+        assert not img.any() and not cnt.any()
+        for sums in ctx.render(none, 20, 12, fp64=True):
+            assert not sums.any()
+        assert ctx.last_stats()["paths"] == 0
+    finally:
+        ctx.release(some)
+        ctx.release(none)
