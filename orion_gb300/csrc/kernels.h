@@ -230,6 +230,24 @@ __device__ __forceinline__ long long slot_index(const WaveView& w, int pid) {
 }
 #endif
 
+// Pixel `pos` of a film in tile order: tiles of 8 x 4 pixels, tile row after
+// tile row, row by row within a tile (edge tiles are smaller). Films of more than
+// 2^28 pixels a row, where a tile row's pixels pass 32 bits: row by row.
+ORION_HD inline void tile_pixel(int64_t pos, int width, int height, int* x, int* y) {
+  if (width > 1 << 28) {
+    *y = (int)(pos / width);
+    *x = (int)(pos - (int64_t)*y * width);
+    return;
+  }
+  const uint32_t band_pixels = 4u * (uint32_t)width;
+  const int band = pos >> 32 ? (int)(pos / band_pixels) : (int)((uint32_t)pos / band_pixels), y0 = 4 * band;
+  const int left = height - y0, rows = left < 4 ? left : 4, in_band = (int)(pos - (int64_t)band * band_pixels);
+  const int tile = in_band / (8 * rows), x0 = 8 * tile, cols = width - x0 < 8 ? width - x0 : 8;
+  const int in_tile = in_band - 8 * rows * tile, row = in_tile / cols;
+  *x = x0 + in_tile - row * cols;
+  *y = y0 + row;
+}
+
 // A wave renders `passes` sample passes of some of the film's pixels. Its slots
 // hold pixel after pixel, and each pixel's passes in order: slot = local
 // pixel x passes + pass, so the rays of a warp leave through one pixel or a few

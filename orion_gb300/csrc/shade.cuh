@@ -43,18 +43,6 @@ __device__ __forceinline__ void class_append(int* counters, int* queues, int str
   queues[(size_t)cls * stride + base + __popc(peers & ((1u << lane) - 1u))] = value;
 }
 
-// Pixel `pos` of a film in tile order: tiles of 8 x 4 pixels, tile row after
-// tile row, row by row within a tile (edge tiles are smaller).
-__device__ __forceinline__ void tile_pixel(int64_t pos, int width, int height, int* x, int* y) {
-  const uint32_t band_pixels = 4u * (uint32_t)width;
-  const int band = pos >> 32 ? (int)(pos / band_pixels) : (int)((uint32_t)pos / band_pixels), y0 = 4 * band;
-  const int rows = min(4, height - y0), in_band = (int)(pos - (int64_t)band * band_pixels);
-  const int tile = in_band / (8 * rows), x0 = 8 * tile, cols = min(8, width - x0);
-  const int in_tile = in_band - 8 * rows * tile, row = in_tile / cols;
-  *x = x0 + in_tile - row * cols;
-  *y = y0 + row;
-}
-
 struct Hit {
   V3 p, ng, ns, su, sv;
 };

@@ -19,6 +19,8 @@ def native(tmp_path_factory):
 
     def compile_one(name, *sources):
         exe = str(out / name)
+        if os.path.exists(exe):
+            return exe
         subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-I", build.CSRC, "-I",
                         os.path.join(build.CUDA_HOME, "include"), os.path.join(NATIVE, name + ".cpp"),
                         *(os.path.join(build.CSRC, s) for s in sources), "-o", exe, "-lpthread", "-ldl"], check=True)
@@ -55,3 +57,11 @@ def test_waves_cover_the_film_within_their_capacity(native, pixels, spp, wave, e
 @pytest.mark.parametrize("spp", [0, -3])
 def test_no_samples_make_no_waves(native, spp):
     _run(native("wave_plan"), 64 * 48, spp, 1, 0)
+
+
+@pytest.mark.parametrize("width,height", [
+    (1, 1), (7, 3), (8, 4), (9, 5), (33, 6), (1, 97), (641, 359), (1 << 28, 3), ((1 << 28) + 1, 7), (1 << 29, 4),
+    (1 << 30, 1),  # a tile row of 2^32 pixels
+    (1 << 30, 4), (INT32_MAX, 1), (INT32_MAX, 9), (65536, 65536), (3, 1 << 29)])
+def test_tile_order_visits_each_pixel_once(native, width, height):
+    _run(native("tile_pixel"), width, height)
