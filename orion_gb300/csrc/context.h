@@ -105,6 +105,11 @@ struct DevBuf {
     release();
     if (n == 0) n = 16;
     cudaError_t e = cudaMallocFromPoolAsync(&p, n, pool, s);
+    if (e == cudaErrorMemoryAllocation) {  // as alloc: another context's pool may hold what is missing
+      cudaGetLastError();
+      trim_scene_pools();
+      e = cudaMallocFromPoolAsync(&p, n, pool, s);
+    }
     if (e != cudaSuccess) {
       p = nullptr;
       return fail(e == cudaErrorMemoryAllocation ? ORION_ERR_NOMEM : ORION_ERR_CUDA,

@@ -65,3 +65,8 @@ def test_no_samples_make_no_waves(native, spp):
     (1 << 30, 4), (INT32_MAX, 1), (INT32_MAX, 9), (65536, 65536), (3, 1 << 29)])
 def test_tile_order_visits_each_pixel_once(native, width, height):
     _run(native("tile_pixel"), width, height)
+
+
+@pytest.mark.parametrize("kind", ["plain", "pooled"])
+def test_allocations_out_of_memory_trim_the_pools_and_retry(native, kind):
+    _run(native("device_buffers"), kind, 1, "retried")
