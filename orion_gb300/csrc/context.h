@@ -94,6 +94,7 @@ struct DevBuf {
     }
     if (e != cudaSuccess) {
       p = nullptr;
+      cudaGetLastError();  // reported here, not by the next call
       return fail(e == cudaErrorMemoryAllocation ? ORION_ERR_NOMEM : ORION_ERR_CUDA,
                   std::string("cudaMalloc(") + std::to_string(n) + "): " + cudaGetErrorString(e));
     }
@@ -112,6 +113,7 @@ struct DevBuf {
     }
     if (e != cudaSuccess) {
       p = nullptr;
+      cudaGetLastError();  // reported here, not by the next call
       return fail(e == cudaErrorMemoryAllocation ? ORION_ERR_NOMEM : ORION_ERR_CUDA,
                   std::string("cudaMallocFromPoolAsync(") + std::to_string(n) + "): " + cudaGetErrorString(e));
     }

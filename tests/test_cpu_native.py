@@ -70,3 +70,9 @@ def test_tile_order_visits_each_pixel_once(native, width, height):
 @pytest.mark.parametrize("kind", ["plain", "pooled"])
 def test_allocations_out_of_memory_trim_the_pools_and_retry(native, kind):
     _run(native("device_buffers"), kind, 1, "retried")
+
+
+@pytest.mark.parametrize("kind", ["plain", "pooled"])
+def test_refused_allocations_leave_no_error_behind(native, kind):
+    """The autotuners skip a configuration that does not fit; the launches after it must not fail over it."""
+    _run(native("device_buffers"), kind, 2, "refused")
