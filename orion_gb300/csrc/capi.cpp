@@ -870,6 +870,7 @@ struct QueryBuffers {
   float *rays = nullptr, *t = nullptr, *u = nullptr, *v = nullptr;
   int* prim = nullptr;
   int load(orion_gpu_ctx* ctx, int64_t n, const float* host) {
+    if ((uint64_t)n > SIZE_MAX / 48) return fail(ORION_ERR_NOMEM, "a query of " + std::to_string(n) + " rays");
     const size_t bytes = 48 * (size_t)n;
     if (bytes <= ((size_t)64 << 20))
       RC(ws.alloc_pooled(bytes, ctx->scene_pool, ctx->stream));

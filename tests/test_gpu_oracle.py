@@ -199,6 +199,22 @@ def test_ray_queries_at_ragged_sizes(ctx, port, tmp_path, n):
     assert (t[prim >= 0] > rays[prim >= 0, 6]).all() and (t[prim >= 0] <= rays[prim >= 0, 7]).all()
 
 
+@pytest.mark.parametrize("n", [2**59, 2**60, 2**63 - 1])
+def test_ray_queries_beyond_any_memory_are_refused(ctx, tmp_path, n):
+    """Counts whose buffers' bytes wrap 64 bits: ORION_ERR_NOMEM before any device work."""
+    import ctypes
+    import orion_gb300 as og
+    host = og.HostScene.load(helpers.write_scene("cornell", str(tmp_path / "c"), res=32, spp=1))
+    sid = ctx.upload(host)
+    rays = np.zeros((1, 8), np.float32)
+    out = [np.zeros(1, np.float32) for _ in range(3)] + [np.zeros(1, np.int32)]
+    ptr = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+    for any_hit in (0, 1):
+        assert og.library().orion_gpu_trace(ctx._h, sid, n, ptr(rays), any_hit, *(ptr(a) for a in out)) == -5
+    assert (ctx.trace(sid, rays)[3] == -1).all()
+    ctx.release(sid)
+
+
 @pytest.mark.parametrize("name,kw", [
     ("caustics", dict(res=48, iterations=8, photons=20000, radius=0.08, max_depth=5)),
     ("envlit_sppm", dict(res=32, iterations=4, photons=10000, radius=0.08)),
