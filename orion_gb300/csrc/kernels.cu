@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(kQueryBlock, 8) k_trace_closest(SceneView s, i
     if (mine >= 0) lane_visit<false, kQueryStack, false, kMaxStack, true>(r, ts, st, nullptr);
     warp_triangles<false, false, true, true>(r, ts, tsc, nullptr);
     if (mine >= 0 && lane_pop(r, st)) {
-      const bool hit = r.tri >= 0 && !(r.tmax < 0.f);  // a hit behind the origin (tnear < 0) counts as a miss
+      const bool hit = r.tri >= 0;  // no test by the sign of tmax: hits behind the origin (tnear < 0) count
       t[mine] = hit ? r.tmax : 0.f;
       u[mine] = r.u;
       v[mine] = r.v;

@@ -199,6 +199,34 @@ def test_ray_queries_at_ragged_sizes(ctx, port, tmp_path, n):
     assert (t[prim >= 0] > rays[prim >= 0, 6]).all() and (t[prim >= 0] <= rays[prim >= 0, 7]).all()
 
 
+@pytest.mark.parametrize("n", [63, 8193, 100001])
+def test_ray_queries_that_begin_behind_the_origin(ctx, port, tmp_path, n):
+    """Negative near bounds (three rays of four, among others whose hits all lie ahead), some with negative far
+    bounds too: the least t in (tnear, tfar], as the oracle finds it, and the same rays hit something in
+    orion_gpu_trace's any-hit form; edge rays (10 per million, one at least) excepted."""
+    import orion_gb300 as og
+    host = og.HostScene.load(helpers.write_scene("zoo", str(tmp_path / "zoo"), res=32, spp=1))
+    lo, hi = _bounds(host)
+    size = float(np.max(hi - lo))
+    rays = helpers.random_rays(n, lo, hi, seed=41)
+    behind = np.arange(n) % 4 != 0
+    rays[behind, 6] = (-helpers.splitmix_uniform(n, 42) * size)[behind].astype(np.float32)
+    rays[:, 7] = rays[:, 6] + (helpers.splitmix_uniform(n, 43) * size).astype(np.float32)
+    sid = ctx.upload(host)
+    t, _, _, prim = ctx.trace(sid, rays)
+    _, _, _, occ = ctx.trace(sid, rays, any_hit=True)
+    ctx.release(sid)
+    rt, _, _, rprim = port.Scene(host).trace(rays)
+    edge = max(1, int(n * 1e-5))
+    assert n < 100 or np.count_nonzero((rprim >= 0) & (rt < 0)) > n // 10
+    assert np.count_nonzero((prim >= 0) != (rprim >= 0)) <= edge
+    assert np.count_nonzero((occ >= 0) != (rprim >= 0)) <= edge
+    both = (prim >= 0) & (rprim >= 0)
+    tol = helpers.t_tolerance(rays, rt, rprim, host.arrays()["positions"])
+    assert np.count_nonzero(both & ~(np.abs(t.astype(np.float64) - rt) <= tol)) <= edge
+    assert (t[prim >= 0] > rays[prim >= 0, 6]).all() and (t[prim >= 0] <= rays[prim >= 0, 7]).all()
+
+
 @pytest.mark.parametrize("n", [2**59, 2**60, 2**63 - 1])
 def test_ray_queries_beyond_any_memory_are_refused(ctx, tmp_path, n):
     """Counts whose buffers' bytes wrap 64 bits: ORION_ERR_NOMEM before any device work."""
