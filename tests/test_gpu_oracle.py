@@ -296,23 +296,32 @@ def test_sppm_at_ragged_sizes(ctx, port, width, height, iterations, photons, rad
     assert np.sqrt(np.mean((gpu - ref) ** 2)) <= 0.01 * np.sqrt(np.mean(ref ** 2))
 
 
-@pytest.mark.parametrize("width,height,photons", [(2, 2, 300_000), (4, 3, 500_000)])
-def test_sppm_hash_cells_of_many_hits(ctx, port, width, height, photons):
+@pytest.mark.parametrize("width,height", [(3, 3), (4, 3)])
+def test_sppm_hash_cells_of_many_hits(ctx, port, width, height):
     """A film of few pixels has as few hash cells, so each holds far more photon hits than the gather adds up
-    together (2^14) and turns up many times in one sphere: cells one by one, the image within 1% RMSE as above
-    (thousands of photons a pixel)."""
+    together (2^14; about 50,000 here) and turns up many times in one sphere: cells one by one, the image
+    within 1% RMSE as above (thousands of photons a pixel). How often a photon counts hangs on which cells a
+    sphere reaches, and films this small easily have one that ends at a cell's edge: the oracle's own film
+    must not hang on the last bits of the camera."""
     from orion_gb300 import scenegen
-    s = scenegen.caustics(64, subdiv=2)
-    s.width, s.height = width, height
-    host = scenegen.to_host_scene(s)
-    kw = dict(iterations=1, photons=photons, radius=0.4, max_depth=5)
-    ref, _ = port.Scene(host).render_sppm(**kw)
-    sid = ctx.upload(host)
+
+    def scene(shift=(0.0, 0.0, 0.0)):
+        s = scenegen.caustics(64, subdiv=2)
+        s.width, s.height = width, height
+        s.eye = tuple(e + d for e, d in zip((0.113, 0.071, 3.437), shift))
+        return scenegen.to_host_scene(s)
+
+    kw = dict(iterations=1, photons=500_000, radius=0.37, max_depth=5)
+    rms = lambda a: np.sqrt(np.mean(a ** 2))
+    ref = port.Scene(scene()).render_sppm(**kw)[0].astype(np.float64)
+    for axis in range(3):
+        moved, _ = port.Scene(scene([1e-5 * (axis == k) for k in range(3)])).render_sppm(**kw)
+        assert rms(moved - ref) < 1e-3 * rms(ref)
+    sid = ctx.upload(scene())
     gpu, cnt = ctx.render_sppm(sid, width, height, **kw)
     ctx.release(sid)
     assert (cnt == 1).all() and np.isfinite(gpu).all()
-    ref = ref.astype(np.float64).reshape(gpu.shape)
-    assert np.sqrt(np.mean((gpu - ref) ** 2)) <= 0.01 * np.sqrt(np.mean(ref ** 2))
+    assert rms(gpu - ref.reshape(gpu.shape)) <= 0.01 * rms(ref)
 
 
 def test_sppm_parameters_and_errors(ctx, tmp_path):
