@@ -325,7 +325,8 @@ typedef struct orion_launch_config {
 
 /* How orion_gpu_render_batch (and the server) run a batch:
  * ORION_BATCH_WAVES (default): the jobs' concatenated work list in waves of
- *   batch_slots paths, each launched for as many bounces as the deepest job has;
+ *   batch_slots paths, each launched for as many bounces as its own deepest job
+ *   has, or (beyond depth 16) until none of its paths is left;
  * ORION_BATCH_POOLED: a pool of batch_slots path slots refilled from the
  *   work list every bounce. */
 enum { ORION_BATCH_POOLED = 0, ORION_BATCH_WAVES = 1 };

@@ -562,73 +562,85 @@ void launch_batch_iteration(const WaveView& w, const BatchView& b, const uint32_
   enqueue_iteration(w, b, sobol, cfg, class_mask, cudaGraphConditionalHandle{}, 0, stream, timer);
 }
 
-void launch_batch_wave(const WaveView& w, const BatchView& b, const uint32_t* sobol, const LaunchConfig& cfg,
-                       unsigned class_mask, unsigned long long base, int n, int bounces, bool complete,
-                       cudaStream_t stream, int64_t* launches, StageTimer* timer) {
-  const WaveView bw = batch_view(w, b);
-  const bool append = n <= kAppendPaths;
-  const int persistent = cfg.num_sms * cfg.blocks_per_sm;
-  const int tgrid = grid_cap(n, cfg.trace_block, persistent);
-  const int sgrid = grid_cap(n, cfg.shade_block, persistent * 2);
-  const int cgrid = grid_cap(n, kCompactSpan, cfg.num_sms * 8);
-  int64_t nl = 0;
-  auto timed = [&](int st, auto&& launch) {
-    if (timer) timer->begin(st, stream);
-    nl += launch();
-    if (timer) timer->end(stream);
-  };
-  timed(ST_CAMERA, [&] {
-    k_wb_camera<<<grid_cap(n, 256, cfg.num_sms * 32), 256, 0, stream>>>(bw, b, sobol, base, n);
+namespace {
+
+// launch() on the wave's stream, counted (it returns how many) and timed as `stage`.
+template <class F>
+void staged(const BatchWave& v, int stage, F&& launch) {
+  if (v.timer) v.timer->begin(stage, v.stream);
+  const int n = launch();
+  if (v.timer) v.timer->end(v.stream);
+  if (v.launches) *v.launches += n;
+}
+
+}  // namespace
+
+void launch_batch_wave_begin(const BatchWave& v) {
+  staged(v, ST_CAMERA, [&] {
+    k_wb_camera<<<grid_cap(v.n, 256, v.cfg.num_sms * 32), 256, 0, v.stream>>>(batch_view(v.w, v.b), v.b, v.sobol, v.base, v.n);
     return 1;
   });
-  int cur = 0;
-  for (int bounce = 0; bounce < bounces; ++bounce, cur ^= 1) {
-    if (!timer) {
-      b_trace(cfg, bw, b, bounce > 0 ? TK_ALL : TK_EXT, cur, tgrid, !append, bounce == 0, stream);
-      ++nl;
+}
+
+void launch_batch_wave_bounces(const BatchWave& v, int from, int to, int all) {
+  const WaveView bw = batch_view(v.w, v.b);
+  const bool append = v.n <= kAppendPaths;
+  const int persistent = v.cfg.num_sms * v.cfg.blocks_per_sm;
+  const int tgrid = grid_cap(v.n, v.cfg.trace_block, persistent);
+  const int sgrid = grid_cap(v.n, v.cfg.shade_block, persistent * 2);
+  const int cgrid = grid_cap(v.n, kCompactSpan, v.cfg.num_sms * 8);
+  auto trace = [&](int stage, int kinds, int bounce) {
+    staged(v, stage, [&] {
+      b_trace(v.cfg, bw, v.b, kinds, bounce & 1, tgrid, !append, bounce == 0, v.stream);
+      return 1;
+    });
+  };
+  for (int bounce = from; bounce < to; ++bounce) {
+    const int cur = bounce & 1;
+    if (!v.timer) {
+      trace(ST_TRACE_EXT, bounce > 0 ? TK_ALL : TK_EXT, bounce);
     } else {  // timed: kind by kind
-      const int stage[3] = {ST_TRACE_EXT, ST_TRACE_SHADOW, ST_TRACE_MIS};
-      const int kinds[3] = {TK_EXT, TK_SHADOW, TK_MIS | TK_MIS_ENV};
-      for (int k = 0; k < (bounce > 0 ? 3 : 1); ++k)
-        timed(stage[k], [&] {
-          b_trace(cfg, bw, b, kinds[k], cur, tgrid, !append, bounce == 0, stream);
-          return 1;
-        });
+      trace(ST_TRACE_EXT, TK_EXT, bounce);
+      if (bounce > 0) trace(ST_TRACE_SHADOW, TK_SHADOW, bounce);
+      if (bounce > 0) trace(ST_TRACE_MIS, TK_MIS | TK_MIS_ENV, bounce);
     }
     if (bounce > 0)
-      timed(ST_RESOLVE, [&] {
-        k_b_resolve<<<sgrid, cfg.shade_block, 0, stream>>>(bw, b, cur);
+      staged(v, ST_RESOLVE, [&] {
+        k_b_resolve<<<sgrid, v.cfg.shade_block, 0, v.stream>>>(bw, v.b, cur);
         return 1;
       });
     const int* list = bounce == 0 ? nullptr : bw.q_ext[cur];  // the slots traced this bounce
     const int* count = bw.counters + cnt_rays(RK_EXT, cur);
     if (!append)
-      timed(ST_OTHER, [&] {
+      staged(v, ST_OTHER, [&] {
         CompactTargets tg{};
         for (int c = 0; c < kShadeClasses; ++c)
           tg.queue[c] = bw.q_cls + (size_t)c * bw.capacity, tg.counter[c] = bw.counters + cnt_cls(c, cur);
-        k_wb_compact<kShadeClasses><<<cgrid, kCompactThreads, 0, stream>>>(bw.qflags, list, count, tg);
+        k_wb_compact<kShadeClasses><<<cgrid, kCompactThreads, 0, v.stream>>>(bw.qflags, list, count, tg);
         return 1;
       });
-    timed(ST_SHADE, [&] {
-      return launch_wb_shading(bw, b, sobol, class_mask, cur, append, n, cfg, stream);
+    staged(v, ST_SHADE, [&] {
+      return launch_wb_shading(bw, v.b, v.sobol, v.class_mask, cur, append, v.n, v.cfg, v.stream);
     });
-    if (!append && !(complete && bounce + 1 == bounces))  // no path goes on after the last bounce
-      timed(ST_OTHER, [&] {
+    if (!append && bounce + 1 < all)  // no path goes on after the last bounce
+      staged(v, ST_OTHER, [&] {
         CompactTargets tg{};
         int* qs[5] = {bw.q_ext[cur ^ 1], bw.q_mis, bw.q_sh, bw.q_mis_env, bw.q_nee};  // as the QueueFlag bits
         for (int k = 0; k < 5; ++k)
           tg.queue[k] = qs[k],
           tg.counter[k] = bw.counters + (k < kRayKinds ? cnt_rays(k, cur ^ 1) : CNT_NEE + (cur ^ 1));
-        k_wb_compact<5><<<cgrid, kCompactThreads, 0, stream>>>(bw.qflags, list, count, tg);
+        k_wb_compact<5><<<cgrid, kCompactThreads, 0, v.stream>>>(bw.qflags, list, count, tg);
         return 1;
       });
   }
-  timed(ST_FILM, [&] {
-    k_wb_film<<<grid_cap(n, kWbFilmThreads, cfg.num_sms * 8), kWbFilmThreads, 0, stream>>>(bw, b, base, n, complete ? -1 : cur);
+}
+
+void launch_batch_wave_film(const BatchWave& v, int unfinished) {
+  staged(v, ST_FILM, [&] {
+    k_wb_film<<<grid_cap(v.n, kWbFilmThreads, v.cfg.num_sms * 8), kWbFilmThreads, 0, v.stream>>>(
+        batch_view(v.w, v.b), v.b, v.base, v.n, unfinished < 0 ? -1 : unfinished & 1);
     return 1;
   });
-  if (launches) *launches += nl;
 }
 
 // FP64 film sums rounded to FP32 (orion_job.sum32).

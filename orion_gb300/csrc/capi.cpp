@@ -238,6 +238,8 @@ extern "C" int orion_gpu_create(const orion_gpu_opts* opts, orion_gpu_ctx** out)
   CUDA_TRY(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
   for (cudaEvent_t& e : c->ev_join) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   for (cudaEvent_t& e : c->ev_film) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&c->batch_counters),
+                         2 * orion_gpu_ctx::kBatchEngines * kCounterSlots * sizeof(int), cudaHostAllocDefault));
   size_t free_b = 0, total_b = 0;
   CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
   c->budget = (opts && opts->memory_budget > 0) ? opts->memory_budget : (int64_t)(free_b * 0.9);
@@ -297,6 +299,7 @@ extern "C" int orion_gpu_destroy(orion_gpu_ctx* ctx) {
     if (e) cudaEventDestroy(e);
   for (cudaEvent_t e : ctx->ev_film)
     if (e) cudaEventDestroy(e);
+  cudaFreeHost(ctx->batch_counters);
   for (cudaStream_t x : ctx->xstream)
     if (x) cudaStreamDestroy(x);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);

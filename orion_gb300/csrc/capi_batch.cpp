@@ -293,13 +293,18 @@ static int run_batch_waves_locked(orion_gpu_ctx* ctx, std::vector<DevJob>& dj, u
     CUDA_TRY(cudaMemcpyAsync(bvs[e].jobs, dj.data(), (size_t)njobs * sizeof(DevJob), cudaMemcpyHostToDevice, es));
     CUDA_TRY(cudaMemcpyAsync(bvs[e].ctl, &zero, sizeof(BatchCtl), cudaMemcpyHostToDevice, es));
   }
-  // Bounces 0 .. the deepest job's depth end every path (the test limit cuts waves short).
-  const int all_bounces = max_depth_all + 1;
-  const int bounces =
-      ctx->cfg.test_batch_iterations > 0 ? std::min(ctx->cfg.test_batch_iterations, all_bounces) : all_bounces;
+  // Bounces that end every path of the work items [base, base + n): one more than
+  // the deepest depth among their own jobs.
+  auto bounces_of = [&](unsigned long long base, int n) {
+    int deepest = 0;
+    for (const DevJob& J : dj)
+      if ((unsigned long long)J.work_begin < base + n && (unsigned long long)(J.work_begin + J.num_paths) > base)
+        deepest = std::max(deepest, J.max_depth);
+    return deepest + 1;
+  };
   StageTimer timer{nullptr, nullptr, 0, 0};
   if (ctx->profiling) {
-    const int need = (int)std::min<int64_t>(nwaves * (bounces + 1) * 8, 200000);
+    const int need = (int)std::min<int64_t>(nwaves * (max_depth_all + 2) * 8, 200000);
     while ((int)ctx->prof_events.size() < 2 * need) {
       cudaEvent_t e;
       CUDA_TRY(cudaEventCreate(&e));
@@ -308,17 +313,76 @@ static int run_batch_waves_locked(orion_gpu_ctx* ctx, std::vector<DevJob>& dj, u
     ctx->prof_stage.resize(need);
     timer = StageTimer{ctx->prof_events.data(), ctx->prof_stage.data(), need, 0};
   }
-  int64_t launches = 0;
-  for (int64_t k = 0; k < nwaves; ++k) {
+  // A wave's first bounces are launched at once. Deeper ones (roulette ends most
+  // paths long before) follow a few at a time, and no more once the counters of
+  // the stretch before last show that nothing was left: a stretch is always
+  // queued ahead of the one whose counters the host waits for, and the engines'
+  // waves advance in turn, so the device does not wait for the host.
+  constexpr int kUncheckedBounces = 17, kCheckedBounces = 8;
+  struct OpenWave {
+    int64_t k = -1;  // none
+    int done;        // bounces launched
+    int all, limit;  // those that end every path; those to launch at most (the test limit cuts waves short)
+    int stretch;     // its counters go to half stretch & 1 of the engine's batch_counters
+  };
+  std::vector<OpenWave> open(ne);
+  int64_t launches = 0, iterations = 0;
+  auto wave_of = [&](int64_t k) {
     const int e = (int)(k % ne);
-    cudaStream_t es = engine_stream(ctx, e);
-    const WaveView& wv = engine_wave(ctx, e).view;
     const unsigned long long base = (unsigned long long)(k * wave);
-    const int n = (int)std::min<unsigned long long>((unsigned long long)wave, total - base);
-    launch_batch_wave(wv, bvs[e], ctx->sobol.as<uint32_t>(), ctx->cfg, mask, base, n, bounces, bounces == all_bounces, es,
-                      &launches, ctx->profiling ? &timer : nullptr);
+    return BatchWave{engine_wave(ctx, e).view, bvs[e], ctx->sobol.as<uint32_t>(), ctx->cfg, mask, base,
+                     (int)std::min<unsigned long long>((unsigned long long)wave, total - base), engine_stream(ctx, e),
+                     &launches, ctx->profiling ? &timer : nullptr};
+  };
+  auto snapshot = [&](const OpenWave& o) { return 2 * (int)(o.k % ne) + (o.stretch & 1); };
+  // Queues the bounces up to `to` and a copy of the counters they leave.
+  auto stretch = [&](OpenWave& o, const BatchWave& w, int to) -> int {
+    launch_batch_wave_bounces(w, o.done, to, o.all);
+    o.done = to;
+    ++o.stretch;
+    if (to < o.limit) {
+      CUDA_TRY(cudaMemcpyAsync(ctx->batch_counters + kCounterSlots * snapshot(o), w.b.ctl->counters,
+                               kCounterSlots * sizeof(int), cudaMemcpyDeviceToHost, w.stream));
+      CUDA_TRY(cudaEventRecord(ctx->ev_film[snapshot(o)], w.stream));
+    }
+    return ORION_OK;
+  };
+  auto close = [&](OpenWave& o, const BatchWave& w) -> int {
+    launch_batch_wave_film(w, o.done < o.all ? o.done : -1);
     CUDA_TRY(cudaGetLastError());
+    iterations += o.done;
+    o.k = -1;
+    return ORION_OK;
+  };
+  auto advance = [&](OpenWave& o) -> int {
+    const BatchWave w = wave_of(o.k);
+    const int at = snapshot(o), parity = o.done & 1;
+    RC(stretch(o, w, std::min(o.limit, o.done + kCheckedBounces)));
+    CUDA_TRY(cudaEventSynchronize(ctx->ev_film[at]));
+    const int* c = ctx->batch_counters + kCounterSlots * at;
+    // Paths that ended may still have had a light sample to trace and add.
+    const bool left = c[cnt_rays(RK_EXT, parity)] > 0 || c[CNT_NEE + parity] > 0;
+    return left && o.done < o.limit ? ORION_OK : close(o, w);
+  };
+  auto advance_all = [&]() -> int {
+    for (OpenWave& o : open)
+      if (o.k >= 0) RC(advance(o));
+    return ORION_OK;
+  };
+  for (int64_t k = 0; k < nwaves; ++k) {
+    OpenWave& o = open[k % ne];
+    while (o.k >= 0) RC(advance_all());
+    const BatchWave w = wave_of(k);
+    o.k = k;
+    o.done = o.stretch = 0;
+    o.all = bounces_of(w.base, w.n);
+    o.limit = ctx->cfg.test_batch_iterations > 0 ? std::min(ctx->cfg.test_batch_iterations, o.all) : o.all;
+    launch_batch_wave_begin(w);
+    RC(stretch(o, w, std::min(o.limit, kUncheckedBounces)));
+    if (o.done == o.limit) RC(close(o, w));
   }
+  for (OpenWave& o : open)
+    while (o.k >= 0) RC(advance_all());
   for (int e = 1; e < ne; ++e) {
     CUDA_TRY(cudaEventRecord(ctx->ev_join[e - 1], engine_stream(ctx, e)));
     CUDA_TRY(cudaStreamWaitEvent(s, ctx->ev_join[e - 1], 0));
@@ -348,7 +412,7 @@ static int run_batch_waves_locked(orion_gpu_ctx* ctx, std::vector<DevJob>& dj, u
     }
     error_bits |= o.error;
   }
-  out.iterations = (int)std::min<int64_t>(nwaves * bounces, INT32_MAX);
+  out.iterations = (int)std::min<int64_t>(iterations, INT32_MAX);
   out.error = error_bits;
   ctx->last.paths = (int64_t)out.paths_done;
   ctx->last.ext_rays = (int64_t)out.rays[0];

@@ -192,7 +192,8 @@ struct orion_gpu_ctx {
   Wave wave;
   // Plain renders overlap consecutive waves on up to kWaveStreams streams:
   // per extra stream its wave state, the stream, its join event; the events
-  // that order the film writes of waves with other passes of the same pixels.
+  // that order the film writes of waves with other passes of the same pixels
+  // (batches: batch_counters).
   static constexpr int kWaveStreams = orion_gb300::kMaxWaveStreams;
   // Four: the eight-sphere 1080p render (eight waves) 2583 -> 2822 Mpaths/s
   // against two. Renders of fewer than two full waves are split two ways
@@ -231,6 +232,10 @@ struct orion_gpu_ctx {
   // engine e on the wave state and stream of wave slot e.
   static constexpr int kBatchEngines = 2;
   BatchEngine beng[kBatchEngines];
+  // Pinned copies of the engines' queue counters (wave mode's deep waves): two per
+  // engine, each behind the event of the same number in ev_film.
+  int* batch_counters = nullptr;
+  static_assert(2 * kBatchEngines <= kWaveStreams, "an event per copy");
   int batch_mode = ORION_BATCH_WAVES;
   // SPPM: per-pixel state in one block, the grid's cell lists apart
   DevBuf sppm_block, sppm_hits;

@@ -372,13 +372,26 @@ cudaError_t capture_batch_iteration(const WaveView& w, const BatchView& b, const
 // each stage timed by `timer`: the profiling path of the pooled engine.
 void launch_batch_iteration(const WaveView& w, const BatchView& b, const uint32_t* sobol, const LaunchConfig& cfg,
                             unsigned class_mask, cudaStream_t stream, StageTimer* timer);
-// Wave mode: renders the work items [base, base + n) on slots 0..n-1, a plain
-// wave's launches with `bounces` bounces, and adds the radiance of the n paths
-// to their jobs' films. complete: `bounces` is one more than the deepest job's
-// depth, which ends every path (else paths left report kErrIterationCap).
-void launch_batch_wave(const WaveView& w, const BatchView& b, const uint32_t* sobol, const LaunchConfig& cfg,
-                       unsigned class_mask, unsigned long long base, int n, int bounces, bool complete,
-                       cudaStream_t stream, int64_t* launches, StageTimer* timer);
+// Wave mode: the work items [base, base + n) on slots 0..n-1, a plain wave's launches.
+// _begin starts the paths; _bounces runs the bounces [from, to), every path's last one at
+// the latest `all` - 1 (one more than the depth of the deepest job among them); _film adds
+// the radiance of the n paths to their jobs' films (unfinished: -1, or the number of bounces
+// run if some paths may be left, which are then reported as kErrIterationCap).
+struct BatchWave {
+  const WaveView& w;
+  const BatchView& b;
+  const uint32_t* sobol;
+  const LaunchConfig& cfg;
+  unsigned class_mask;
+  unsigned long long base;
+  int n;
+  cudaStream_t stream;
+  int64_t* launches;   // added to
+  StageTimer* timer;   // or null
+};
+void launch_batch_wave_begin(const BatchWave& wave);
+void launch_batch_wave_bounces(const BatchWave& wave, int from, int to, int all);
+void launch_batch_wave_film(const BatchWave& wave, int unfinished);
 // dst[i] = (float)src[i] for i < n.
 void launch_film_to_f32(const double* src, float* dst, long long n, int num_sms, cudaStream_t stream);
 // Resets the batch control block and the free-slot list for `capacity` slots.

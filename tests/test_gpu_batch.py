@@ -187,3 +187,63 @@ def test_batch_fp32_readback(ctx, scenes, mode):
     for (a, _, ca), (b, q, cb) in zip(f64, f32):
         assert b.dtype == np.float32 and q is None
         assert np.all(np.abs(a - b) <= 2.0 ** -23 * np.abs(a) + 1e-30) and np.array_equal(ca, cb)
+
+
+def test_waves_run_the_bounces_of_their_own_jobs(ctx):
+    """Wave mode launches each wave for the bounces of the jobs in it (one wave per job here), deep waves only
+    while paths are left: counted in the batch's iterations. Films as the plain render's."""
+    from orion_gb300 import scenegen
+    s = scenegen.zoo(subdiv=1)
+    s.width = s.height = 32
+    sid = ctx.upload(scenegen.to_host_scene(s))
+    cfg = ctx.get_config()
+    depths = [4, 0, 2, 16, 120, 1, 4]
+    jobs = [dict(sid=sid, width=32, height=32, spp=8, max_depth=d, first_pass=8 * i) for i, d in enumerate(depths)]
+    want = [ctx.render(sid, 32, 32, spp=8, max_depth=j["max_depth"], first_pass=j["first_pass"], fp64=True)
+            for j in jobs]
+
+    def check(outs, which):
+        for (got, sq, count), i in zip(outs, which):
+            assert (count == 8).all()
+            assert np.allclose(got, want[i][0], rtol=1e-5, atol=1e-7), depths[i]
+            assert np.allclose(sq, want[i][1], rtol=1e-5, atol=1e-7), depths[i]
+
+    shallow = [i for i, d in enumerate(depths) if d <= 16]
+    try:
+        ctx.set_config(batch_slots=32 * 32 * 8)
+        outs, st = ctx.render_batch([jobs[i] for i in shallow])
+        check(outs, shallow)
+        expect = sum(depths[i] + 1 for i in shallow)
+        assert st["iterations"] == expect
+        outs, st = ctx.render_batch(jobs)
+        check(outs, range(len(jobs)))
+        assert expect + 17 <= st["iterations"] < expect + 121  # roulette leaves no path for 120 bounces
+        for slots in (5000, 1 << 24):  # waves across jobs; all in one
+            ctx.set_config(batch_slots=slots)
+            check(ctx.render_batch(jobs)[0], range(len(jobs)))
+    finally:
+        ctx.set_config(**cfg)
+        ctx.release(sid)
+
+
+def test_deep_waves_report_paths_that_a_limit_leaves(ctx):
+    """Without roulette some paths of a Cornell box live past 20 bounces: a batch stopped there is reported,
+    and one that runs to its depth is not."""
+    import orion_gb300 as og
+    from orion_gb300 import scenegen
+    s = scenegen.cornell(subdiv=1)
+    s.width = s.height = 32
+    sid = ctx.upload(scenegen.to_host_scene(s))
+    jobs = [dict(sid=sid, width=32, height=32, spp=8, max_depth=40, rr_depth=1000)]
+    try:
+        for limit in (17, 18, 20):
+            ctx.set_test_limits(batch_iterations=limit)
+            with pytest.raises(og.OrionError, match="iteration cap"):
+                ctx.render_batch(jobs)
+        ctx.set_test_limits()
+        (got, _, _), = ctx.render_batch(jobs)[0]
+        want, _ = ctx.render(sid, 32, 32, spp=8, max_depth=40, rr_depth=1000, fp64=True)
+        assert np.allclose(got, want, rtol=1e-5, atol=1e-7)
+    finally:
+        ctx.set_test_limits()
+        ctx.release(sid)
