@@ -168,7 +168,8 @@ struct Builder {
     queue.push_back(Task{0, count, 0, &root});
     unfinished = 1;
     std::vector<std::thread> th;
-    for (int t = 1; t < n; ++t) th.emplace_back([this, t] { work(arenas[t]); });
+    th.reserve(n);
+    for (int t = 1; t < n && start_thread(th, [this, t] { work(arenas[t]); });) ++t;
     work(arenas[0]);
     for (std::thread& x : th) x.join();
     return root;

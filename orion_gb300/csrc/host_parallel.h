@@ -4,23 +4,35 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <system_error>
 #include <thread>
+#include <utility>
 #include <vector>
 
 namespace orion_gb300 {
 
+// Starts f on a thread of its own, added to `th` (with room for it); false if the
+// system gives no more threads.
+template <class F>
+bool start_thread(std::vector<std::thread>& th, F&& f) {
+  try {
+    th.emplace_back(std::forward<F>(f));
+    return true;
+  } catch (const std::system_error&) {
+    return false;
+  }
+}
+
 // f(begin, end, part) over `parts` contiguous pieces of [begin, end); the
-// caller's thread takes the last one.
+// caller's thread takes the last one, and those that get no thread.
 template <class F>
 void parallel_parts(int64_t begin, int64_t end, int parts, const F& f) {
   const int64_t n = end - begin;
   std::vector<std::thread> th;
+  th.reserve(parts);
   for (int t = 0; t < parts; ++t) {
     const int64_t b = begin + n * t / parts, e = begin + n * (t + 1) / parts;
-    if (t + 1 < parts)
-      th.emplace_back([&f, b, e, t] { f(b, e, t); });
-    else
-      f(b, e, t);
+    if (t + 1 == parts || !start_thread(th, [&f, b, e, t] { f(b, e, t); })) f(b, e, t);
   }
   for (std::thread& x : th) x.join();
 }

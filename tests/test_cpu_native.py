@@ -76,3 +76,9 @@ def test_allocations_out_of_memory_trim_the_pools_and_retry(native, kind):
 def test_refused_allocations_leave_no_error_behind(native, kind):
     """The autotuners skip a configuration that does not fit; the launches after it must not fail over it."""
     _run(native("device_buffers"), kind, 2, "refused")
+
+
+@pytest.mark.parametrize("triangles,threads", [(2000, 0), (5000, 0), (5000, 2), (100_000, 0), (100_000, 3)])
+def test_bvh_build_does_without_threads(native, triangles, threads):
+    """A process at its thread limit builds the same tree on the threads it has."""
+    _run(native("bvh_threads", "bvh_build.cpp"), "threads", triangles, threads)
