@@ -157,6 +157,7 @@ struct Builder {
   std::condition_variable wake;
   std::deque<Task> queue;
   int unfinished = 0;  // tasks queued or being built
+  FirstError error;    // a subtree that failed is given up; the others are built to the end
 
   Builder(const BvhBuildOptions& o, PrimRef* r, int nthreads) : opt(o), refs(r), threads(nthreads) {}
 
@@ -172,6 +173,7 @@ struct Builder {
     for (int t = 1; t < n && start_thread(th, [this, t] { work(arenas[t]); });) ++t;
     work(arenas[0]);
     for (std::thread& x : th) x.join();
+    error.rethrow();
     return root;
   }
 
@@ -183,7 +185,7 @@ struct Builder {
       const Task t = queue.front();
       queue.pop_front();
       g.unlock();
-      *t.slot = build(t.begin, t.end, t.depth, arena);
+      error.guard([&] { *t.slot = build(t.begin, t.end, t.depth, arena); });
       g.lock();
       if (--unfinished == 0) wake.notify_all();
     }

@@ -14,6 +14,7 @@
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -330,7 +331,7 @@ extern "C" int orion_gpu_scene_upload(orion_gpu_ctx* ctx, const orion_host_scene
   CUDA_TRY(cudaSetDevice(ctx->device));
   const HostScene& hs = scene->s;
   orion_host_scene* hsm = const_cast<orion_host_scene*>(scene);
-  {
+  try {
     std::lock_guard<std::mutex> sg(hsm->mu);
     if (!hsm->prep) {
       std::unique_ptr<PreparedScene> ps(new PreparedScene());
@@ -365,6 +366,8 @@ extern "C" int orion_gpu_scene_upload(orion_gpu_ctx* ctx, const orion_host_scene
       pin(hsm, hsm->tri_class);
       pin(hsm, hsm->prep->prims);
     }
+  } catch (const std::bad_alloc&) {
+    return fail(ORION_ERR_NOMEM, "out of host memory preparing the scene");
   }
   const PreparedScene& ps = *hsm->prep;
   const BvhBuild& bvh = *hsm->bvh;

@@ -82,3 +82,9 @@ def test_refused_allocations_leave_no_error_behind(native, kind):
 def test_bvh_build_does_without_threads(native, triangles, threads):
     """A process at its thread limit builds the same tree on the threads it has."""
     _run(native("bvh_threads", "bvh_build.cpp"), "threads", triangles, threads)
+
+
+@pytest.mark.parametrize("triangles", [5000, 100_000])
+def test_bvh_build_hands_a_threads_exception_on(native, triangles):
+    """Out of memory on a worker thread: the caller gets the exception, once, and can build again."""
+    _run(native("bvh_threads", "bvh_build.cpp"), "memory", triangles)
