@@ -343,8 +343,9 @@ struct Builder {
     V4 cl = box.clo, scale = splat(0.f);
     cl[3] = 0.f;
     for (int axis = 0; axis < 3; ++axis) {
-      float ext = box.chi[axis] - box.clo[axis];
-      scale[axis] = ext > 0.f ? B / ext : 0.f;
+      // An axis along which the centres lie too close for B / ext is not split.
+      const float ext = box.chi[axis] - box.clo[axis], s = B / ext;
+      scale[axis] = ext > 0.f && s <= std::numeric_limits<float>::max() ? s : 0.f;
     }
     Bins all;
     const int parts = scan_parts(end - begin);

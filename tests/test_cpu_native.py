@@ -5,6 +5,7 @@ from __future__ import annotations
 import os
 import subprocess
 
+import numpy as np
 import pytest
 
 from orion_gb300 import build
@@ -88,3 +89,28 @@ def test_bvh_build_does_without_threads(native, triangles, threads):
 def test_bvh_build_hands_a_threads_exception_on(native, triangles):
     """Out of memory on a worker thread: the caller gets the exception, once, and can build again."""
     _run(native("bvh_threads", "bvh_build.cpp"), "memory", triangles)
+
+
+def _soup(n, seed=5):
+    """n small triangles in the unit cube (n x 3 x 3)."""
+    g = np.random.RandomState(seed)
+    return g.uniform(size=(n, 1, 3)) + 0.01 * g.uniform(size=(n, 3, 3))
+
+
+def _bvh_of(native, tmp_path, positions):
+    path = str(tmp_path / "positions.bin")
+    with np.errstate(over="ignore"):
+        positions.astype(np.float32).reshape(-1).tofile(path)
+    _run(native("bvh_inputs", "bvh_build.cpp"), path)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 7, 64, 1000, 70000])
+@pytest.mark.parametrize("extent", [(1, 1, 1), (1e-39,) * 3, (3e-38,) * 3, (1, 1, 1e-42), (1, 1, 0), (0, 0, 0)])
+def test_bvh_of_any_extent(native, tmp_path, n, extent):
+    """Extents down to denormal ones, where bins per unit of length overflow a float, and flat ones."""
+    _bvh_of(native, tmp_path, _soup(n) * np.array(extent))
+
+
+def test_bvh_of_mixed_magnitudes(native, tmp_path):
+    g = np.random.RandomState(6)
+    _bvh_of(native, tmp_path, _soup(5000) * 10.0 ** g.uniform(-44, 30, size=(5000, 1, 1)))
