@@ -413,11 +413,12 @@ struct Builder {
 
 void write_node(BvhNode* dst, const TmpNode* n) {
   for (int k = 0; k < 3; ++k) {
-    float ext = n->hi[k] - n->lo[k];
+    constexpr float kMax = std::numeric_limits<float>::max();
+    float ext = std::min(n->hi[k] - n->lo[k], kMax);
     float mag = std::max(std::fabs(n->lo[k]), std::fabs(n->hi[k]));
     float pad = ext * 1e-6f + mag * 2e-7f;
-    dst->lo[k] = n->lo[k] - pad;
-    dst->hi[k] = n->hi[k] + pad;
+    dst->lo[k] = std::max(n->lo[k] - pad, -kMax);
+    dst->hi[k] = std::min(n->hi[k] + pad, kMax);
   }
   dst->a = n->count > 0 ? n->begin : 0;
   dst->b = n->count;
@@ -756,10 +757,20 @@ void build_bvh(const float* positions, int64_t num_tris, const BvhBuildOptions& 
     return;
   }
   int threads = opt.threads > 0 ? opt.threads : (int)std::max(1u, std::thread::hardware_concurrency());
+  // Triangles with an infinite or NaN coordinate are never hit (woop_record): they
+  // stand at a corner of a triangle that can be, where they widen no box.
+  auto finite = [&](int i) {
+    const float* p = positions + 9 * (size_t)i;
+    return std::all_of(p, p + 9, [](float x) { return std::isfinite(x); });
+  };
+  int first_finite = 0;
+  while (first_finite < T && !finite(first_finite)) ++first_finite;
+  float point[9] = {};
+  for (int k = 0; k < 9 && first_finite < T; ++k) point[k] = positions[9 * (size_t)first_finite + k % 3];
   std::vector<PrimRef> refs(T);
   parallel_parts(0, T, std::max(1, std::min(threads, T / 4096)), [&](int s, int e, int) {
     for (int i = s; i < e; ++i) {
-      const float* p = positions + 9 * (size_t)i;
+      const float* p = finite(i) ? positions + 9 * (size_t)i : point;
       PrimRef& r = refs[i];
       for (int k = 0; k < 3; ++k) {
         r.lo[k] = std::min(std::min(p[k], p[3 + k]), p[6 + k]);

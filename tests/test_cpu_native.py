@@ -114,3 +114,23 @@ def test_bvh_of_any_extent(native, tmp_path, n, extent):
 def test_bvh_of_mixed_magnitudes(native, tmp_path):
     g = np.random.RandomState(6)
     _bvh_of(native, tmp_path, _soup(5000) * 10.0 ** g.uniform(-44, 30, size=(5000, 1, 1)))
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 7, 64, 1000, 70000])
+@pytest.mark.parametrize("kind", ["nan corner", "nan", "infinite", "all nan", "huge"])
+def test_bvh_with_corners_that_are_not_finite(native, tmp_path, n, kind):
+    """Triangles with NaN or infinite corners are in the tree and widen no box; finite ones whose extent
+    overflows a float have boxes that hold them."""
+    p = _soup(n)
+    if kind == "nan corner":
+        p[::7, 1, 2] = np.nan
+    elif kind == "nan":
+        p[::7] = np.nan
+    elif kind == "infinite":
+        p[::5, 0, 0] = np.inf
+        p[1::5, 0, 1] = -np.inf
+    elif kind == "all nan":
+        p[:] = np.nan
+    else:
+        p = np.clip((p - 0.5) * 6.8e38, -np.finfo(np.float32).max, np.finfo(np.float32).max)
+    _bvh_of(native, tmp_path, p)
