@@ -9,7 +9,7 @@
 //            device-side loop captured once as a CUDA graph;
 //   waves  - the jobs' sample indices are laid end to end and cut into waves
 //            of `batch_slots` paths, each wave the plain render's launches for
-//            the deepest job's bounces, with no graph.
+//            the deepest of its own jobs' bounces, with no graph.
 // Up to two engines run a batch concurrently, engine e on the wave state and
 // stream of plain-render wave slot e.
 #include <cuda_runtime.h>
@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <cstring>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "context.h"
@@ -316,14 +317,14 @@ static int run_batch_waves_locked(orion_gpu_ctx* ctx, std::vector<DevJob>& dj, u
   // A wave's first bounces are launched at once. Deeper ones (roulette ends most
   // paths long before) follow a few at a time, and no more once the counters of
   // the stretch before last show that nothing was left: a stretch is always
-  // queued ahead of the one whose counters the host waits for, and the engines'
-  // waves advance in turn, so the device does not wait for the host.
+  // queued ahead of the one whose counters the host waits for, on whichever
+  // engine they come first, so the device does not wait for the host.
   constexpr int kUncheckedBounces = 17, kCheckedBounces = 8;
   struct OpenWave {
     int64_t k = -1;  // none
     int done;        // bounces launched
     int all, limit;  // those that end every path; those to launch at most (the test limit cuts waves short)
-    int stretch;     // its counters go to half stretch & 1 of the engine's batch_counters
+    int stretch;     // stretches queued; one's counters go to the engine's half (number & 1) of batch_counters
   };
   std::vector<OpenWave> open(ne);
   int64_t launches = 0, iterations = 0;
@@ -334,19 +335,7 @@ static int run_batch_waves_locked(orion_gpu_ctx* ctx, std::vector<DevJob>& dj, u
                      (int)std::min<unsigned long long>((unsigned long long)wave, total - base), engine_stream(ctx, e),
                      &launches, ctx->profiling ? &timer : nullptr};
   };
-  auto snapshot = [&](const OpenWave& o) { return 2 * (int)(o.k % ne) + (o.stretch & 1); };
-  // Queues the bounces up to `to` and a copy of the counters they leave.
-  auto stretch = [&](OpenWave& o, const BatchWave& w, int to) -> int {
-    launch_batch_wave_bounces(w, o.done, to, o.all);
-    o.done = to;
-    ++o.stretch;
-    if (to < o.limit) {
-      CUDA_TRY(cudaMemcpyAsync(ctx->batch_counters + kCounterSlots * snapshot(o), w.b.ctl->counters,
-                               kCounterSlots * sizeof(int), cudaMemcpyDeviceToHost, w.stream));
-      CUDA_TRY(cudaEventRecord(ctx->ev_film[snapshot(o)], w.stream));
-    }
-    return ORION_OK;
-  };
+  auto snapshot = [&](const OpenWave& o, int s) { return 2 * (int)(o.k % ne) + (s & 1); };
   auto close = [&](OpenWave& o, const BatchWave& w) -> int {
     launch_batch_wave_film(w, o.done < o.all ? o.done : -1);
     CUDA_TRY(cudaGetLastError());
@@ -354,35 +343,55 @@ static int run_batch_waves_locked(orion_gpu_ctx* ctx, std::vector<DevJob>& dj, u
     o.k = -1;
     return ORION_OK;
   };
-  auto advance = [&](OpenWave& o) -> int {
-    const BatchWave w = wave_of(o.k);
-    const int at = snapshot(o), parity = o.done & 1;
-    RC(stretch(o, w, std::min(o.limit, o.done + kCheckedBounces)));
-    CUDA_TRY(cudaEventSynchronize(ctx->ev_film[at]));
-    const int* c = ctx->batch_counters + kCounterSlots * at;
-    // Paths that ended may still have had a light sample to trace and add.
-    const bool left = c[cnt_rays(RK_EXT, parity)] > 0 || c[CNT_NEE + parity] > 0;
-    return left && o.done < o.limit ? ORION_OK : close(o, w);
-  };
-  auto advance_all = [&]() -> int {
-    for (OpenWave& o : open)
-      if (o.k >= 0) RC(advance(o));
+  // Queues `bounces` more and a copy of the counters they leave, or what is left
+  // of the wave and its film.
+  auto stretch = [&](OpenWave& o, const BatchWave& w, int bounces) -> int {
+    const int to = std::min(o.limit, o.done + bounces);
+    launch_batch_wave_bounces(w, o.done, to, o.all);
+    o.done = to;
+    ++o.stretch;
+    if (to == o.limit) return close(o, w);
+    CUDA_TRY(cudaMemcpyAsync(ctx->batch_counters + kCounterSlots * snapshot(o, o.stretch), w.b.ctl->counters,
+                             kCounterSlots * sizeof(int), cudaMemcpyDeviceToHost, w.stream));
+    CUDA_TRY(cudaEventRecord(ctx->ev_film[snapshot(o, o.stretch)], w.stream));
     return ORION_OK;
+  };
+  // Waits until an open wave has finished its stretch before last, and queues its
+  // next one or, if that left nothing, its film.
+  auto advance = [&]() -> int {
+    while (true) {
+      for (OpenWave& o : open) {
+        if (o.k < 0) continue;
+        const int at = snapshot(o, o.stretch - 1), parity = (o.done - kCheckedBounces) & 1;
+        const cudaError_t e = cudaEventQuery(ctx->ev_film[at]);
+        if (e == cudaErrorNotReady) {
+          cudaGetLastError();
+          continue;
+        }
+        CUDA_TRY(e);
+        const BatchWave w = wave_of(o.k);
+        const int* c = ctx->batch_counters + kCounterSlots * at;
+        // Paths that ended may still have had a light sample to trace and add.
+        const bool left = c[cnt_rays(RK_EXT, parity)] > 0 || c[CNT_NEE + parity] > 0;
+        return left ? stretch(o, w, kCheckedBounces) : close(o, w);
+      }
+      std::this_thread::yield();
+    }
   };
   for (int64_t k = 0; k < nwaves; ++k) {
     OpenWave& o = open[k % ne];
-    while (o.k >= 0) RC(advance_all());
+    while (o.k >= 0) RC(advance());
     const BatchWave w = wave_of(k);
     o.k = k;
     o.done = o.stretch = 0;
     o.all = bounces_of(w.base, w.n);
     o.limit = ctx->cfg.test_batch_iterations > 0 ? std::min(ctx->cfg.test_batch_iterations, o.all) : o.all;
     launch_batch_wave_begin(w);
-    RC(stretch(o, w, std::min(o.limit, kUncheckedBounces)));
-    if (o.done == o.limit) RC(close(o, w));
+    RC(stretch(o, w, kUncheckedBounces));
+    if (o.k >= 0) RC(stretch(o, w, kCheckedBounces));
   }
   for (OpenWave& o : open)
-    while (o.k >= 0) RC(advance_all());
+    while (o.k >= 0) RC(advance());
   for (int e = 1; e < ne; ++e) {
     CUDA_TRY(cudaEventRecord(ctx->ev_join[e - 1], engine_stream(ctx, e)));
     CUDA_TRY(cudaStreamWaitEvent(s, ctx->ev_join[e - 1], 0));
