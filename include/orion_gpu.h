@@ -242,9 +242,10 @@ int orion_gpu_last_stats(orion_gpu_ctx* ctx, orion_render_stats* out);
  * on (CUDA events around every kernel; adds a little launch overhead).
  * Stages: 0 camera, 1 extension-ray trace, 2 shade, 3 shadow-ray trace,
  * 4 MIS-ray trace, 5 direct-light resolve, 6 film, 7 bookkeeping.
- * A batched render under profiling runs its loop from the host instead of a
- * graph while-node (same kernels and results; stage 0 is then slot refill,
- * stage 6 retirement into the films). */
+ * Under profiling the rays of a bounce are traced kind by kind, in a launch
+ * each, waves follow one another, and a pooled batch runs its loop from the host
+ * instead of a graph while-node (same results; stage 0 of a pooled batch is slot
+ * refill, stage 6 retirement into the films). */
 #define ORION_NUM_STAGES 8
 typedef struct orion_stage_times {
   double ms[ORION_NUM_STAGES];
@@ -310,7 +311,9 @@ int orion_gpu_render_batch(orion_gpu_ctx* ctx, int32_t njobs, const orion_job* j
 /* Launch configuration: the autotuned knobs. */
 typedef struct orion_launch_config {
   int32_t trace_block;    /* threads per block of the traversal kernels (64..512) */
-  int32_t shade_block;    /* threads per block of the shading kernels (64..512) */
+  int32_t shade_block;    /* threads per block (32..128) of the shading kernels with little code and of the
+                             resolve kernels; the classes with the most code (textured, general, plastic,
+                             dielectric) run in blocks of 320 threads whatever this says */
   int32_t smem_stack;     /* traversal stack entries kept in shared memory: 0, 8, 16, 24 or 32 */
   int32_t blocks_per_sm;  /* persistent trace blocks per SM; the grid-stride kernels launch twice as many */
   int32_t wave_paths;     /* paths per plain-render wave */
@@ -424,15 +427,17 @@ int orion_gpu_mem_info(orion_gpu_ctx* ctx, int64_t* free_bytes, int64_t* total_b
 /* Failure-path test knobs (0, 0 = normal operation). stack_entries = 2 makes
  * plain renders and orion_gpu_trace_wave trace with kernels whose traversal
  * stack holds 2 entries, so deep traversals overflow and the call returns
- * ORION_ERR_DEVICE; batch_iterations > 0 stops every batch loop after that
- * many iterations, so unfinished batches return ORION_ERR_DEVICE. No
+ * ORION_ERR_DEVICE; batch_iterations > 0 stops a pooled batch's loop after that
+ * many iterations and a wave after that many bounces, so unfinished batches
+ * return ORION_ERR_DEVICE. No
  * counterpart in the reference, which prints and continues (src/orion.h:33-37). */
 int orion_gpu_set_test_limits(orion_gpu_ctx* ctx, int32_t stack_entries, int32_t batch_iterations);
 /* orion_gpu_trace without any device allocation. No counterpart in the
  * reference: it exists for callers that must not allocate, such as a ray query
  * (picking) from a second context while a long render runs on the same device
- * (cudaFree in orion_gpu_trace synchronises the whole device, and a serving
- * memory budget has already committed every device byte). Rays and hits go
+ * (orion_gpu_trace takes its buffers from the context's pool, or above 64 MB by
+ * cudaMalloc, which may wait for the device, and a serving memory budget has
+ * already committed every device byte). Rays and hits go
  * through one fixed static device array of ORION_NOALLOC_MAX_RAYS rays
  * (3 MiB); larger n is rejected with ORION_ERR_INVALID. Nothing in that array
  * must start at zero. Calls on one context are serialised by the context; calls

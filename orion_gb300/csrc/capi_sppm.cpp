@@ -96,7 +96,7 @@ extern "C" int orion_gpu_render_sppm(orion_gpu_ctx* ctx, orion_scene_id id, cons
     launch_sppm_visible_points(d.view, v, iter, st);
     launch_sppm_photons(d.view, v, iter, st);
     CUDA_TRY(cudaGetLastError());
-    launches += (nscan > 1 ? 8 : 7) + (nscan > 4 * kScanBlock ? 1 : 0) + (photons > 0 ? 1 : 0);
+    launches += (nscan > 1 ? 8 : 7) + (nscan > kScanRaw ? 1 : 0) + (photons > 0 ? 1 : 0);
   }
   CUDA_TRY(cudaEventRecord(ctx->ev1, st));
   unsigned long long rays = 0;

@@ -81,11 +81,11 @@ __global__ void __launch_bounds__(512, 2) k_trace(const __grid_constant__ TraceA
 // One bounce for every path whose extension ray hit a material of shading
 // class SC (or, for SC_MISS, left the scene), with that class's BSDF code only.
 // Launch bounds: at most 96 registers (640 threads per SM).
-// The queues a path goes to next (light-sample resolution, shadow ray, MIS
-// rays, next extension ray) are recorded as bits of its qflags byte, and
-// k_compact_queues lists them in slot order: the next trace launches then
-// take rays of neighbouring pixels together instead of in the order the
-// shading finished them.
+// The queues a path goes to next (next extension ray, shadow ray, MIS rays)
+// are recorded as bits of its qflags byte, and k_compact_queues lists them in
+// slot order: the next trace then takes rays of neighbouring pixels together
+// instead of in the order the shading finished them. Small waves append to the
+// queues here (WaveArgs::append).
 // The classes' launches do not depend on one another: each lets the next one
 // start as soon as its own last blocks run (launch_shading), so the short
 // ones overlap; block 0 ends only when the launch before has, which makes the
@@ -208,9 +208,8 @@ __global__ void k_sobol(const uint32_t* sobol, int64_t n, const uint64_t* index,
 // Ray queries (Scene::intersect): closest hit in (tnear, tfar]. Warps take
 // their rays from pieces of the list of their own, neighbouring rays together,
 // and refill idle lanes from it (no counter to clear); triangles are tested by
-// the whole warp. A query of 100,000 rays took 422 us
-// with one ray per thread and five device allocations, 181 us so; one ray 216
-// and 59 us.
+// the whole warp. A query of 100,000 rays took 422 us with one ray per thread
+// and five device allocations, 181 us so; one ray 216 and 59 us.
 constexpr int kQueryStack = 8, kQueryBlock = 128, kQueryRefill = 20;
 
 __global__ void __launch_bounds__(kQueryBlock, 8) k_trace_closest(SceneView s, int64_t n, const float4* rays, float* t,

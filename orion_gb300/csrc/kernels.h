@@ -56,8 +56,9 @@ struct PathRec {
 static_assert(sizeof(PathRec) == 96, "PathRec is three sectors");
 
 // Next-event-estimation record of a path, 128 bytes: written whole by the
-// shading kernel; the shadow trace reads [sh_o, sh_d], the MIS trace
-// [mis_o, mis_d], the resolve kernel the first two sectors.
+// shading kernel; the trace reads [sh_o, sh_d] of shadow rays and [mis_o, mis_d]
+// of MIS rays, and what adds the sample to the radiance the first two sectors (the
+// path's next shading or k_film; in batches k_b_resolve).
 struct NeeRec {
   float4 p;      // shading point xyz, light-selection pdf
   float4 beta;   // beta before the bounce, w = flags | light << 8 (int bits)
@@ -87,7 +88,7 @@ struct WaveView {
   int* mis_occluded;  // MIS ray towards an environment light: anything hit
   int* q_mis_env;     // MIS rays towards an environment light (occlusion queries)
   int* q_ext[2];     // extension-ray queues (current / next bounce)
-  int* q_nee;        // paths that sampled a light this bounce
+  int* q_nee;        // batches: paths that sampled a light this bounce
   int* q_sh;         // shadow rays
   int* q_mis;        // BSDF-sampled rays towards a non-delta light
   int* q_cls;        // extension hits by shading class: kShadeClasses queues of `capacity`
@@ -286,7 +287,7 @@ struct FilmView {
 struct LaunchConfig {
   int num_sms;
   int trace_block;   // threads per block of the trace kernels
-  int shade_block;
+  int shade_block;   // threads per block of the shading kernels with little code (shade_shape), resolve and retire
   int blocks_per_sm; // persistent grid size factor
   int smem_stack;    // shared-memory stack entries per thread (0, 8, 16, 24, 32)
   int refill_below;  // a traversal warp refills idle lanes when fewer lanes than this hold a ray (1..32)
@@ -343,8 +344,9 @@ struct StageTimer {
   }
 };
 
-// One full wave: camera rays, then (trace, shade, shadow/MIS trace,
-// resolve) per bounce, then film accumulation. All on `stream`, no host sync.
+// One full wave: camera rays, then per bounce one trace of all waiting rays (its
+// extension rays, the previous bounce's shadow and MIS rays) and the shading, then
+// film accumulation. All on `stream`, no host sync.
 // The film kernel first waits for `film_wait` (the film write of an earlier
 // wave of the same pixels) and then records `film_done`.
 void launch_wave(const SceneView& s, const WaveView& w, const WaveArgs& a, const FilmView& film,
@@ -356,7 +358,7 @@ void launch_wave(const SceneView& s, const WaveView& w, const WaveArgs& a, const
 // opt-in maximum, so any accepted stack depth x block size can launch).
 struct KernelLimits {
   int max_trace_block;  // threads per block the traversal kernels can launch with
-  int max_shade_block;  // same for the shade / resolve / retire kernels
+  int max_shade_block;  // same for the kernels that LaunchConfig::shade_block applies to
 };
 cudaError_t configure_kernels(int smem_bytes, KernelLimits* lim);
 cudaError_t configure_batch_kernels(int smem_bytes, KernelLimits* lim);
@@ -458,6 +460,7 @@ ORION_HD inline bool photons_dealt(unsigned base, unsigned count, int photons) {
 
 constexpr int kSppmBoundsBlocks = 1024;  // blocks of the bounds pass (part_lo / part_hi entries)
 constexpr int kScanBlock = 1024;         // elements per block of the cell-count scan
+constexpr int kScanRaw = 4 * kScanBlock;  // block sums up to which the scan needs no pass over them (k_scan_add)
 
 // Resets per-pixel state (radius r0, no visible point) and the film, and
 // fills photon_mats from the scene's materials.

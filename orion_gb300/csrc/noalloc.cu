@@ -1,13 +1,13 @@
 // Ray queries that allocate no device memory: orion_gpu_trace_noalloc.
 //
-// The same traversal kernel as orion_gpu_trace (k_trace_rays through
-// launch_trace), but its ray and hit buffers live in one file-scope static
-// device array instead of per-call cudaMalloc/cudaFree. It exists for callers
-// that must not allocate: a ray query (picking, a probe) issued from a second
-// context while a long render runs on the same device. cudaFree synchronises
-// the whole device, so orion_gpu_trace would wait for that render to finish;
-// and under the serving loop's memory budget every device byte is already
-// accounted for. This entry point waits only for its own stream.
+// The same kernels as orion_gpu_trace (k_trace_closest, k_trace_any through
+// launch_trace), but the ray and hit buffers live in one file-scope static
+// device array instead of memory from the context's pool or, above 64 MB,
+// cudaMalloc. It exists for callers that must not allocate: a ray query (picking, a
+// probe) issued from a second context while a long render runs on the same device.
+// A pool that has to grow, and cudaMalloc and cudaFree, may wait for the device; and
+// under the serving loop's memory budget every device byte is already accounted
+// for. This entry point waits only for its own stream.
 //
 // Limits and rules:
 //   * at most ORION_NOALLOC_MAX_RAYS rays per call (3 MiB of scratch in all);

@@ -541,9 +541,7 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_parts(int* part, int nparts
 }
 
 // raw: `part` holds the blocks' sums, not their scan: each block adds up those
-// before it itself (one launch less, while there are few).
-constexpr int kScanRaw = 4 * kScanBlock;
-
+// before it itself (one launch less, while there are at most kScanRaw).
 __global__ void __launch_bounds__(kScanBlock) k_scan_add(int* a, int n, const int* part, int raw) {
   __shared__ int warp_sum[32];
   const int i = blockIdx.x * kScanBlock + threadIdx.x;

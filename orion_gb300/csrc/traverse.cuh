@@ -258,11 +258,10 @@ __device__ __forceinline__ int take_child(uint2& ng, uint32_t oct) {
 }
 
 // First hit found over (tnear, tfar], one ray per thread, children visited far
-// to near (see lane_visit). A stack overflow ends the traversal with a miss
-// (see the file comment).
-template <int SMEM, int CAP>
+// to near (see lane_visit).
+template <int SMEM>
 __device__ __forceinline__ RayHit traverse_any(const TraceScene& s, V3 o, V3 d, float tnear, float tfar,
-                                               TraversalStack<SMEM, CAP>& st) {
+                                               TraversalStack<SMEM>& st) {
   RayHit h;
   h.t = tfar;
   h.u = h.v = 0.f;
@@ -275,8 +274,7 @@ __device__ __forceinline__ RayHit traverse_any(const TraceScene& s, V3 o, V3 d, 
   while (true) {
     if (ng.y > 0x00ffffffu) {
       const int child = take_child(ng, ord);
-      if (ng.y && !st.push(make_int2((int)ng.x, (int)ng.y)))
-        h.t = -1.f;  // poisoned: nothing passes a test against tmax < tnear
+      if (ng.y) st.push(make_int2((int)ng.x, (int)ng.y));  // (a kMaxStack stack: never full)
       wide_node(s.nodes, child, o, idir, oct, tnear, h.t, ng, tg, ord);
     } else {
       tg = ng;
@@ -300,7 +298,6 @@ __device__ __forceinline__ RayHit traverse_any(const TraceScene& s, V3 o, V3 d, 
       ng = make_uint2((uint32_t)e.x, (uint32_t)e.y);
     }
   }
-  if (h.t < 0.f) h.t = tfar;  // stack overflow: reported as a miss
   return h;
 }
 
