@@ -252,8 +252,8 @@ __global__ void __launch_bounds__(kCompactThreads) k_wb_compact(uint8_t* flags, 
 // The wave's radiance into the jobs' films. A block takes 256 slots at a time
 // into shared memory; slots of one pixel are neighbours, a run, and a run ends
 // in one FP64 atomic per channel (a pixel's samples may go on in the next 256
-// slots or another wave). The FP64 unit bounds it (2 lanes a clock and SM, and
-// a warp holds it as long for one lane as for 32): a run's samples are added in
+// slots or another wave). The FP64 unit is its busiest (64% of peak; 2 lanes a clock
+// and SM, and a warp holds it as long for one lane as for 32): a run's samples are added in
 // pieces of up to kWbPiece slots, one thread per piece and channel, then the
 // pieces of a run by one thread, so that the lanes are full whatever the
 // samples per pixel. Film stage of a batch, one thread per run / pieces: 33.5M

@@ -27,13 +27,13 @@
 // material and frame are loaded once, and no flux atomics are needed.
 // The camera and photon kernels hold all of the sampling and BSDF code, and
 // with every warp at a place of its own they waited for instructions most of
-// the time (no-instruction stalls of 8 and 7 cycles per issue, 10 and 4 of 32
-// lanes active). So all lanes of a block go step by step together (trace,
-// shade, shadow rays, ...: block barriers in between), rays are traced by whole
-// warps (warp_trace, one copy of each traversal), and warps take new photons
-// for those that ended. 512x512, 262,144 photons: camera pass 614 -> 477 us an
-// iteration, photon pass 585 -> 425 us, gather 738 -> 337 us (see there); 16
-// iterations 28.4 -> 19.7 ms.
+// the time (12.2 and 10.5 cycles per issue, 10.0 and 4.2 of 32 lanes active,
+// 1024x1024 pixels, 1M photons). So all lanes of a block go step by step together
+// (trace, shade, shadow rays, ...: block barriers in between), rays are traced by
+// whole warps (warp_trace, one copy of each traversal), and warps take new photons
+// for those that ended: 2.8 and 6.6 cycles, 14.7 and 9.6 lanes, camera pass 2.01 ->
+// 1.16 ms an iteration, photon pass 2.26 -> 1.34 ms, gather 3.84 -> 2.21 ms (see
+// there). 512x512, 16 iterations of 262,144 photons: 28.4 -> 18.8 ms.
 // Sample indices and dimensions follow the reference: the camera path of
 // pixel (i, j) in iteration k uses index k*W*H + j*W + i, photon p uses
 // iterations*W*H + k*photons + p, each from dimension 5.
@@ -382,8 +382,9 @@ __global__ void __launch_bounds__(256) k_sppm_fill(SppmView v) {
 // visible point: the lanes look up the cells (at most 27) at once, then take
 // the hits of all cells as one list, and the hits within the radius are
 // collected 32 at a time before their BSDF is evaluated, so lanes idle neither
-// in short cells nor over the hits outside the sphere (738 -> 337 us against cell
-// after cell, each hit's BSDF where it is found: 592M -> 239M instructions).
+// in short cells nor over the hits outside the sphere (1024x1024 pixels, 1M photons:
+// 3.84 -> 2.21 ms against cell after cell, each hit's BSDF where it is found; 2,582M
+// -> 1,543M warp instructions, 19.5 -> 30.1 of 32 lanes).
 // Every lane runs the same material's BSDF, inline for the diffuse class; the
 // lanes' sums are added at the end. The counts of 32 cells are summed in an int:
 // where one is above kGatherTogether (films of few pixels, whose few hash cells hold
