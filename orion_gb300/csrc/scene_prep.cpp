@@ -177,8 +177,10 @@ bool prepare_scene(const HostScene& s, PreparedScene* out, std::string* err) {
       p.light = s.light_of_prim[i];
       for (int c = 0; c < 3; ++c)
         for (int k = 0; k < 3; ++k) {
-          b.lo[k] = std::min(b.lo[k], p.p[3 * c + k]);
-          b.hi[k] = std::max(b.hi[k], p.p[3 * c + k]);
+          const float x = p.p[3 * c + k];
+          if (!std::isfinite(x)) continue;  // a triangle that no ray hits
+          b.lo[k] = std::min(b.lo[k], x);
+          b.hi[k] = std::max(b.hi[k], x);
         }
     }
     part[t] = b;
@@ -193,12 +195,17 @@ bool prepare_scene(const HostScene& s, PreparedScene* out, std::string* err) {
     }
   }
   // Bounds3::boundingSphere (src/core/geometry.h:551-554).
-  for (int k = 0; k < 3; ++k) out->world_center[k] = (lo[k] + hi[k]) * 0.5f;
+  for (int k = 0; k < 3; ++k) {
+    out->world_center[k] = (lo[k] + hi[k]) * 0.5f;
+    if (!std::isfinite(out->world_center[k])) out->world_center[k] = lo[k] * 0.5f + hi[k] * 0.5f;
+  }
   bool inside = T > 0;
   for (int k = 0; k < 3; ++k) inside = inside && out->world_center[k] >= lo[k] && out->world_center[k] <= hi[k];
   if (inside) {
     float d[3] = {out->world_center[0] - hi[0], out->world_center[1] - hi[1], out->world_center[2] - hi[2]};
     out->world_radius = std::sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+    // Where its square overflows: rays to points at infinity would pass every box.
+    if (!std::isfinite(out->world_radius)) out->world_radius = 1e18f;
   } else {
     out->world_radius = 0.f;
   }

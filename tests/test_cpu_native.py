@@ -134,3 +134,26 @@ def test_bvh_with_corners_that_are_not_finite(native, tmp_path, n, kind):
     else:
         p = np.clip((p - 0.5) * 6.8e38, -np.finfo(np.float32).max, np.finfo(np.float32).max)
     _bvh_of(native, tmp_path, p)
+
+
+@pytest.mark.parametrize("kind,radius", [
+    ("plain", 0.505 * 3 ** 0.5), ("infinite", 0.505 * 3 ** 0.5), ("nan", 0.505 * 3 ** 0.5), ("none", 0), ("wide", 1e18),
+    ("far", 0)])
+def test_world_sphere_is_finite(native, tmp_path, kind, radius):
+    """Corners that are not finite, and extents whose square overflows a float, leave the sphere that distant and
+    environment lights stand on finite (a ray to a point at infinity passes every box of the tree)."""
+    p = _soup(1000).astype(np.float64)
+    p[0], p[1] = 0.0, 1.01  # the corners of the bounds
+    if kind == "infinite":
+        p[2, 0, 0], p[3, 1, 2] = np.inf, -np.inf
+    elif kind == "nan":
+        p[2] = np.nan
+    elif kind == "none":
+        p[:] = np.inf
+    elif kind == "wide":
+        p = (p - 0.5) * 4e38
+    elif kind == "far":
+        p = 3.2e38 + p * 1e37
+    path = str(tmp_path / "positions.bin")
+    p.astype(np.float32).reshape(-1).tofile(path)
+    _run(native("world_bounds", "scene_prep.cpp"), path, radius)
