@@ -375,10 +375,10 @@ cudaError_t capture_batch_iteration(const WaveView& w, const BatchView& b, const
 void launch_batch_iteration(const WaveView& w, const BatchView& b, const uint32_t* sobol, const LaunchConfig& cfg,
                             unsigned class_mask, cudaStream_t stream, StageTimer* timer);
 // Wave mode: the work items [base, base + n) on slots 0..n-1, a plain wave's launches.
-// _begin starts the paths; _bounces runs the bounces [from, to), every path's last one at
-// the latest `all` - 1 (one more than the depth of the deepest job among them); _film adds
-// the radiance of the n paths to their jobs' films (unfinished: -1, or the number of bounces
-// run if some paths may be left, which are then reported as kErrIterationCap).
+// _begin starts the paths. _bounces runs the bounces [from, to); `all` bounces (one more
+// than the depth of the deepest job among them) end every path. _film adds the radiance of
+// the n paths to their jobs' films; unfinished: -1, or the number of bounces run if paths
+// may be left, which are then reported as kErrIterationCap.
 struct BatchWave {
   const WaveView& w;
   const BatchView& b;
